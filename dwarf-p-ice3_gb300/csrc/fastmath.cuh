@@ -26,13 +26,20 @@
 //          r = z*invc - 1 exact in one FMA (|r| < 2^-7); log x = e ln2 -
 //          log(invc) + log1p(r), log1p by its Taylor series (to r^4 in FP64,
 //          r^5 .. r^8 in FP32).  9 FP64 ops.
-//   frcp   1/d: a correctly rounded FP32 reciprocal of d (truncated to FP32)
-//          as the seed r0 (|eps| = |1 - d r0| < 2^-22), then one Newton-
-//          Raphson step with the quadratic term of 1/(1-eps) = 1 + eps +
-//          eps^2 + ..., r1 = r0 (1 + eps + eps^2), leaving eps^3 < 2^-66.
-//          3 FP64 ops (an IEEE FP64 divide costs ~9 on GB300).  fdiv(a, b) =
-//          a * frcp(b), within 2 ulp.  Outside 2^-125 < |d| < 2^125 (and for
-//          zero, inf, NaN) it falls back to the IEEE division.
+//   frcp   1/d and fdiv a/b, the IEEE results bit for bit, in integer
+//          arithmetic (no FP64 operation): with d = x 2^k, x in [1, 2), the
+//          hardware's FP32 reciprocal y0 of x (24 bits, |eps| = |1 - x y0| <
+//          2^-21), one Newton-Raphson step with its quadratic term, y0 (1 +
+//          eps + eps^2), in 64-bit fixed point (eps exact, remainder eps^3 <
+//          2^-63), the significand (of a times it) rounded to 53 bits, and
+//          the rounding settled by the exact remainder (a - q b modulo 2^64).
+//          A quotient of doubles is never halfway between two doubles, so the
+//          sign of |r| - |b|/2 decides; the seed's error cannot reach the
+//          result.  The FP64 pipe was 78 % busy with the issue slots 83 %
+//          idle; taking the 3 / 7 FP64 operations of a reciprocal / rounded
+//          division to the integer pipe gave rain_ice 13.60 -> 12.01 ms,
+//          the adjoint 26.3 -> 24.8 ms (256x256x90).  Where an operand is zero, subnormal, infinite or NaN, or
+//          the result leaves the normal range, the IEEE division.
 //   frsqrt 1/sqrt(d): y0 = the FP32 reciprocal of the FP32 square root of d
 //          (truncated to FP32; |eps| = |1 - d y0^2| < 2^-21), then
 //          y0 (1 + eps/2 + 3 eps^2/8), the series of (1 - eps)^(-1/2) to its
@@ -119,6 +126,16 @@ __device__ __forceinline__ double from_bits_(int64_t b) { return __longlong_as_d
 __device__ __forceinline__ int32_t fbits_(float x) { return __float_as_int(x); }
 __device__ __forceinline__ float ffrom_bits_(int32_t b) { return __int_as_float(b); }
 __device__ __forceinline__ int clz32_(uint32_t v) { return __clz((int)v); }
+__device__ __forceinline__ uint32_t hi_(double x) { return (uint32_t)__double2hiint(x); }
+__device__ __forceinline__ uint32_t lo_(double x) { return (uint32_t)__double2loint(x); }
+__device__ __forceinline__ uint32_t mulhi_(uint32_t a, uint32_t b) { return __umulhi(a, b); }
+// 1/x within 2^-22 for the integer reciprocal (its error cannot reach a result)
+__device__ __forceinline__ float rcp_seed_(float x)
+{
+  float y;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
 #else
 static const ExpEntry kExpTable[256] = FM_EXP_TABLE_INIT;
 static const LogEntry kLogTable[128] = FM_LOG_TABLE_INIT;
@@ -147,6 +164,10 @@ inline double from_bits_(int64_t b) { double x; memcpy(&x, &b, 8); return x; }
 inline int32_t fbits_(float x) { int32_t b; memcpy(&b, &x, 4); return b; }
 inline float ffrom_bits_(int32_t b) { float x; memcpy(&x, &b, 4); return x; }
 inline int clz32_(uint32_t v) { return v ? __builtin_clz(v) : 32; }
+inline uint32_t hi_(double x) { return (uint32_t)((uint64_t)bits_(x) >> 32); }
+inline uint32_t lo_(double x) { return (uint32_t)bits_(x); }
+inline uint32_t mulhi_(uint32_t a, uint32_t b) { return (uint32_t)(((uint64_t)a * b) >> 32); }
+inline float rcp_seed_(float x) { return rcpf_(x); }
 #endif
 
 // double -> float by truncation of the significand, with integer operations
@@ -277,65 +298,98 @@ FM_NI double flog(double x)
   return add_(hi, add_(r, tail));
 }
 
-// The IEEE 1/d and 1/sqrt(d), out of line: the rare fallbacks of frcp and
-// frsqrt, which are inlined at many sites.
-FM_NI double rcp_ieee_(double d) { return 1.0 / d; }
+// The IEEE 1/sqrt(d), out of line: the rare fallback of frsqrt.
 FM_NI double rsqrt_ieee_(double d) { return 1.0 / sqrt(d); }
 
-// 1/d (see the header): FP32 seed + one Newton-Raphson step with its
-// quadratic term.
-FM_NI double frcp(double d)
-{
-  const int64_t e = (bits_(d) >> 52) & 0x7ff;
-  if (e < 1023 - 125 || e > 1023 + 125) return rcp_ieee_(d);     // zero, tiny, huge, inf, NaN
-  const double r0 = to_f64(rcpf_(to_f32(d)));
-  const double eps = fma_(-d, r0, 1.0);
-  return fma_(r0, fma_(eps, eps, eps), r0);
-}
-FM_HD double fdiv(double a, double b) { return mul_(a, frcp(b)); }
-
-// a / b rounded to nearest (the IEEE quotient) for 2^-400 <= |a|, |b| <=
-// 2^400, from y = frcp(b): q0 = a y, then q1 = q0 + (a - b q0) y, checked
-// with the exact remainder r = a - b q1 (one fma): q1 is the rounded quotient
-// iff |r| < |b| ulp(q1) / 2 (a / b is never halfway between two doubles; q1
-// a power of two, whose lower neighbour is closer, is not accepted).  Where
-// the check fails or the operands are out of range, the IEEE division.  4
-// FP64 operations per quotient besides the reciprocal; the check is integer
-// work.  fdiv_rn2 shares the reciprocal between two numerators.
 // the IEEE division, out of line (the rare fallback of the paths below)
 FM_NI double div_ieee_(double a, double b) { return a / b; }
-FM_HD bool div_rn_range_(double x)
+
+// 1/x to within 2^-62 for x in [1, 2) as a fixed-point fraction, Y 2^-63;
+// mh : ml the 53-bit significand of x.
+FM_HD uint64_t rcp_fixed_(uint32_t mh, uint32_t ml)
 {
-  const int64_t e = (bits_(x) >> 52) & 0x7ff;
-  return e >= 1023 - 400 && e <= 1023 + 400;
+  const float xf = ffrom_bits_((int32_t)(0x3f800000u | ((mh & 0xfffffu) << 3) | (ml >> 29)));   // x truncated
+  // y0 2^24, below 2^24 (y0 = 1 is taken one unit lower)
+  const uint32_t yb = (uint32_t)fbits_(rcp_seed_(xf));
+  const uint32_t y0 = ((yb < 0x3f7fffffu ? yb : 0x3f7fffffu) & 0x7fffffu) | 0x800000u;
+  // eps 2^84 = 2^84 - (x 2^60) (y0 2^24), modulo 2^64 (|eps| < 2^-21)
+  const uint32_t xl = ml << 8, xh = (mh << 8) | (ml >> 24);
+  const uint64_t p = (uint64_t)xl * y0 + ((uint64_t)(xh * y0) << 32);
+  const int64_t e = (int64_t)(0u - p);
+  const int32_t eh = (int32_t)(e >> 32);
+  const int64_t w = e + (((int64_t)eh * eh) >> 20);               // eps + eps^2
+  // y0 + y0 w
+  const int64_t t = (int64_t)(int32_t)(w >> 32) * (int32_t)y0 + (int64_t)mulhi_((uint32_t)w, y0);   // y0 w 2^76
+  return ((uint64_t)y0 << 39) + (uint64_t)(t >> 13);
 }
-FM_HD double div_rn_with_(double a, double b, double y)
+
+// The 53-bit quotient settled by its exact remainder r = a - q b (|r| far
+// below 2^63, so its low 64 bits tell it): q is the rounded quotient iff
+// |r| <= b / 2.
+FM_HD uint64_t settle_(uint64_t q, int64_t r, uint64_t mb)
 {
-  const double q0 = mul_(a, y);
-  const double q1 = fma_(fma_(-q0, b, a), y, q0);
-  const double r = fma_(-q1, b, a);
-  const int64_t bq = bits_(q1) & 0x7fffffffffffffffLL, bb = bits_(b) & 0x7fffffffffffffffLL;
-  // |b| ulp(q1) / 2 = |b| 2^(E(q1) - 1023 - 53): add to b's exponent
-  const int64_t eh = (bb >> 52) + (bq >> 52) - (1023 + 53);
-  if (eh >= 1 && (bq & 0x000fffffffffffffLL) != 0 && (bits_(r) & 0x7fffffffffffffffLL) < bb + ((eh - (bb >> 52)) << 52))
-    return q1;
-  return div_ieee_(a, b);
+  const int64_t half = (int64_t)(mb >> 1);
+  if (r > half) return q + 1;
+  if (r < -half) return q - 1;
+  return q;
 }
+
+// 1/d, correctly rounded.
+FM_NI double frcp(double d)
+{
+  const uint32_t h = hi_(d), l = lo_(d), e = (h >> 20) & 0x7ffu;
+  if (e - 1u >= 2044u) return div_ieee_(1.0, d);                  // zero, subnormal, inf, NaN; subnormal result
+  const uint32_t mh = (h & 0xfffffu) | 0x100000u;
+  const uint64_t m = ((uint64_t)mh << 32) | l;
+  uint64_t q = (rcp_fixed_(mh, l) + 512u) >> 10;                  // 2^53 / x, in [2^52, 2^53]
+  q = settle_(q, (int64_t)(0u - q * m), m);
+  return from_bits_((int64_t)(q + ((uint64_t)(2044u - e) << 52) + ((uint64_t)(h & 0x80000000u) << 32)));
+}
+
+// a / b from Y = rcp_fixed_ of b's significand, correctly rounded.  ex: the
+// exponent fields' difference plus 1023, in [2, 2045].
+FM_HD double quot_(uint32_t ah, uint32_t al, uint32_t bh, uint32_t bl, uint64_t y, uint32_t ex)
+{
+  const uint32_t mah = (ah & 0xfffffu) | 0x100000u, mbh = (bh & 0xfffffu) | 0x100000u;
+  // a / b 2^62 in (2^61, 2^63): (significand of a, 64 bits) times Y, high half
+  const uint32_t th = (mah << 11) | (al >> 21), tl = al << 11, yh = (uint32_t)(y >> 32), yl = (uint32_t)y;
+  const uint64_t qp = (uint64_t)th * yh + mulhi_(th, yl) + mulhi_(tl, yh);
+  const uint32_t lt1 = (qp >> 62) == 0 ? 1u : 0u;                 // quotient below 1: one bit more
+  uint64_t q = (qp + (512u >> lt1)) >> (10u - lt1);
+  const uint64_t mb = ((uint64_t)mbh << 32) | bl;
+  const int64_t r = (int64_t)(((uint64_t)(al << (20u + lt1)) << 32) - q * mb);   // a 2^(52 + lt1) - q b, modulo 2^64
+  q = settle_(q, r, mb);
+  return from_bits_((int64_t)(q + ((uint64_t)(ex - lt1 - 1u) << 52) + ((uint64_t)((ah ^ bh) & 0x80000000u) << 32)));
+}
+
+// a / b, correctly rounded (the IEEE quotient bit for bit).
 FM_NI double fdiv_rn(double a, double b)
 {
-  if (!(div_rn_range_(a) && div_rn_range_(b))) return div_ieee_(a, b);
-  return div_rn_with_(a, b, frcp(b));
+  const uint32_t ah = hi_(a), al = lo_(a), bh = hi_(b), bl = lo_(b);
+  const uint32_t ea = (ah >> 20) & 0x7ffu, eb = (bh >> 20) & 0x7ffu, ex = ea - eb + 1023u;
+  if (ea - 1u >= 2046u || eb - 1u >= 2046u || ex - 2u >= 2044u) {
+    // 0 / b is common (an absent species): a signed zero
+    if (((ah << 1) | al) == 0u && eb - 1u < 2046u) return from_bits_((int64_t)((uint64_t)((ah ^ bh) & 0x80000000u) << 32));
+    return div_ieee_(a, b);
+  }
+  return quot_(ah, al, bh, bl, rcp_fixed_((bh & 0xfffffu) | 0x100000u, bl), ex);
 }
+
+FM_HD double fdiv(double a, double b) { return fdiv_rn(a, b); }
+
+// Two quotients with one divisor.
 FM_NI void fdiv_rn2(double a1, double a2, double b, double &q1, double &q2)
 {
-  if (!(div_rn_range_(a1) && div_rn_range_(a2) && div_rn_range_(b))) {
-    q1 = div_ieee_(a1, b);
-    q2 = div_ieee_(a2, b);
+  const uint32_t ah = hi_(a1), al = lo_(a1), ch = hi_(a2), cl = lo_(a2), bh = hi_(b), bl = lo_(b);
+  const uint32_t ea = (ah >> 20) & 0x7ffu, ec = (ch >> 20) & 0x7ffu, eb = (bh >> 20) & 0x7ffu;
+  if (ea - 1u >= 2046u || ec - 1u >= 2046u || eb - 1u >= 2046u || ea - eb + 1021u >= 2044u || ec - eb + 1021u >= 2044u) {
+    q1 = fdiv_rn(a1, b);
+    q2 = fdiv_rn(a2, b);
     return;
   }
-  const double y = frcp(b);
-  q1 = div_rn_with_(a1, b, y);
-  q2 = div_rn_with_(a2, b, y);
+  const uint64_t y = rcp_fixed_((bh & 0xfffffu) | 0x100000u, bl);
+  q1 = quot_(ah, al, bh, bl, y, ea - eb + 1023u);
+  q2 = quot_(ch, cl, bh, bl, y, ec - eb + 1023u);
 }
 
 // 1/sqrt(d) (see the header) for 2^-120 < d < 2^120; frsqrt_ok tells.
