@@ -1,31 +1,34 @@
-// fastmath.cuh — FP64 exp, exp10 and log that spend as few FP64 instructions
-// as the result's 53 bits need.
+// fastmath.cuh — FP64 exp, exp10, log, reciprocal, division, reciprocal
+// square root and arc tangent that spend few or no FP64 instructions.
 //
-// GB300 issues FP64 at 1/64 of its FP32 rate (a measured 1.0 TFLOP/s FMA),
-// and on it an FP64 compare, min/max or conversion costs as much as an FP64
-// FMA, while integer and FP32 instructions are almost free beside them.  The
-// microphysics kernels need a few dozen exp/log per grid point per sub-step,
-// so these functions do in FP64 only the steps that need 53 bits and move
-// the rest to the integer and FP32 pipes: range checks on the bit pattern,
-// the integer part of the argument reduction in FP32, int -> double by bit
-// construction, and the high-order polynomial terms (whose size is below
-// 2^-28 of the result, so FP32's 2^-24 suffices) in FP32.
+// GB300 issues FP64 at 1/64 of its FP32 rate (a measured 1.0 TFLOP/s FMA): a
+// warp's FP64 instruction holds the SM's pipe for 16 cycles, in which the four
+// schedulers could issue 64 others, and an FP64 compare, min/max or conversion
+// costs as much as an FMA.  The microphysics kernels need a few dozen of these
+// functions per grid point and ran the FP64 pipe at 78-85 % with 80-88 % of
+// the issue slots idle, so the functions work in 64-bit fixed point on the
+// integer pipe (32 x 32 -> 64-bit multiplies), to a few units of 2^-60 of the
+// result, rounded once: a function of ~70 integer instructions in place of 6-9
+// FP64 ones is about 1/6 of their cost, and more accurate (0.53 ulp instead of
+// about 1).  256x256x90, exp / log on FP64 -> integer: rain_ice 12.01 -> 9.60
+// ms, adjoint 24.8 -> 19.1 ms; ice_adjust (4.1 M points) 2.12 -> 1.61 ms;
+// sedimentation (65,535 x 87) 4.27 -> 2.88 ms.
 //
-//   fexp   P. T. P. Tang, "Table-driven implementation of the exponential
-//          function in IEEE floating-point arithmetic", ACM TOMS 15(2), 1989:
-//          x = (256 m + j) ln2/256 + r, |r| <= ln2/512; e^x = 2^m 2^(j/256) e^r,
-//          2^(j/256) tabulated as a double + float pair, e^r - 1 by its Taylor
-//          series (r, r^2/2 in FP64; r^3/6 and beyond in FP32).  6 FP64 ops.
-//   fexp10 the same with log10(2)/256 and r scaled by ln 10.  7 FP64 ops.
-//   flog   P. T. P. Tang, "Table-driven implementation of the logarithm
-//          function in IEEE floating-point arithmetic", ACM TOMS 16(4), 1990,
-//          with the reduction made exact: x = 2^e z, z in [1, 2) split into
-//          128 intervals by its leading 7 fraction bits, intervals above
-//          sqrt(2) folded to [sqrt(1/2), 1) (e + 1); invc, a reciprocal of the
-//          interval's centre rounded to 8 significant bits, makes
-//          r = z*invc - 1 exact in one FMA (|r| < 2^-7); log x = e ln2 -
-//          log(invc) + log1p(r), log1p by its Taylor series (to r^4 in FP64,
-//          r^5 .. r^8 in FP32).  9 FP64 ops.
+//   fexp   after P. T. P. Tang, "Table-driven implementation of the
+//          exponential function in IEEE floating-point arithmetic", ACM TOMS
+//          15(2), 1989: x = k ln2/512 + r, 0 < r < 2^-8.8 (k from an FP32
+//          estimate, one low so that every term of the series is positive;
+//          r exact modulo 2^-6 in units of 2^-70); e^x = 2^(k/512) e^r,
+//          2^(j/512) tabulated to 62 bits, e^r - 1 by its Taylor series to
+//          r^5.  Within 0.52 ulp.
+//   fexp10 the same with log10(2)/512 and r scaled by ln 10.
+//   flog   after P. T. P. Tang, "Table-driven implementation of the logarithm
+//          function in IEEE floating-point arithmetic", ACM TOMS 16(4), 1990:
+//          x = 2^e z, z in [1, 2) in 512 intervals; per interval an integer
+//          c = ceil(2048 / lower end) makes r = z c/2048 - 1 exact, 0 <= r <
+//          2^-8.4; log x = e ln2 - log(c/2048) + log1p(r), log1p by its Taylor
+//          series to r^7, the sum in 96 bits (2^-72).  Within 0.54 ulp.  Within
+//          2^-8 of x = 1, where the sum cancels, log1p(x - 1) in FP64.
 //   frcp   1/d and fdiv a/b, the IEEE results bit for bit, in integer
 //          arithmetic (no FP64 operation): with d = x 2^k, x in [1, 2), the
 //          hardware's FP32 reciprocal y0 of x (24 bits, |eps| = |1 - x y0| <
@@ -35,10 +38,9 @@
 //          the rounding settled by the exact remainder (a - q b modulo 2^64).
 //          A quotient of doubles is never halfway between two doubles, so the
 //          sign of |r| - |b|/2 decides; the seed's error cannot reach the
-//          result.  The FP64 pipe was 78 % busy with the issue slots 83 %
-//          idle; taking the 3 / 7 FP64 operations of a reciprocal / rounded
-//          division to the integer pipe gave rain_ice 13.60 -> 12.01 ms,
-//          the adjoint 26.3 -> 24.8 ms (256x256x90).  Where an operand is zero, subnormal, infinite or NaN, or
+//          result.  In place of 3 / 7 FP64 operations of a reciprocal /
+//          rounded division: rain_ice 13.60 -> 12.01 ms, adjoint 26.3 ->
+//          24.8 ms (256x256x90).  Where an operand is zero, subnormal, infinite or NaN, or
 //          the result leaves the normal range, the IEEE division.
 //   frsqrt 1/sqrt(d): y0 = the FP32 reciprocal of the FP32 square root of d
 //          (truncated to FP32; |eps| = |1 - d y0^2| < 2^-21), then
@@ -53,9 +55,8 @@
 //          tabulated.  ~15 FP64 ops.
 //
 // Accuracy: within 2 ulp (tests compare the host build of this code with
-// 200-bit mpmath values, and the device build with the host build bit for
-// bit).  Every FP64 and FP32 operation is an explicit fma or a separately
-// rounded add/multiply, so host and device builds agree exactly.  Special
+// 200-bit mpmath values).  Every FP64 and FP32 operation is an explicit fma or
+// a separately rounded add/multiply, so host and device builds agree exactly.  Special
 // inputs (NaN, infinities, zero, negative, subnormal, overflow and underflow
 // ranges) leave the fast path through one integer test and get the IEEE
 // results of exp/log.
@@ -85,13 +86,12 @@
 
 namespace fm {
 
-struct ExpEntry { double hi; float lo; int pad; };
 struct AtanEntry { double hi; float lo; int pad; };
-struct LogEntry { double invc, nlog_hi; float nlog_lo; int fold; double pad; };
+struct alignas(16) LogEntry { uint32_t c, n0, n1, n2; };
 
 #if defined(__CUDA_ARCH__)
-__device__ const ExpEntry kExpTable[256] = FM_EXP_TABLE_INIT;
-__device__ const LogEntry kLogTable[128] = FM_LOG_TABLE_INIT;
+__device__ const uint64_t kExpTable[512] = FM_EXP_TABLE_INIT;
+__device__ const LogEntry kLogTable[512] = FM_LOG_TABLE_INIT;
 __device__ const AtanEntry kAtanTable[65] = FM_ATAN_TABLE_INIT;
 __device__ const AtanEntry kAtanCTable[65] = FM_ATANC_TABLE_INIT;
 __device__ __forceinline__ void atan_entry(bool comp, int j, double &hi, float &lo)
@@ -102,19 +102,16 @@ __device__ __forceinline__ void atan_entry(bool comp, int j, double &hi, float &
 }
 __device__ __forceinline__ float rcpf_(float x) { return __frcp_rn(x); }
 __device__ __forceinline__ float sqrtf_(float x) { return __fsqrt_rn(x); }
-__device__ __forceinline__ void exp_entry(int j, double &hi, float &lo)
+__device__ __forceinline__ uint64_t exp_entry(uint32_t j)
 {
-  const double2 v = __ldg(reinterpret_cast<const double2 *>(kExpTable) + j);
-  hi = v.x;
-  lo = __int_as_float((int)(uint32_t)__double_as_longlong(v.y));
+  return __ldg(reinterpret_cast<const unsigned long long *>(kExpTable) + j);
 }
-__device__ __forceinline__ void log_entry(int i, double &invc, double &nlog_hi, float &nlog_lo, int &fold)
+__device__ __forceinline__ LogEntry log_entry(uint32_t i)
 {
-  const double2 *p = reinterpret_cast<const double2 *>(kLogTable) + 2 * i;
-  const double2 a = __ldg(p);
-  const float2 b = __ldg(reinterpret_cast<const float2 *>(p + 1));
-  invc = a.x; nlog_hi = a.y; nlog_lo = b.x; fold = __float_as_int(b.y);
+  const uint4 v = __ldg(reinterpret_cast<const uint4 *>(kLogTable) + i);
+  return {v.x, v.y, v.z, v.w};
 }
+__device__ __forceinline__ uint32_t funnel_l_(uint32_t lo, uint32_t hi, uint32_t n) { return __funnelshift_lc(lo, hi, n); }
 __device__ __forceinline__ double fma_(double a, double b, double c) { return __fma_rn(a, b, c); }
 __device__ __forceinline__ double add_(double a, double b) { return __dadd_rn(a, b); }
 __device__ __forceinline__ double mul_(double a, double b) { return __dmul_rn(a, b); }
@@ -137,8 +134,8 @@ __device__ __forceinline__ float rcp_seed_(float x)
   return y;
 }
 #else
-static const ExpEntry kExpTable[256] = FM_EXP_TABLE_INIT;
-static const LogEntry kLogTable[128] = FM_LOG_TABLE_INIT;
+static const uint64_t kExpTable[512] = FM_EXP_TABLE_INIT;
+static const LogEntry kLogTable[512] = FM_LOG_TABLE_INIT;
 static const AtanEntry kAtanTable[65] = FM_ATAN_TABLE_INIT;
 static const AtanEntry kAtanCTable[65] = FM_ATANC_TABLE_INIT;
 inline void atan_entry(bool comp, int j, double &hi, float &lo)
@@ -148,10 +145,11 @@ inline void atan_entry(bool comp, int j, double &hi, float &lo)
 }
 inline float rcpf_(float x) { volatile float r = 1.0f / x; return r; }
 inline float sqrtf_(float x) { volatile float r = std::sqrt(x); return r; }
-inline void exp_entry(int j, double &hi, float &lo) { hi = kExpTable[j].hi; lo = kExpTable[j].lo; }
-inline void log_entry(int i, double &invc, double &nlog_hi, float &nlog_lo, int &fold)
+inline uint64_t exp_entry(uint32_t j) { return kExpTable[j]; }
+inline LogEntry log_entry(uint32_t i) { return kLogTable[i]; }
+inline uint32_t funnel_l_(uint32_t lo, uint32_t hi, uint32_t n)
 {
-  invc = kLogTable[i].invc; nlog_hi = kLogTable[i].nlog_hi; nlog_lo = kLogTable[i].nlog_lo; fold = kLogTable[i].fold;
+  return n >= 32 ? lo : (uint32_t)((((uint64_t)hi << 32 | lo) << n) >> 32);
 }
 inline double fma_(double a, double b, double c) { return std::fma(a, b, c); }
 inline double add_(double a, double b) { volatile double s = a + b; return s; }
@@ -211,82 +209,98 @@ FM_HD int32_t rint_f32(float t)
   return fbits_(addf_(t, sh)) - fbits_(sh);
 }
 
-// 2^(k/256) * e^r * (1 - corr) for |r| <= ~ln2/512 and |corr| < 2^-40.
-FM_HD double exp_core(int32_t k, double r, float corr)
+// hi : lo of a 64 x 64-bit product's upper half, without the carry of the
+// lowest partial product (at most two units low).
+FM_HD uint64_t mulhi64_(uint64_t a, uint64_t b)
 {
-  const float rf = to_f32(r);
-  // (e^r - 1 - r - r^2/2) / r^3 = 1/6 + r/24 + r^2/120 (+ r^3/720 < 2^-31 of r^3/6)
-  float s = fmaf_(rf, 1.0f / 120.0f, 1.0f / 24.0f);
-  s = fmaf_(rf, s, 1.0f / 6.0f);
-  const double q = fma_(r, to_f64(s), 0.5);
-  const double p = fma_(mul_(r, r), q, r);                      // e^r - 1
-  double thi;
-  float tlo;
-  exp_entry(k & 255, thi, tlo);
-  // lo' = T_lo - T_hi*corr (both terms < 2^-38: FP32 carries them to 2^-62)
-  const float lo = fmaf_(-to_f32(thi), corr, tlo);
-  const double y = add_(thi, fma_(thi, p, to_f64(lo)));           // in [0.997, 2)
-  const int32_t m = k >> 8;
-  if (m >= -1021 && m <= 1022) return from_bits_(bits_(y) + (int64_t)m * ((int64_t)1 << 52));
+  const uint32_t ah = (uint32_t)(a >> 32), al = (uint32_t)a, bh = (uint32_t)(b >> 32), bl = (uint32_t)b;
+  return (uint64_t)ah * bh + mulhi_(ah, bl) + mulhi_(al, bh);
+}
+
+// The square of R 2^-70 in units of 2^-76 (at most two units low).
+FM_HD uint64_t sqr70_(uint64_t R)
+{
+  const uint32_t h = (uint32_t)(R >> 32), l = (uint32_t)R;
+  return (uint64_t)h * h + (((uint64_t)h * l) >> 31);
+}
+
+// x 2^70 modulo 2^64 plus `bias`, minus kb (cl + ch 2^32) 2^-32: the exact
+// argument reduction of fexp / fexp10 (|x| < 1024, kb < 2^21).
+FM_HD uint64_t exp_reduce_(uint32_t h, uint32_t l, uint64_t bias, uint32_t kb, uint64_t c, uint32_t clo)
+{
+  const uint32_t e = (h >> 20) & 0x7ffu;
+  const uint64_t m = ((uint64_t)((h & 0xfffffu) | 0x100000u) << 32) | l;
+  // 2^(e - 1075) m = m 2^(e - 1005) 2^-70; below 2^-18 the bits under 2^-70 drop
+  const uint32_t down = 1005u - e;
+  uint64_t X = e >= 1005u ? m << (e - 1005u) : (down < 64u ? m >> down : 0u);
+  if ((int32_t)h < 0) X = 0u - X;
+  const uint64_t kc = (uint64_t)kb * (uint32_t)c + ((uint64_t)(kb * (uint32_t)(c >> 32)) << 32);
+  return X + bias - kc - mulhi_(kb, clo);
+}
+
+// 2^(k/512) e^r for r = R 2^-70 in (0, 2^-8.8), k = kb - 2^20: T + T (e^r - 1)
+// with T = 2^(j/512) 2^62 from the table and
+// e^r - 1 = r + r^2/2 + r^3 (1/6 + r/24 + r^2/120), all terms positive, each
+// held to 2^-60 or better of the result; rounded once to 53 bits.
+FM_HD double exp_core_(uint64_t R, uint32_t kb)
+{
+  const uint64_t r2 = sqr70_(R);
+  const uint32_t r40 = (uint32_t)(R >> 30);                       // r 2^40
+  const uint32_t u = 357913941u + mulhi_(r40, 279620u);          // (1/24 + r/120) 2^33
+  const uint32_t t = 2863311531u + (mulhi_(r40, u) >> 7);        // (1/6 + r/24 + ...) 2^34
+  const uint32_t s = (uint32_t)(((uint64_t)r40 * t) >> 31);      // r times it, 2^43
+  const uint64_t p = (R >> 6) + (r2 >> 13) + (((uint64_t)(uint32_t)(r2 >> 27) * s) >> 28);   // (e^r - 1) 2^64
+  const uint64_t T = exp_entry(kb & 511u);
+  const uint64_t y = T + mulhi64_(T, p);                          // [2^62, 2^63.004)
+  const uint32_t ov = (uint32_t)(y >> 63);
+  const int32_t m = (int32_t)(kb >> 9) - 2048 + (int32_t)ov;
+  const uint64_t q = (y + (512u << ov)) >> (10u + ov);            // 53 bits
+  if (m >= -1022 && m <= 1022) return from_bits_((int64_t)(q + ((uint64_t)(uint32_t)(m + 1022) << 52)));
   // gradual underflow / overflow edges: scale in two steps
-  const double y1 = from_bits_(bits_(y) + (int64_t)(m / 2) * ((int64_t)1 << 52));
-  return mul_(y1, from_bits_((int64_t)(1023 + m - m / 2) << 52));
+  const double d = from_bits_((int64_t)(q + ((uint64_t)(uint32_t)(m / 2 + 1022) << 52)));
+  return mul_(d, from_bits_((int64_t)(1023 + m - m / 2) << 52));
+}
+
+// k + 2^20 with k the integer nearest x s less one (|x s| < 2^20, x as a
+// float to 2^-23: k is at most 1.6 below x s, and below it).
+FM_HD uint32_t exp_index_(float x, float s)
+{
+  const float sh = 12582912.0f;                                   // 1.5 * 2^23
+  return (uint32_t)(fbits_(fmaf_(x, s, sh)) - fbits_(sh)) + 1048575u;
 }
 
 // e^x.
 FM_NI double fexp(double x)
 {
-  const int64_t ax = bits_(x) & 0x7fffffffffffffffLL;
-  if (ax > 0x40861f0000000000LL) {                               // |x| > 707.875, inf, NaN
-    if (ax > 0x7ff0000000000000LL) return x;                     // NaN
+  const uint32_t h = hi_(x);
+  if ((h & 0x7fffffffu) >= 0x40862e43u) {                         // |x| > 709.78, inf, NaN
+    if (x != x) return x;
     if (x > 709.782712893384) return from_bits_(0x7ff0000000000000LL);
     if (x < -745.1332191019412) return 0.0;
   }
-  const int32_t k = rint_f32(mulf_(to_f32(x), FM_INV_L256_F));   // |k| < 2^18; off by one at most
-  const double kd = i2d(k);
-  const double r = fma_(-kd, FM_L256_HI, x);                     // one rounding, < 2^-62
-  return exp_core(k, r, mulf_((float)k, FM_L256_LO_F));
+  const uint32_t kb = exp_index_(to_f32(x), FM_INV_L512_F);
+  return exp_core_(exp_reduce_(h, lo_(x), FM_L512_BIAS, kb, FM_L512_HI, FM_L512_LO), kb);
 }
 
 // 10^x.
 FM_NI double fexp10(double x)
 {
-  const int64_t ax = bits_(x) & 0x7fffffffffffffffLL;
-  if (ax > 0x4073300000000000LL) {                               // |x| > 307, inf, NaN
-    if (ax > 0x7ff0000000000000LL) return x;
+  const uint32_t h = hi_(x);
+  if ((h & 0x7fffffffu) >= 0x40734413u) {                         // |x| > 308.25, inf, NaN
+    if (x != x) return x;
     if (x > 308.2547155599167) return from_bits_(0x7ff0000000000000LL);
     if (x < -323.60766413161369) return 0.0;
   }
-  const int32_t k = rint_f32(mulf_(to_f32(x), FM_INV_LG256_F));
-  const double kd = i2d(k);
-  const double r10 = fma_(-kd, FM_LG256_HI, x);                  // |r10| <= ~log10(2)/512
-  return exp_core(k, mul_(r10, FM_LN10), mulf_(mulf_((float)k, FM_LG256_LO_F), FM_LN10_F));
+  const uint32_t kb = exp_index_(to_f32(x), FM_INV_LG512_F);
+  const uint64_t r10 = exp_reduce_(h, lo_(x), FM_LG512_BIAS, kb, FM_LG512_HI, FM_LG512_LO);
+  return exp_core_(mulhi64_(r10, FM_LN10_62) << 2, kb);
 }
 
-// Natural logarithm.
-FM_NI double flog(double x)
+// log1p(r) for |r| <= 2^-8 (exact r = x - 1): r + r^2 q, q to r in FP64 and
+// from r^3 on in FP32.
+FM_NI double log_near1_(double x)
 {
-  int64_t b = bits_(x);
-  int ebias = 0;
-  if (b < 0x0010000000000000LL || b >= 0x7ff0000000000000LL) {   // <= 0, subnormal, inf, NaN
-    if (x != x) return x;
-    if (x < 0.0) return from_bits_(0x7ff8000000000000LL);
-    if (x == 0.0) return from_bits_((int64_t)0xfff0000000000000ULL);
-    if (b >= 0x7ff0000000000000LL) return x;                      // +inf
-    x = mul_(x, 18014398509481984.0);                              // subnormal: * 2^54
-    b = bits_(x);
-    ebias = -54;
-  }
-  double invc, nlog_hi;
-  float nlog_lo;
-  int fold;
-  log_entry((int)((b >> 45) & 127), invc, nlog_hi, nlog_lo, fold);
-  const int32_t e = (int32_t)(b >> 52) - 1023 + ebias + fold;
-  const double z = from_bits_((b & 0x000fffffffffffffLL) | 0x3ff0000000000000LL);
-  const double r = fma_(z, invc, -1.0);                          // exact
-  const double hi = fma_(i2d(e), FM_LN2_HI, nlog_hi);            // e*LN2_HI exact
-  const float lo = fmaf_((float)e, FM_LN2_LO_F, nlog_lo);        // < 2^-34: FP32 suffices
-  // (log1p(r) - r) / r^2 = -1/2 + r/3 - r^2/4 + r^3 s,  s = 1/5 - r/6 + r^2/7 - r^3/8
+  const double r = add_(x, -1.0);
   const float rf = to_f32(r);
   float s = fmaf_(rf, -1.0f / 8.0f, 1.0f / 7.0f);
   s = fmaf_(rf, s, -1.0f / 6.0f);
@@ -294,8 +308,51 @@ FM_NI double flog(double x)
   double q = fma_(r, to_f64(s), -0.25);
   q = fma_(r, q, 1.0 / 3.0);
   q = fma_(r, q, -0.5);
-  const double tail = fma_(mul_(r, r), q, to_f64(lo));
-  return add_(hi, add_(r, tail));
+  return fma_(mul_(r, r), q, r);
+}
+
+// Natural logarithm.
+FM_NI double flog(double x)
+{
+  uint32_t h = hi_(x), l = lo_(x);
+  uint32_t ebias = 77u;                                           // 1100 - 1023
+  if (h - 0x3fefe000u < 0x3000u) return log_near1_(x);            // 1 - 2^-8 <= x < 1 + 2^-8
+  if (h - 0x00100000u >= 0x7fe00000u) {                           // <= 0, subnormal, inf, NaN
+    if (x != x) return x;
+    if (x < 0.0) return from_bits_(0x7ff8000000000000LL);
+    if (x == 0.0) return from_bits_((int64_t)0xfff0000000000000ULL);
+    if (h >= 0x7ff00000u) return x;                               // +inf
+    x = mul_(x, 18014398509481984.0);                             // subnormal: * 2^54
+    h = hi_(x);
+    l = lo_(x);
+    ebias = 77u - 54u;
+  }
+  const LogEntry t = log_entry((h >> 11) & 511u);
+  const uint32_t eb = (h >> 20) + ebias;                          // e + 1100
+  // r 2^70 = (z c / 2048 - 1) 2^70, exact
+  const uint64_t zl = (uint64_t)l * t.c;
+  const uint32_t zh = ((h & 0xfffffu) | 0x100000u) * t.c + (uint32_t)(zl >> 32) - 0x80000000u;
+  const uint64_t R = (((uint64_t)zh << 32) | (uint32_t)zl) << 7;
+  // log1p(r) = r - r G, G = r/2 - r^2 K, K = 1/3 - r (1/4 - r (1/5 - r (1/6 - r/7)))
+  const uint64_t r2 = sqr70_(R);
+  const uint32_t r40 = (uint32_t)(R >> 30);                       // r 2^40
+  const uint32_t w = 715827883u - mulhi_(r40, 2396745u);         // (1/6 - r/7) 2^32
+  const uint32_t u = 1717986918u - (mulhi_(r40, w) >> 7);        // 2^33
+  const uint32_t v = 2147483648u - (mulhi_(r40, u) >> 8);        // 2^33
+  const uint64_t K = 0x5555555555555555ull - (((uint64_t)r40 * v) >> 9);   // 2^64
+  const uint64_t G = (R >> 1) - (mulhi64_(r2, K) >> 6);           // 2^70
+  const uint64_t L = (R << 2) - (mulhi64_(R, G) >> 4);            // log1p(r) 2^72
+  // V = eb ln2 + (table) + L in 96 bits, 2^-72
+  const uint64_t s0 = (uint64_t)eb * FM_LN2_W0 + t.n0 + (uint32_t)L;
+  const uint64_t s1 = (uint64_t)eb * FM_LN2_W1 + t.n1 + (uint32_t)(L >> 32) + (uint32_t)(s0 >> 32);
+  const uint32_t s2 = eb * FM_LN2_W2 + t.n2 + (uint32_t)(s1 >> 32);
+  // |V| (2^-72 low where negative), its 64 leading bits, rounded to 53
+  const uint32_t sg = (uint32_t)((int32_t)s2 >> 31);
+  const uint32_t v2 = s2 ^ sg, v1 = (uint32_t)s1 ^ sg, v0 = (uint32_t)s0 ^ sg;
+  const uint32_t lz = (uint32_t)clz32_(v2);                       // 0..32: |V| >= 2^-9
+  const uint64_t top = ((uint64_t)funnel_l_(v1, v2, lz) << 32) | funnel_l_(v0, v1, lz);
+  const uint64_t q = (top >> 11) + ((uint32_t)(top >> 10) & 1u);
+  return from_bits_((int64_t)(q + ((uint64_t)(1045u - lz) << 52) + ((uint64_t)(sg & 0x80000000u) << 32)));
 }
 
 // The IEEE 1/sqrt(d), out of line: the rare fallback of frsqrt.

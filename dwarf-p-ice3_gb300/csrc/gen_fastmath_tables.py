@@ -4,22 +4,20 @@ and rounded to nearest.
 
     python dwarf-p-ice3_gb300/csrc/gen_fastmath_tables.py
 
-exp (Tang, ACM TOMS 15(2), 1989): 2^(j/256), j = 0..255, as a double hi and
-a float lo (the rounding error of hi, < 2^-53, needs only ~20 bits).
+exp (after Tang, ACM TOMS 15(2), 1989, in fixed point): 2^(j/512), j = 0..511,
+as a 64-bit integer times 2^-62; ln2/512 and log10(2)/512 as a 64-bit integer
+times 2^-70 and 32 further bits, and 2^20 times each modulo 2^-6 (the bias
+that keeps the multiple positive).
 
 atan (table-driven reduction in the manner of Tang's methods): atan(j/64) and
 pi/2 - atan(j/64), j = 0..64, as a double hi and a float lo.
 
-log (Tang, ACM TOMS 16(4), 1990, with an exact reduction): the mantissa
-z in [1, 2) is split into 128 intervals by its 7 leading fraction bits.
-Intervals at or above sqrt(2) are folded (z/2, exponent + 1) so that results
-near x = 1 never cancel against e*ln2.  For each interval c is its centre
-(halved when folded) and invc a reciprocal of c rounded to 8 significant
-bits, so that r = z*invc - 1 is exact in one FMA; the two intervals that
-touch 1 use invc = 1 (log1p(r) alone, r exact).  The table stores
-invc_tab = invc (halved for folded intervals, so r = fma(z, invc_tab, -1)
-takes the unfolded z), -log(invc) of the unhalved reciprocal as a double hi
-and a float lo, and the exponent increment of the fold.
+log (after Tang, ACM TOMS 16(4), 1990, in fixed point): the significand z in
+[1, 2) is split into 512 intervals by its 9 leading fraction bits; per
+interval [z0, z0 + 1/512) the integer c = ceil(2048/z0), so that r = z c/2048
+- 1 is exact in 64 bits and not negative (r < 2^-8.4), and -log(c/2048) -
+1100 ln2 as a 96-bit integer times 2^-72 (the bias keeps the exponent's
+multiple of ln2 positive).
 """
 from __future__ import annotations
 
@@ -30,7 +28,6 @@ import numpy as np
 
 mp.mp.prec = 200
 HERE = os.path.dirname(os.path.abspath(__file__))
-FOLD = 53          # first interval [1 + 53/128, ...) at or above sqrt(2)
 
 
 def dbl(x) -> float:
@@ -41,12 +38,14 @@ def flt(x) -> float:
     return float(np.float32(dbl(x)))  # nearest float (values here are far from float ties)
 
 
-def round_bits(x, bits: int) -> float:
-    """x rounded to `bits` significant bits (exactly representable)."""
-    x = mp.mpf(x)
-    e = int(mp.floor(mp.log(x, 2)))
-    q = mp.mpf(2) ** (e - bits + 1)
-    return float(mp.nint(x / q) * q)
+def fix(x, bits: int) -> int:
+    """x 2^bits rounded to an integer."""
+    return int(mp.nint(mp.mpf(x) * mp.mpf(2) ** bits))
+
+
+def words(n: int, count: int):
+    """The 32-bit words of n modulo 2^(32 count), lowest first."""
+    return [(n >> (32 * i)) & 0xffffffff for i in range(count)]
 
 
 def fhex(v: float) -> str:
@@ -56,27 +55,17 @@ def fhex(v: float) -> str:
 def main() -> None:
     lines = ["// Generated by gen_fastmath_tables.py (mpmath, 200-bit) - do not edit.",
              "#pragma once", "",
-             "// 2^(j/256): {hi (double), lo (float)}, j = 0..255",
+             "// 2^(j/512) 2^62, j = 0..511",
              "#define FM_EXP_TABLE_INIT { \\"]
-    for j in range(256):
-        v = mp.mpf(2) ** (mp.mpf(j) / 256)
-        hi = dbl(v)
-        lo = flt(v - mp.mpf(hi))
-        lines.append(f"  {{{hi.hex()}, {fhex(lo)}, 0}}, \\")
+    for j in range(512):
+        lines.append(f"  {fix(mp.mpf(2) ** (mp.mpf(j) / 512), 62):#018x}ull, \\")
     lines += ["}", "",
-              "// per 7-bit mantissa interval: {invc_tab, -log(invc) hi, -log(invc) lo (float), fold}",
+              "// per 9-bit significand interval: {c, (-log(c/2048) - 1100 ln2) 2^72 in three words, lowest first}",
               "#define FM_LOG_TABLE_INIT { \\"]
-    for i in range(128):
-        centre = 1 + (mp.mpf(i) + mp.mpf(0.5)) / 128
-        fold = i >= FOLD
-        if fold:
-            centre = centre / 2
-        invc = 1.0 if i in (0, 127) else round_bits(1 / centre, 8)
-        v = -mp.log(mp.mpf(invc))
-        hi = dbl(v)
-        lo = flt(v - mp.mpf(hi))
-        invc_tab = invc / 2 if fold else invc
-        lines.append(f"  {{{invc_tab.hex()}, {hi.hex()}, {fhex(lo)}, {1 if fold else 0}, 0.0}}, \\")
+    for i in range(512):
+        c = -(-2048 * 512 // (512 + i))
+        w = words(fix(-mp.log(mp.mpf(c) / 2048) - 1100 * mp.log(2), 72), 3)
+        lines.append(f"  {{{c}u, {w[0]:#010x}u, {w[1]:#010x}u, {w[2]:#010x}u}}, \\")
     lines += ["}", "",
               "// atan(j/64): {hi (double), lo (float)}, j = 0..64",
               "#define FM_ATAN_TABLE_INIT { \\"]
@@ -91,18 +80,20 @@ def main() -> None:
         bh = dbl(b)
         lines.append(f"  {{{bh.hex()}, {fhex(flt(b - mp.mpf(bh)))}, 0}}, \\")
     lines += ["}", ""]
-    ln2_hi = round_bits(mp.log(2), 42)             # e*ln2_hi exact for |e| < 2^11
-    l256 = mp.log(2) / 256
-    lg256 = mp.log10(2) / 256
+    l512 = mp.log(2) / 512
+    lg512 = mp.log10(2) / 512
+    ln2 = words(fix(mp.log(2), 72), 3)
     consts = {
-        "FM_LN2_HI": ln2_hi.hex(), "FM_LN2_LO_F": fhex(flt(mp.log(2) - mp.mpf(ln2_hi))),
-        "FM_INV_L256_F": fhex(flt(256 / mp.log(2))),
-        "FM_L256_HI": dbl(l256).hex(), "FM_L256_LO_F": fhex(flt(l256 - mp.mpf(dbl(l256)))),
-        "FM_INV_LG256_F": fhex(flt(256 / mp.log10(2))),
-        "FM_LG256_HI": dbl(lg256).hex(), "FM_LG256_LO_F": fhex(flt(lg256 - mp.mpf(dbl(lg256)))),
-        "FM_LN10": dbl(mp.log(10)).hex(), "FM_LN10_F": fhex(flt(mp.log(10))),
+        "FM_INV_L512_F": fhex(flt(512 / mp.log(2))), "FM_INV_LG512_F": fhex(flt(512 / mp.log10(2))),
+        "FM_LN10_62": f"{fix(mp.log(10), 62):#018x}ull",
+        "FM_LN2_W0": f"{ln2[0]:#010x}u", "FM_LN2_W1": f"{ln2[1]:#010x}u", "FM_LN2_W2": f"{ln2[2]}u",
         "FM_PIO2": dbl(mp.pi / 2).hex(),
     }
+    for name, v in (("L512", l512), ("LG512", lg512)):
+        f102 = fix(v, 102)
+        consts[f"FM_{name}_HI"] = f"{f102 >> 32:#018x}ull"               # 2^-70 units
+        consts[f"FM_{name}_LO"] = f"{f102 & 0xffffffff:#010x}u"          # the next 32 bits
+        consts[f"FM_{name}_BIAS"] = f"{fix(v * 2 ** 20, 70) % 2 ** 64:#018x}ull"
     for k, v in consts.items():
         lines.append(f"#define {k} {v}")
     with open(os.path.join(HERE, "fastmath_tables.h"), "w") as f:
