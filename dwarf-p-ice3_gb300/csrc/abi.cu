@@ -160,20 +160,6 @@ int validate_ice_adjust(Handle *h, const Ice3gbIceAdjustFields *f, int nk)
   return ICE3GB_OK;
 }
 
-bool ia_vec2_ok(const Ice3gbIceAdjustFields *f, long n)
-{
-  if (n % 2) return false;
-  const void *ptrs[] = {f->pabs, f->sigs, f->th, f->exn, f->exn_ref, f->rho_dry_ref, f->rv, f->rc, f->ri, f->rr,
-                        f->rs, f->rg, f->cf_mf, f->rc_mf, f->ri_mf, f->rvs, f->rcs, f->ris, f->ths, f->t,
-                        f->rv_out, f->rc_out, f->ri_out, f->cldfr, f->hlc_hrc, f->hlc_hcf, f->hli_hri, f->hli_hcf,
-                        f->cph, f->lv, f->ls};
-  for (const void *p : ptrs)
-    if (!aligned16(p)) return false;
-  if (f->sigqsat_3d && !aligned16(f->sigqsat)) return false;
-  if (f->srcs && !aligned16(f->srcs)) return false;
-  return true;
-}
-
 int validate_sed(Handle *h, const Ice3gbSedimentationFields *f)
 {
   if (!f) return fail(h, ICE3GB_ERR_NULL, "fields pointer is NULL");
@@ -499,7 +485,7 @@ int run_physics_step(Handle *h, int nij, int nk, double dt, const Ice3gbRainIceO
   int rc = ICE3GB_OK;
   {
     ProfScope ps(h, K_ICE_ADJUST, s);
-    e = launch_ice_adjust(h->c, k1, nij, nk, dt, ia_vec2_ok(&a, n), h->num_sms, s);
+    e = launch_ice_adjust(h->c, k1, nij, nk, dt, h->num_sms, s);
   }
   if (e != cudaSuccess) rc = cuda_fail(h, e, "ice_adjust launch");
   // 2. rain_ice on the time-t state with S1
@@ -524,9 +510,8 @@ int run_physics_step(Handle *h, int nij, int nk, double dt, const Ice3gbRainIceO
     b.hlc_hrc = f->hlc_hrc; b.hlc_hcf = f->hlc_hcf; b.hli_hri = f->hli_hri; b.hli_hcf = f->hli_hcf;
     k2.rrs = f->rrs; k2.rss = f->rss; k2.rgs = f->rgs;
     k2.adv_dt = dt;
-    const bool v2 = ia_vec2_ok(&b, n) && aligned16(f->rrs) && aligned16(f->rss) && aligned16(f->rgs);
     ProfScope ps(h, K_ICE_ADJUST, s);
-    e = launch_ice_adjust(h->c, k2, nij, nk, dt, v2, h->num_sms, s);
+    e = launch_ice_adjust(h->c, k2, nij, nk, dt, h->num_sms, s);
     if (e != cudaSuccess) rc = cuda_fail(h, e, "ice_adjust launch");
   }
   cudaFreeAsync(scr, s);
@@ -1002,7 +987,7 @@ int ice3gb_ice_adjust(void *handle, int nij, int nk, double dt, const Ice3gbIceA
   cudaError_t e;
   {
     ProfScope ps(h, K_ICE_ADJUST, static_cast<cudaStream_t>(stream));
-    e = launch_ice_adjust(h->c, kf, nij, nk, dt, ia_vec2_ok(f, n), h->num_sms, static_cast<cudaStream_t>(stream));
+    e = launch_ice_adjust(h->c, kf, nij, nk, dt, h->num_sms, static_cast<cudaStream_t>(stream));
   }
   if (e != cudaSuccess) return cuda_fail(h, e, "ice_adjust launch");
   return ICE3GB_OK;
@@ -1273,7 +1258,7 @@ int ice3gb_ice_adjust_host(void *handle, int nij, int nk, double dt, const Ice3g
   kf.tiwmx = h->d_tiwmx;
   {
     ProfScope ps(h, K_ICE_ADJUST, s);
-    e = launch_ice_adjust(h->c, kf, nij, nk, dt, ia_vec2_ok(&d, (long)n), h->num_sms, s);
+    e = launch_ice_adjust(h->c, kf, nij, nk, dt, h->num_sms, s);
   }
   if (e != cudaSuccess) return cuda_fail(h, e, "ice_adjust launch");
   for (int i = 0; i < 4 && e == cudaSuccess; ++i) e = cudaMemcpyAsync(*io_src[i], *io_dst[i], b3, cudaMemcpyDeviceToHost, s);

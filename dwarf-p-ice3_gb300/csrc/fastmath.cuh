@@ -42,17 +42,17 @@
 //          rounded division: rain_ice 13.60 -> 12.01 ms, adjoint 26.3 ->
 //          24.8 ms (256x256x90).  Where an operand is zero, subnormal, infinite or NaN, or
 //          the result leaves the normal range, the IEEE division.
-//   frsqrt 1/sqrt(d): y0 = the FP32 reciprocal of the FP32 square root of d
-//          (truncated to FP32; |eps| = |1 - d y0^2| < 2^-21), then
-//          y0 (1 + eps/2 + 3 eps^2/8), the series of (1 - eps)^(-1/2) to its
-//          quadratic term (remainder 5 eps^3/16 < 2^-63).  5 FP64 ops, within
-//          1 ulp; outside 2^-120 < d < 2^120 (and for zero, negative, inf,
-//          NaN) 1 / sqrt(d).
+//   frsqrt 1/sqrt(d) in the same way: d = x 4^k, x in [1, 4); y0 = the FP32
+//          reciprocal of the FP32 square root of x (24 bits, |eps| = |1 - x
+//          y0^2| < 2^-21, exact in integers), y0 (1 + eps/2 + 3 eps^2/8), the
+//          series of (1 - eps)^(-1/2) to its quadratic term (remainder below
+//          2^-64), rounded once: within 0.51 ulp, no FP64 operation.
 //   fatan  reduction to [0, 1] by atan(x) = pi/2 - atan(1/x), then
 //          atan(y) = atan(c) + atan(r), c = j/64 the nearest table point,
-//          r = (y - c)/(1 + y c) (|r| <= 1/128), atan(r) by its Taylor series
-//          (r^3 in FP64, r^5 .. r^9 in FP32); atan(c) and pi/2 - atan(c)
-//          tabulated.  ~15 FP64 ops.
+//          r = (y - c)/(1 + y c) (|r| <= 1/128; for y = 1/|x| numerator and
+//          denominator times |x|, so that one division serves), atan(r) by
+//          its Taylor series (r^3 in FP64, r^5 .. r^9 in FP32); atan(c) and
+//          pi/2 - atan(c) tabulated.  8 FP64 ops.
 //
 // Accuracy: within 2 ulp (tests compare the host build of this code with
 // 200-bit mpmath values).  Every FP64 and FP32 operation is an explicit fma or
@@ -355,9 +355,6 @@ FM_NI double flog(double x)
   return from_bits_((int64_t)(q + ((uint64_t)(1045u - lz) << 52) + ((uint64_t)(sg & 0x80000000u) << 32)));
 }
 
-// The IEEE 1/sqrt(d), out of line: the rare fallback of frsqrt.
-FM_NI double rsqrt_ieee_(double d) { return 1.0 / sqrt(d); }
-
 // the IEEE division, out of line (the rare fallback of the paths below)
 FM_NI double div_ieee_(double a, double b) { return a / b; }
 
@@ -449,22 +446,54 @@ FM_NI void fdiv_rn2(double a1, double a2, double b, double &q1, double &q2)
   q2 = quot_(ch, cl, bh, bl, y, ec - eb + 1023u);
 }
 
-// 1/sqrt(d) (see the header) for 2^-120 < d < 2^120; frsqrt_ok tells.
-FM_HD bool frsqrt_ok(double d)
+// The IEEE 1/sqrt(d), out of line (the rare fallback).
+FM_NI double rsqrt_ieee_(double d) { return 1.0 / sqrt(d); }
+
+// x = X 2^-52 in [1, 4) and d = x 4^k for a positive normal d.
+FM_HD void sqrt_split_(uint32_t h, uint32_t l, uint64_t &X, uint32_t &odd)
 {
-  const int64_t e = bits_(d) >> 52;                               // the sign bit makes e >= 2048
-  return e >= 1023 - 120 && e <= 1023 + 120;
+  odd = ~(h >> 20) & 1u;                                          // E - 1023 odd
+  X = (((uint64_t)((h & 0xfffffu) | 0x100000u) << 32) | l) << odd;
 }
-FM_HD double frsqrt(double d)
+
+// 1/sqrt(x) to within 2^-60 as a fixed-point fraction, Y 2^-62 in (1/2, 1].
+FM_HD uint64_t rsqrt_fixed_(uint64_t X, uint32_t odd)
 {
-  if (!frsqrt_ok(d)) return rsqrt_ieee_(d);                       // zero, tiny, huge, negative, inf, NaN
-  const double y0 = to_f64(rcpf_(sqrtf_(to_f32(d))));
-  const double eps = fma_(-d, mul_(y0, y0), 1.0);                  // y0^2 exact (24-bit y0)
-  return fma_(mul_(y0, eps), fma_(eps, 0.375, 0.5), y0);
+  const uint32_t xh = (uint32_t)(X >> 32), xl = (uint32_t)X;
+  // x truncated to FP32: the leading 24 bits of X
+  const uint32_t m = (uint32_t)(X >> (29u + odd));                // 24 bits
+  const float xf = ffrom_bits_((int32_t)(((127u + odd) << 23) | (m & 0x7fffffu)));
+  const uint32_t yb = (uint32_t)fbits_(rcpf_(sqrtf_(xf)));
+  const uint32_t y0 = ((yb < 0x3f7fffffu ? yb : 0x3f7fffffu) & 0x7fffffu) | 0x800000u;   // y0 2^24
+  // eps 2^80 = 2^80 - x y0^2 2^80 from the middle of the 102-bit product x 2^52 y0^2 2^48
+  const uint64_t s = (uint64_t)y0 * y0;
+  const uint32_t sl = (uint32_t)s, sh = (uint32_t)(s >> 32);
+  const uint64_t p0 = (uint64_t)xl * sl;
+  const uint64_t mid = (uint64_t)xl * sh + (uint64_t)xh * sl + (p0 >> 32);
+  const uint64_t top = (mid >> 32) + (uint64_t)(xh * sh);
+  const int64_t e = (int64_t)(0u - ((top << 44) + ((uint64_t)(uint32_t)mid << 12) + ((uint32_t)p0 >> 20)));
+  const int32_t eh = (int32_t)(e >> 32);
+  const int64_t w = (e >> 1) + ((3 * ((int64_t)eh * eh)) >> 19);  // eps/2 + 3 eps^2/8
+  const int64_t t = (int64_t)(int32_t)(w >> 32) * (int32_t)y0 + (int64_t)mulhi_((uint32_t)w, y0);   // y0 w 2^72
+  return ((uint64_t)y0 << 38) + (uint64_t)(t >> 10);
+}
+
+// 1/sqrt(d) for a positive normal d; frsqrt_ok tells.
+FM_HD bool frsqrt_ok(double d) { return hi_(d) - 0x00100000u < 0x7fe00000u; }
+FM_NI double frsqrt(double d)
+{
+  if (!frsqrt_ok(d)) return rsqrt_ieee_(d);                       // zero, subnormal, negative, inf, NaN
+  const uint32_t h = hi_(d);
+  uint64_t X;
+  uint32_t odd;
+  sqrt_split_(h, lo_(d), X, odd);
+  const uint64_t q = (rsqrt_fixed_(X, odd) + 256u) >> 9;          // [2^52, 2^53]
+  const uint32_t k2 = (h >> 20) - odd;                            // 2 k + 1023
+  return from_bits_((int64_t)(q + ((uint64_t)(1021u + 511u - (k2 >> 1)) << 52)));
 }
 
 // Arc tangent (see the header).
-FM_HD double fatan(double x)
+FM_NI double fatan(double x)
 {
   const int64_t b = bits_(x), ab = b & 0x7fffffffffffffffLL;
   if (ab < 0x3e10000000000000LL) return x;                        // |x| < 2^-30: atan x = x (1 - x^2/3), +-0
@@ -474,10 +503,12 @@ FM_HD double fatan(double x)
   }
   const bool comp = ab > 0x3ff0000000000000LL;                    // |x| > 1: pi/2 - atan(1/|x|)
   const double ax = from_bits_(ab);
-  const double y = comp ? frcp(ax) : ax;
-  const int32_t j = rint_f32(mulf_(to_f32(y), 64.0f));            // 0..64
+  const float xf = to_f32(ax);
+  const int32_t j = rint_f32(mulf_(comp ? rcpf_(xf) : xf, 64.0f));   // 0..64
   const double c = j == 0 ? 0.0 : from_bits_(bits_(i2d(j)) - ((int64_t)6 << 52));   // j/64, exact
-  const double r = mul_(add_(y, -c), frcp(fma_(y, c, 1.0)));      // y - c exact (Sterbenz)
+  // r = (y - c) / (1 + y c), y = |x| or 1/|x| (then numerator and denominator times |x|)
+  const double num = comp ? fma_(-c, ax, 1.0) : add_(ax, -c);
+  const double r = fdiv_rn(num, comp ? add_(ax, c) : fma_(ax, c, 1.0));
   const double r2 = mul_(r, r);
   const float r2f = to_f32(r2);
   // (atan r - r) / r^3 = -1/3 + r^2 (1/5 - r^2/7 + r^4/9)

@@ -102,6 +102,8 @@ ICE3_HD bool negd(double x) { return fm::bits_(x) < 0 && fm::bits_(x) != INT64_M
 ICE3_HD bool abs_gtp(double a, double b) { return (fm::bits_(a) & 0x7fffffffffffffffLL) > fm::bits_(b); }
 // a != 0 (nor -0), on the bit pattern.
 ICE3_HD bool nz(double a) { return (opaque_bits(a) << 1) != 0; }
+// neither infinite nor NaN.
+ICE3_HD bool finite_(double a) { return (fm::hi_(a) & 0x7fffffffu) < 0x7ff00000u; }
 // True on every lane when the predicate holds on some active lane of the warp:
 // a block of arithmetic that is exact when skipped on lanes whose inputs are
 // zero runs for the warp or for none of it (the host build: the lane alone).
@@ -159,11 +161,5 @@ ICE3_HD double tiwmx_at(const double *tab, double t)
 }
 
 #if defined(__CUDACC__)
-// 128-bit streaming accessors (LDG.128 / STG.128).
-__device__ __forceinline__ double2 ld2(const double *p, long i) { return __ldg(reinterpret_cast<const double2 *>(p + i)); }
-__device__ __forceinline__ void st2(double *p, long i, double a, double b)
-{
-  __stcs(reinterpret_cast<double2 *>(p + i), make_double2(a, b));
-}
 __device__ __forceinline__ double ld1(const double *p, long i) { return __ldg(p + i); }
 #endif

@@ -174,7 +174,7 @@ constexpr int kTiwmxTableN = 24117, kTiwmxTables = 6;
 void tiwmx_tables(const Ice3gbConstants &c, double *tab);
 
 cudaError_t launch_ice_adjust(const Ice3gbConstants &c, const IaKernelFields &kf, int nij, int nk, double dt,
-                              bool vec2, int num_sms, cudaStream_t s);
+                              int num_sms, cudaStream_t s);
 cudaError_t launch_sedimentation(const Ice3gbConstants &c, const SedArgs &a, cudaStream_t s);
 cudaError_t launch_fog_deposition(const Ice3gbConstants &c, const FogArgs &a, cudaStream_t s);
 cudaError_t launch_rain_ice_points(const Ice3gbConstants &c, const RainIceArgs &a, int num_sms, cudaStream_t s);

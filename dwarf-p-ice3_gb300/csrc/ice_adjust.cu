@@ -1,10 +1,8 @@
 // ice_adjust.cu — saturation adjustment with CB02 subgrid condensation.
 //
 // Restates src/ice3/jax/stencils/ice_adjust.py:26-398 (IceAdjustJAX) for one
-// grid point per lane; each thread owns two consecutive points so every field
-// moves with one 128-bit load/store (LDG.128/STG.128).  Pure map over the
-// nij*nk points: 19 3-D fields read (+ sigqsat per column), 16 written,
-// 280 algorithmic bytes per point.
+// grid point per lane.  Pure map over the nij*nk points: 19 3-D fields read
+// (+ sigqsat per column), 16 written, 280 algorithmic bytes per point.
 #include <cmath>
 
 #include "ice3gb_device.cuh"
@@ -14,86 +12,32 @@
 namespace {
 using namespace ice3ia;
 
-// Two points per thread, double2 loads/stores; requires an even point count
-// and 16-byte aligned fields (checked by the host).  ADV: the state adjusted
-// is adv_dt times the sources (th = dt*ths, r = dt*rs, the state after the
-// microphysics in the chained physics step) instead of th/rv/.../rg, which
-// are then not read; rrs/rss/rgs are read instead.  Output pointers may be
-// NULL in the internal chained use (store skipped).
-// Blocks of 256 per SM the registers are capped for: the default leaves
-// 158-162 registers (one block, 8 warps per SM); two blocks (128 registers)
-// measured 35.67 against 35.58 ms per launch at 1024x1024x90, three (80
-// registers, spilling) 39.95 against 39.43 ms before the saturation terms
-// were skipped by their weight.
-#ifndef IA_MIN_BLOCKS
-#define IA_MIN_BLOCKS 1
-#endif
-template <bool ADV, bool SRC>
-__global__ void __launch_bounds__(256, IA_MIN_BLOCKS) ice_adjust_v2_kernel(const __grid_constant__ Cst c,
-                                                            const __grid_constant__ IaKernelFields kf,
-                                                            long npairs, int nij, double dt)
+// p mod nij, in 32 bits where p allows it (a 64-bit remainder is a call of
+// ~100 instructions).
+__device__ __forceinline__ long column_of(long p, int nij)
 {
-  const Ice3gbIceAdjustFields &f = kf.f;
-  const double inv_dt = 1.0 / dt;
-  const IaDerived d = ia_derived(c);
-  for (long q = blockIdx.x * (long)blockDim.x + threadIdx.x; q < npairs; q += (long)gridDim.x * blockDim.x) {
-    const long p = 2 * q;
-    IaIn x0, x1;
-#define LD2(field, name)                 \
-  {                                      \
-    const double2 v = ld2(f.field, p);   \
-    x0.name = v.x;                       \
-    x1.name = v.y;                       \
-  }
-    LD2(pabs, pabs) LD2(sigs, sigs) LD2(exn, exn) LD2(exn_ref, exn_ref) LD2(rho_dry_ref, rho)
-    LD2(cf_mf, cf_mf) LD2(rc_mf, rc_mf) LD2(ri_mf, ri_mf)
-    LD2(rvs, rvs) LD2(rcs, rcs) LD2(ris, ris) LD2(ths, ths)
-    if (ADV) {
-      const double a = kf.adv_dt;
-      const double2 vr = ld2(kf.rrs, p), vs = ld2(kf.rss, p), vg = ld2(kf.rgs, p);
-      x0.th = a * x0.ths; x1.th = a * x1.ths;
-      x0.rv = a * x0.rvs; x1.rv = a * x1.rvs;
-      x0.rc = a * x0.rcs; x1.rc = a * x1.rcs;
-      x0.ri = a * x0.ris; x1.ri = a * x1.ris;
-      x0.rr = a * vr.x;   x1.rr = a * vr.y;
-      x0.rs = a * vs.x;   x1.rs = a * vs.y;
-      x0.rg = a * vg.x;   x1.rg = a * vg.y;
-    } else {
-      LD2(th, th) LD2(rv, rv) LD2(rc, rc) LD2(ri, ri) LD2(rr, rr) LD2(rs, rs) LD2(rg, rg)
-    }
-#undef LD2
-    if (f.sigqsat_3d) {
-      const double2 v = ld2(f.sigqsat, p);
-      x0.sigqsat = v.x;
-      x1.sigqsat = v.y;
-    } else {
-      x0.sigqsat = ld1(f.sigqsat, p % nij);
-      x1.sigqsat = ld1(f.sigqsat, (p + 1) % nij);
-    }
-    IaOut o0, o1;
-    double s0 = 0.0, s1 = 0.0;
-    ia_point(c, d, dt, inv_dt, x0, o0, SRC ? &s0 : nullptr);
-    ia_point(c, d, dt, inv_dt, x1, o1, SRC ? &s1 : nullptr);
-    if (SRC) st2(f.srcs, p, s0, s1);
-#define ST2(field) if (f.field) st2(f.field, p, o0.field, o1.field);
-    ST2(t) ST2(rv_out) ST2(rc_out) ST2(ri_out) ST2(cldfr) ST2(hlc_hrc) ST2(hlc_hcf) ST2(hli_hri) ST2(hli_hcf)
-    ST2(cph) ST2(lv) ST2(ls) ST2(rvs) ST2(rcs) ST2(ris) ST2(ths)
-#undef ST2
-  }
+  return p <= 0xffffffffL ? (long)((unsigned)p % (unsigned)nij) : p % nij;
 }
 
-// Scalar path: odd point counts or unaligned fields.
+// One point per thread.  ADV: the state adjusted is adv_dt times the sources
+// (th = dt*ths, r = dt*rs, the state after the microphysics in the chained
+// physics step) instead of th/rv/.../rg, which are then not read; rrs/rss/rgs
+// are read instead.  Output pointers may be NULL in the internal chained use
+// (store skipped).
+// Bound: the FP64 pipe (about 115 operations per point; 1.4 TB/s of HBM).
+// 126 registers, two blocks per SM; two points per thread with 128-bit
+// accesses (152 registers, one block) took 22.45 against 19.26 ms per launch
+// at 1024x1024x90, and with the registers capped for two / three / four
+// blocks either form stays within 19.2-19.5 ms.
 template <bool ADV, bool SRC>
-__global__ void __launch_bounds__(256) ice_adjust_v1_kernel(const __grid_constant__ Cst c,
+__global__ void __launch_bounds__(256) ice_adjust_kernel(const __grid_constant__ Cst c,
                                                             const __grid_constant__ IaKernelFields kf,
-                                                            long n, int nij, double dt)
+                                                            long n, int nij, double dt, double inv_dt, const __grid_constant__ IaDerived d)
 {
   const Ice3gbIceAdjustFields &f = kf.f;
-  const double inv_dt = 1.0 / dt;
-  const IaDerived d = ia_derived(c);
   for (long p = blockIdx.x * (long)blockDim.x + threadIdx.x; p < n; p += (long)gridDim.x * blockDim.x) {
     IaIn x;
-    x.sigqsat = f.sigqsat_3d ? ld1(f.sigqsat, p) : ld1(f.sigqsat, p % nij);
+    x.sigqsat = f.sigqsat_3d ? ld1(f.sigqsat, p) : ld1(f.sigqsat, column_of(p, nij));
     x.pabs = ld1(f.pabs, p); x.sigs = ld1(f.sigs, p); x.exn = ld1(f.exn, p);
     x.exn_ref = ld1(f.exn_ref, p); x.rho = ld1(f.rho_dry_ref, p);
     x.cf_mf = ld1(f.cf_mf, p); x.rc_mf = ld1(f.rc_mf, p); x.ri_mf = ld1(f.ri_mf, p);
@@ -122,14 +66,12 @@ __global__ void __launch_bounds__(256) ice_adjust_v1_kernel(const __grid_constan
 template <bool SRC>
 __global__ void __launch_bounds__(256) ice_adjust_ocnd2_kernel(const __grid_constant__ Cst c,
                                                                const __grid_constant__ IaKernelFields kf, long n,
-                                                               int nij, int nk, double dt)
+                                                               int nij, int nk, double dt, double inv_dt, const __grid_constant__ IaDerived d)
 {
   const Ice3gbIceAdjustFields &f = kf.f;
-  const double inv_dt = 1.0 / dt;
-  const IaDerived d = ia_derived(c);
   for (long p = blockIdx.x * (long)blockDim.x + threadIdx.x; p < n; p += (long)gridDim.x * blockDim.x) {
     IaIn x;
-    x.sigqsat = f.sigqsat_3d ? ld1(f.sigqsat, p) : ld1(f.sigqsat, p % nij);
+    x.sigqsat = f.sigqsat_3d ? ld1(f.sigqsat, p) : ld1(f.sigqsat, column_of(p, nij));
     x.pabs = ld1(f.pabs, p); x.sigs = ld1(f.sigs, p); x.exn = ld1(f.exn, p);
     x.exn_ref = ld1(f.exn_ref, p); x.rho = ld1(f.rho_dry_ref, p);
     x.cf_mf = ld1(f.cf_mf, p); x.rc_mf = ld1(f.rc_mf, p); x.ri_mf = ld1(f.ri_mf, p);
@@ -186,39 +128,30 @@ void tiwmx_tables(const Cst &c, double *tab)
   }
 }
 
-cudaError_t launch_ice_adjust(const Cst &c, const IaKernelFields &kf, int nij, int nk, double dt, bool vec2,
-                              int num_sms, cudaStream_t s)
+cudaError_t launch_ice_adjust(const Cst &c, const IaKernelFields &kf, int nij, int nk, double dt, int num_sms,
+                              cudaStream_t s)
 {
   const long n = (long)nij * nk;
   const int threads = 256;
   const long cap = (long)num_sms * 64;
   const bool adv = kf.adv_dt != 0.0;
   const bool src = kf.f.srcs != nullptr;
+  const double inv_dt = 1.0 / dt;
+  const IaDerived d = ia_derived(c);
   if (c.OCND2 != 0.0) {   // (the host rejects OCND2 with adv_dt)
     long blocks = (n + threads - 1) / threads;
     if (blocks > cap) blocks = cap;
-    if (src) ice_adjust_ocnd2_kernel<true><<<(unsigned)blocks, threads, 0, s>>>(c, kf, n, nij, nk, dt);
-    else ice_adjust_ocnd2_kernel<false><<<(unsigned)blocks, threads, 0, s>>>(c, kf, n, nij, nk, dt);
-  } else if (vec2) {
-    const long npairs = n / 2;
-    long blocks = (npairs + threads - 1) / threads;
-    if (blocks > cap) blocks = cap;
-    if (src) {
-      if (adv) ice_adjust_v2_kernel<true, true><<<(unsigned)blocks, threads, 0, s>>>(c, kf, npairs, nij, dt);
-      else ice_adjust_v2_kernel<false, true><<<(unsigned)blocks, threads, 0, s>>>(c, kf, npairs, nij, dt);
-    } else {
-      if (adv) ice_adjust_v2_kernel<true, false><<<(unsigned)blocks, threads, 0, s>>>(c, kf, npairs, nij, dt);
-      else ice_adjust_v2_kernel<false, false><<<(unsigned)blocks, threads, 0, s>>>(c, kf, npairs, nij, dt);
-    }
+    if (src) ice_adjust_ocnd2_kernel<true><<<(unsigned)blocks, threads, 0, s>>>(c, kf, n, nij, nk, dt, inv_dt, d);
+    else ice_adjust_ocnd2_kernel<false><<<(unsigned)blocks, threads, 0, s>>>(c, kf, n, nij, nk, dt, inv_dt, d);
   } else {
     long blocks = (n + threads - 1) / threads;
     if (blocks > cap) blocks = cap;
     if (src) {
-      if (adv) ice_adjust_v1_kernel<true, true><<<(unsigned)blocks, threads, 0, s>>>(c, kf, n, nij, dt);
-      else ice_adjust_v1_kernel<false, true><<<(unsigned)blocks, threads, 0, s>>>(c, kf, n, nij, dt);
+      if (adv) ice_adjust_kernel<true, true><<<(unsigned)blocks, threads, 0, s>>>(c, kf, n, nij, dt, inv_dt, d);
+      else ice_adjust_kernel<false, true><<<(unsigned)blocks, threads, 0, s>>>(c, kf, n, nij, dt, inv_dt, d);
     } else {
-      if (adv) ice_adjust_v1_kernel<true, false><<<(unsigned)blocks, threads, 0, s>>>(c, kf, n, nij, dt);
-      else ice_adjust_v1_kernel<false, false><<<(unsigned)blocks, threads, 0, s>>>(c, kf, n, nij, dt);
+      if (adv) ice_adjust_kernel<true, false><<<(unsigned)blocks, threads, 0, s>>>(c, kf, n, nij, dt, inv_dt, d);
+      else ice_adjust_kernel<false, false><<<(unsigned)blocks, threads, 0, s>>>(c, kf, n, nij, dt, inv_dt, d);
     }
   }
   return cudaGetLastError();

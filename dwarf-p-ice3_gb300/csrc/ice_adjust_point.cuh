@@ -59,7 +59,7 @@ static const double kSrc1dHost[34] = {ICE3_SRC_1D_VALUES};
 
 // PSIGRC of condensation.F90:566-571 from q1, times the CB lambda3 factor
 // min(3, max(1, 1 - q1)) of :638-647 when LAMBDA3 = CB (0).
-ICE3_HD double sigrc_cb(const Cst &c, double q1)
+ICE3_HD double sigrc_cb(int lambda3, double q1)
 {
   const double x = 2.0 * nmin(100.0, nmax(-100.0, q1));
   const int i = (int)floor(x);
@@ -71,7 +71,7 @@ ICE3_HD double sigrc_cb(const Cst &c, double q1)
   const double s0 = kSrc1dHost[inq1 + 22], s1 = kSrc1dHost[inq1 + 23];
 #endif
   double r = nmin(1.0, (1.0 - inc) * s0 + inc * s1);
-  if ((int)c.LAMBDA3 == 0) r *= nmin(3.0, nmax(1.0, 1.0 - q1));
+  if (lambda3 == 0) r *= nmin(3.0, nmax(1.0, 1.0 - q1));
   return r;
 }
 
@@ -134,15 +134,35 @@ ICE3_HD void icecloud(const Cst &c, double p, double z, double dz, double t, dou
   ssiu = nmax(0.0, ssiu) - 1.0;
 }
 
-// Constants derived once per thread (divisions of table constants).
+// Constants derived once per call on the host (divisions and differences of
+// table constants, and the option switches as integers: formed per thread
+// they were ~40 FP64 operations beside the ~110 of a point).
 struct IaDerived {
   double rdrv, rvrd, irv;   // RD/RV, RV/RD, 1/RV
-  double imix;              // the reciprocal of TMAXMIX - TMINMIX that fm::fdiv would form per point
+  double imix;              // the reciprocal of TMAXMIX - TMINMIX
+  double cpv_cl, cpv_ci;    // CPV - CL, CPV - CI
+  int nrr, fmode, mfpdf, lambda3;
+  int subg, sig_full;       // LSUBG_COND; LSIGMAS and not LSTATNW
 };
 ICE3_HD IaDerived ia_derived(const Cst &c)
 {
-  return {c.RD / c.RV, c.RV / c.RD, 1.0 / c.RV, fm::frcp(c.TMAXMIX - c.TMINMIX)};
+  return {c.RD / c.RV, c.RV / c.RD, 1.0 / c.RV, fm::frcp(c.TMAXMIX - c.TMINMIX), c.CPV - c.CL, c.CPV - c.CI,
+          (int)c.NRR, (int)c.FRAC_ICE_ADJUST, (int)c.SUBG_MF_PDF, (int)c.LAMBDA3,
+          c.LSUBG_COND != 0.0, c.LSIGMAS != 0.0 && c.LSTATNW == 0.0};
 }
+
+// min(e, 0.99 p): the product only where a lane of the warp has e above p / 4
+// (an exponent two below; e and p positive normals, else the full form).
+ICE3_HD double cap_pressure(double e, double p)
+{
+  const bool small = pos(e) && fm::hi_(e) < 0x7ff00000u && (int32_t)(fm::hi_(e) + 0x00200000u) < (int32_t)fm::hi_(p) &&
+                     fm::hi_(p) < 0x7ff00000u;
+  if (warp_any(!small)) e = nmin(e, 0.99 * p);
+  return e;
+}
+// |q1| above which 0.5 + 0.36 atan(1.55 q1) is outside [0, 1]: at 3.6 it is
+// 1.0017 / -0.0017, beyond any rounding.
+#define ICE3_Q1_CLIP 3.6
 
 // srcs (optional): PSRCS of the point (ice_adjust.F90:360, :468).
 // OCND2: the separate liquid / ice cloud option of CONDENSATION
@@ -152,10 +172,10 @@ template <bool OCND2 = false>
 ICE3_HD void ia_point(const Cst &c, const IaDerived &d, double dt, double inv_dt, const IaIn &x, IaOut &o,
                       double *srcs = nullptr, const Ocnd2In *oi = nullptr, Ocnd2Out *oo = nullptr)
 {
-  const int nrr = (int)c.NRR;
+  const int nrr = d.nrr;
   double t = x.th * x.exn;
-  const double lv = c.LVTT + (c.CPV - c.CL) * (t - c.TT);
-  const double ls = c.LSTT + (c.CPV - c.CI) * (t - c.TT);
+  const double lv = c.LVTT + d.cpv_cl * (t - c.TT);
+  const double ls = c.LSTT + d.cpv_ci * (t - c.TT);
   double cph;
   if (nrr == 5) cph = c.CPD + c.CPV * x.rv + c.CL * (x.rc + x.rr) + c.CI * (x.ri + x.rs);
   else if (nrr == 4) cph = c.CPD + c.CPV * x.rv + c.CL * (x.rc + x.rr);
@@ -164,7 +184,7 @@ ICE3_HD void ia_point(const Cst &c, const IaDerived &d, double dt, double inv_dt
   const double inv_cph = fm::frcp(cph);
   double cldfr = 0.0, rv_out = 0.0, rc_out = 0.0, ri_out = 0.0;
   double hlc_hrc = 0.0, hlc_hcf = 0.0, hli_hri = 0.0, hli_hcf = 0.0;
-  if (c.LSUBG_COND != 0.0) {
+  if (d.subg) {
     // OCND2: ZPRIFACT = 0, the ice is kept out of the total water (condensation.F90:265-273)
     const double rt = OCND2 ? x.rv + x.rc : x.rv + x.rc + x.ri;
     const double it = fm::frcp(t);
@@ -175,7 +195,7 @@ ICE3_HD void ia_point(const Cst &c, const IaDerived &d, double dt, double inv_dt
       // the ice fraction: of the temperature (FRAC_ICE_ADJUST 0, the AROME
       // setting; fm::fdiv's product with the reciprocal formed once), else
       // of the condensate
-      const int fmode = (int)c.FRAC_ICE_ADJUST;
+      const int fmode = d.fmode;
       if (fmode == 0) {
         frac = nclip01(fm::mul_(c.TMAXMIX - t, d.imix));
       } else {
@@ -187,8 +207,8 @@ ICE3_HD void ia_point(const Cst &c, const IaDerived &d, double dt, double inv_dt
       // exactly where frac is 0 and qsl_i where it is 1 (the other term is
       // 0 times a finite value); a NaN fraction keeps both
       pv = piv = 0.0;
-      if (fm::bits_(frac) != fm::bits_(1.0)) pv = nmin(fm::fexp(c.ALPW - c.BETAW * it - c.GAMW * lt), 0.99 * x.pabs);
-      if (!zerod_(frac)) piv = nmin(fm::fexp(c.ALPI - c.BETAI * it - c.GAMI * lt), 0.99 * x.pabs);
+      if (fm::bits_(frac) != fm::bits_(1.0)) pv = cap_pressure(fm::fexp(c.ALPW - c.BETAW * it - c.GAMW * lt), x.pabs);
+      if (!zerod_(frac)) piv = cap_pressure(fm::fexp(c.ALPI - c.BETAI * it - c.GAMI * lt), x.pabs);
     } else {
       // condensation.F90:375-395: ICECLOUD, then the tabulated saturation
       // pressures; no ice fraction (:412, ZFRAC = 0)
@@ -202,15 +222,24 @@ ICE3_HD void ia_point(const Cst &c, const IaDerived &d, double dt, double inv_dt
     // (OCND2: frac = 0 and qsi feeds the ice cloud factor below)
     double qsl = (OCND2 || fm::bits_(frac) != fm::bits_(1.0)) ? fm::fdiv(d.rdrv * pv, x.pabs - pv) : 0.0;
     const double qsi = (OCND2 || !zerod_(frac)) ? fm::fdiv(d.rdrv * piv, x.pabs - piv) : 0.0;
-    qsl = (1.0 - frac) * qsl + frac * qsi;
-    const double lvs = (1.0 - frac) * lv + frac * ls;
+    // the weighted sums only where a lane of the warp has a fraction strictly
+    // between 0 and 1 (else one term, exactly)
+    const bool all_i = fm::bits_(frac) == fm::bits_(1.0);
+    const bool mixed = warp_any(!all_i && !zerod_(frac));
+    double lvs = all_i ? ls : lv;
+    if (mixed) {
+      qsl = (1.0 - frac) * qsl + frac * qsi;
+      lvs = (1.0 - frac) * lv + frac * ls;
+    } else if (all_i) {
+      qsl = qsi;
+    }
     const double ah = lvs * qsl * (it * it * d.irv) * (1.0 + qsl * d.rvrd);
     const double a = fm::frcp(1.0 + lvs * inv_cph * ah);
     const double sbar = a * (rt - qsl + ah * lvs * (OCND2 ? x.rc : x.rc + x.ri) * inv_cph);
     // sigma = sqrt(S) as S * S^(-1/2), the reciprocal reused for q1 when the
     // 1e-10 floor leaves sigma alone
     double sigma, isig = 0.0;
-    if (c.LSIGMAS != 0.0 && c.LSTATNW == 0.0 && !(fge(x.sigqsat, 0.0) && fge(0.0, x.sigqsat))) {
+    if (d.sig_full && !(fge(x.sigqsat, 0.0) && fge(0.0, x.sigqsat))) {
       const double s2 = sq(2.0 * x.sigs) + sq(x.sigqsat * qsl * a);
       if (fm::frsqrt_ok(s2)) {
         isig = fm::frsqrt(s2);
@@ -224,16 +253,25 @@ ICE3_HD void ia_point(const Cst &c, const IaDerived &d, double dt, double inv_dt
     const double sig = nmax(1e-10, sigma);
     const double q1 = (nz(isig) && fm::bits_(sig) == fm::bits_(sigma)) ? sbar * isig : fm::fdiv(sbar, sig);
     sigma = sig;
-    if (srcs) *srcs = sigrc_cb(c, q1);
-    double cond;
-    if (fgt(q1, 0.0)) cond = fge(2.0, q1) ? nmin(0.36787944117144233 + 0.66 * q1 + 0.086 * q1 * q1, 2.0) : q1;
-    else cond = fm::fexp(1.2 * q1 - 1.0);
-    cond *= sigma;
-    cldfr = fge(cond, 1e-12) ? nclip01(0.5 + 0.36 * fm::fatan(1.55 * q1)) : 0.0;
-    if (fge(cldfr, 0.0) && fge(0.0, cldfr)) cond = 0.0;
+    if (srcs) *srcs = sigrc_cb(d.lambda3, q1);
+    // where the clipped cloud fraction is 0 the condensate is 0 too: below
+    // -ICE3_Q1_CLIP neither the exponential nor the arc tangent is formed,
+    // above it the fraction is 1
+    double cond = 0.0;
+    if (!fge(-ICE3_Q1_CLIP, q1)) {
+      if (fgt(q1, 0.0)) cond = fge(2.0, q1) ? nmin(0.36787944117144233 + 0.66 * q1 + 0.086 * q1 * q1, 2.0) : q1;
+      else cond = fm::fexp(1.2 * q1 - 1.0);
+      cond *= sigma;
+      if (fge(cond, 1e-12)) cldfr = fge(q1, ICE3_Q1_CLIP) ? 1.0 : nclip01(0.5 + 0.36 * fm::fatan(1.55 * q1));
+      if (fge(cldfr, 0.0) && fge(0.0, cldfr)) cond = 0.0;
+    }
     if (!OCND2) {
-      rc_out = (1.0 - frac) * cond;
-      ri_out = frac * cond;
+      rc_out = all_i ? 0.0 : cond;
+      ri_out = all_i ? cond : 0.0;
+      if (mixed) {
+        rc_out = (1.0 - frac) * cond;
+        ri_out = frac * cond;
+      }
       t = t + ((rc_out - x.rc) * lv + (ri_out - x.ri) * ls) * inv_cph;
       rv_out = rt - rc_out - ri_out;
     } else {
@@ -269,10 +307,13 @@ ICE3_HD void ia_point(const Cst &c, const IaDerived &d, double dt, double inv_dt
   rvs = rvs - w2;
   ris = ris + w2;
   ths = ths + w2 * ls * inv_cphex;
-  if (c.LSUBG_COND == 0.0) {
+  if (!d.subg) {
     cldfr = fgt((rcs + ris) * dt, 1e-12) ? 1.0 : 0.0;
     if (srcs) *srcs = cldfr;
-  } else {
+  } else if (warp_any(nz(x.cf_mf) || nz(x.rc_mf) || nz(x.ri_mf) || !fge(rvs, 0.0) || !finite_(inv_cphex))) {
+    // the mass-flux clouds; a warp without any adds zeros (a negative vapour
+    // source with no mass flux gives 0 * inf = NaN in the limiter, as in the
+    // reference, so it goes through)
     double w1m = x.rc_mf * inv_dt, w2m = x.ri_mf * inv_dt;
     const double tot = w1m + w2m;
     const double scale = fgt(tot, rvs) ? fm::fdiv(rvs, tot) : 1.0;
@@ -283,7 +324,7 @@ ICE3_HD void ia_point(const Cst &c, const IaDerived &d, double dt, double inv_dt
     ris = ris + w2m;
     rvs = rvs - w1m - w2m;
     ths = ths + (w1m * lv + w2m * ls) * inv_cphex;
-    const int mfpdf = (int)c.SUBG_MF_PDF;
+    const int mfpdf = d.mfpdf;
     if (mfpdf == 0 || mfpdf == 1) {
       // the thresholds enter only as cf_mf * threshold: where cf_mf is +-0
       // that is +-0 whatever their (finite, positive) value, so they are
@@ -375,7 +416,7 @@ ICE3_HD void ia_point_vjp(const Cst &c, const IaDerived &d, double dt, double in
 {
   b = IaIn{};
   // ---- forward, keeping what the reverse pass needs ----
-  const int nrr = (int)c.NRR;
+  const int nrr = d.nrr;
   const double t0 = x.th * x.exn;
   const double lv = c.LVTT + (c.CPV - c.CL) * (t0 - c.TT);
   const double ls = c.LSTT + (c.CPV - c.CI) * (t0 - c.TT);
@@ -385,8 +426,8 @@ ICE3_HD void ia_point_vjp(const Cst &c, const IaDerived &d, double dt, double in
   else if (nrr == 2) cph = c.CPD + c.CPV * x.rv + c.CL * x.rc + c.CI * x.ri;
   else cph = c.CPD + c.CPV * x.rv + c.CL * (x.rc + x.rr) + c.CI * (x.ri + x.rs + x.rg);
   const double inv_cph = fm::frcp(cph);
-  const bool subg = c.LSUBG_COND != 0.0;
-  const int fmode = (int)c.FRAC_ICE_ADJUST;
+  const bool subg = d.subg;
+  const int fmode = d.fmode;
   double rt = 0, lt = 0, it = 0, ew = 0, ei = 0, pv = 0, piv = 0, frac = 0, qsl0 = 0, qsi = 0, qsl = 0, lvs = 0;
   double ah = 0, a = 0, G = 0, sigma0 = 0, sigma = 0, q1 = 0, cond0 = 0, cond = 0, cldfr0 = 0;
   double rc_out = 0, ri_out = 0, t = t0;
@@ -420,7 +461,7 @@ ICE3_HD void ia_point_vjp(const Cst &c, const IaDerived &d, double dt, double in
     a = fm::frcp(1.0 + lvs * inv_cph * ah);
     G = rt - qsl + ah * lvs * (x.rc + x.ri) * inv_cph;
     const double sbar = a * G;
-    if (c.LSIGMAS != 0.0 && c.LSTATNW == 0.0) {
+    if (d.sig_full) {
       sig_sqrt = !(fge(x.sigqsat, 0.0) && fge(0.0, x.sigqsat));
       sigma0 = sig_sqrt ? sqrt(sq(2.0 * x.sigs) + sq(x.sigqsat * qsl * a)) : 2.0 * x.sigs;
     } else {
@@ -480,7 +521,7 @@ ICE3_HD void ia_point_vjp(const Cst &c, const IaDerived &d, double dt, double in
     bool cld1_const;
     nmin_sel(1.0, cldfr0 + x.cf_mf, cld1_const);
     double b_w1m = 0.0, b_w2m = 0.0, b_cf = 0.0;
-    const int mfpdf = (int)c.SUBG_MF_PDF;
+    const int mfpdf = d.mfpdf;
     if (mfpdf == 0 || mfpdf == 1) {
       const double criaut = fm::fdiv(c.CRIAUTC, x.rho);
       const double p10 = fm::fexp10(c.ACRIAUTI * (t - c.TT) + c.BCRIAUTI);
