@@ -116,19 +116,24 @@ ICE3_HD bool warp_any(bool p)
 #endif
 }
 
-// num / den to within 2^-22 relative, from the FP32 reciprocal of den
-// (truncated to FP32) and one FP64 multiply; exact in sign.  0 where den is
-// outside FP32's normal range.  Used to skip an IEEE division whose result
-// cannot change a min / max.
-ICE3_HD double quot_est(double num, double den)
+// num / den in FP32, to within 2^-20 relative (both truncated to FP32, the
+// hardware's reciprocal); exact in sign.  0 where either is outside FP32's
+// normal range.  Used to skip an IEEE division whose result cannot change a
+// min / max, without an FP64 operation.
+ICE3_HD float quot_est(double num, double den)
 {
-  const int e = (int)((fm::bits_(den) >> 52) & 0x7ff);
-  if (e <= 898 || e >= 1149) return 0.0;
-  return num * fm::to_f64(fm::rcpf_(fm::to_f32(den)));
+  const uint32_t en = (fm::hi_(num) >> 20) & 0x7ffu, ed = (fm::hi_(den) >> 20) & 0x7ffu;
+  if (en - 899u >= 250u || ed - 899u >= 250u) return 0.0f;
+  return fm::mulf_(fm::to_f32(num), fm::rcp_seed_(fm::to_f32(den)));
 }
 // True only if the quotient that est estimates (quot_est) is above bound
-// for certain.
-ICE3_HD bool est_above(double est, double bound) { return gtd(est, bound + fabs(bound) * 0x1p-18); }
+// for certain: above the truncated bound by 2^-17.
+ICE3_HD bool est_above(float est, double bound)
+{
+  if (((fm::hi_(bound) >> 20) & 0x7ffu) >= 1149u) return false;
+  const float b = fm::to_f32(bound);
+  return est > fm::fmaf_(fabsf(b), 0x1p-17f, b);
+}
 ICE3_HD bool quot_above(double num, double den, double bound) { return est_above(quot_est(num, den), bound); }
 
 // x**a evaluated as exp(a*log(x)) with the FP64-lean exp/log of

@@ -91,7 +91,9 @@ struct Derived {
   // the option switches of the table as integers, so that no lane converts
   // or compares the FP64 table entries
   int aucv_rc, aucv_ri, prpdf, accr, evap, snow_riming;
-  int lwarm, lfeedbackt, lsnow_t, lcrflimit, llrfr;
+  int lwarm, lfeedbackt, lsnow_t, lcrflimit, llrfr, levlimit, lnullwetg, lwetgpost;
+  // FP32 copies for the estimate of the ice autoconversion threshold
+  float acriauti_f, bcriauti_f, tt_f;
   // differences of table constants, formed once per block (the same IEEE
   // values as formed in place)
   double cpv_cl, cpv_ci, ci_cl, tt_m35, tt_m5, tt_m2;
@@ -125,6 +127,12 @@ ICE3_HD void make_derived(const Cst &c, Derived &d)
   d.lsnow_t = c.LSNOW_T != 0.0;
   d.lcrflimit = c.LCRFLIMIT != 0.0;
   d.llrfr = d.accr == 1 || d.evap == 2;
+  d.levlimit = c.LEVLIMIT != 0.0;
+  d.lnullwetg = c.LNULLWETG != 0.0;
+  d.lwetgpost = c.LWETGPOST != 0.0;
+  d.acriauti_f = (float)c.ACRIAUTI;
+  d.bcriauti_f = (float)c.BCRIAUTI;
+  d.tt_f = (float)c.TT;
   d.cpv_cl = c.CPV - c.CL;
   d.cpv_ci = c.CPV - c.CI;
   d.ci_cl = c.CI - c.CL;
@@ -153,6 +161,7 @@ struct PointFix {
   double rho_mcexvt;    // rho**(-CEXVT)
   double rho_mcexvt1;   // rho**(-CEXVT-1)
   double rcrautc;       // CRIAUTC / rho
+  double rc_lo, rc_hi;  // rcrautc -+ sigma_rc
   double zx;            // TT / exn (IEEE division: where th stops at the T = TT limit)
 };
 
@@ -215,8 +224,8 @@ ICE3_HD bool zerod(double x) { return (opaque_bits(x) << 1) == 0; }
 // rates of the same pass reuse while T keeps its bit pattern (no HENI,
 // RRHONG or RIMLTC change in between): log T, 1/T, es_w and es_i.
 struct TTerms {
-  double t, lt, it, esw, esi;
-  bool set, esw_set;   // esw only where the nucleation needed it
+  double t, lt, it, esw, esi, rv, ssi;
+  bool set, esw_set, ssi_set;   // esw only where the nucleation needed it; ssi (of rv) where es_i is below p / 2
 };
 
 // ICE4_NUCLEATION (micro/ice4_nucleation.func.h:69-144, LOCND2 = .FALSE.);
@@ -231,6 +240,7 @@ ICE3_HD void nucleation(const Cst &c, const Derived &d, double tht, double pabst
   if (tt) { tt->t = t; tt->lt = lt; tt->it = it; tt->esi = zzw; tt->set = true; tt->esw_set = false; }
   zzw = dmin(pabst * 0.5, zzw);
   double zssi = fm::fdiv(rvt * (pabst - zzw), c.EPSILO * zzw) - 1.0;
+  if (tt) { tt->rv = rvt; tt->ssi = zssi; tt->ssi_set = fm::bits_(zzw) == fm::bits_(tt->esi); }
   // Not supersaturated over ice: the MIN with the water term below is not
   // positive either, no crystal nucleates, and with cit >= 0 the rest leaves
   // rvheni = 0 and cit as they are (zzw = MIN(-cit, 5e4) <= 0): es_w is not
@@ -259,7 +269,7 @@ ICE3_HD void nucleation(const Cst &c, const Derived &d, double tht, double pabst
     double w;
     if (opaque_bits(rvheni) == 0) w = 0.0;
     else if (gtp(rvheni, 1.e-20) && quot_above(num, lsfact, rvheni)) w = 1.0;
-    else w = dmin(rvheni, pmax0(num / lsfact)) / dmax(rvheni, 1.e-20);
+    else w = fm::fdiv_rn(dmin(rvheni, pmax0(fm::fdiv_rn(num, lsfact))), dmax(rvheni, 1.e-20));
     rvheni *= w;
     zzw *= w;
   }
@@ -269,8 +279,10 @@ ICE3_HD void nucleation(const Cst &c, const Derived &d, double tht, double pabst
 // ICE4_COMPUTE_PDF (micro/mode_ice4_compute_pdf.F90), one point; returns RF.
 // `criauti` receives MIN(CRIAUTI, 10**(ACRIAUTI (T-TT) + BCRIAUTI)), which
 // the ice autoconversion of the same pass uses too.
+// rc_lo, rc_hi: rcrautc -+ sigma_rc (read with SUBG_AUCV_RC = PDF, SUBG_PR_PDF = SIGM only).
 ICE3_HD double compute_pdf(const Cst &c, const Derived &d, double rcrautc, double rct, double rit, double cf,
-                           double t, double sigma_rc, double hl[4], double hi[4], double &criauti, bool soft = false)
+                           double t, double sigma_rc, double rc_lo, double rc_hi, double hl[4], double hi[4],
+                           double &criauti, bool soft = false)
 {
   const int aucv_rc = d.aucv_rc, aucv_ri = d.aucv_ri, prpdf = d.prpdf;
   double hcf = 0, lcf = 0, hrc = 0, lrc = 0;
@@ -285,9 +297,9 @@ ICE3_HD double compute_pdf(const Cst &c, const Derived &d, double rcrautc, doubl
     hcf = hl[0]; lcf = hl[1];
     if (gtp(sum, 1.e-20)) { lrc = hl[3] * rct / sum; hrc = hl[2] * rct / sum; }
   } else if (aucv_rc == 1 && prpdf == 0) {
-    if (gtd(rct, rcrautc + sigma_rc)) {
+    if (gtd(rct, rc_hi)) {
       hcf = 1.0; hrc = rct;
-    } else if (gtd(rct, rcrautc - sigma_rc)) {
+    } else if (gtd(rct, rc_lo)) {
       const double inv2s = fm::frcp(2.0 * sigma_rc);
       hcf = (rct + sigma_rc - rcrautc) * inv2s;
       lcf = pmax0(cf - hcf);
@@ -336,18 +348,18 @@ ICE3_HD double compute_pdf(const Cst &c, const Derived &d, double rcrautc, doubl
   bool ice_high = false;
   if (soft && aucv_ri == 0) {
     // a soft pass reads only rit > MIN(CRIAUTI, 10**x) = rit > CRIAUTI or
-    // rit > 10**x, decided from an FP32 estimate of 10**x (within 1e-5)
-    // unless rit is within 2^-14 of it
+    // rit > 10**x, decided from an FP32 estimate of 10**x (within 2^-16)
+    // unless rit is within 2^-12 of it
     ice_high = gtd(rit, c.CRIAUTI);
     const bool open = !ice_high && gtp(rit, c.I_RTMIN);
-    double x = 0.0, ea = 0.0;
+    bool near = false;
     if (warp_any(open)) {
-      x = c.ACRIAUTI * (t - c.TT) + c.BCRIAUTI;
-      ea = fm::to_f64(exp2f(fm::to_f32(x) * 3.32192809488736235f));
+      const float x = fm::fmaf_(d.acriauti_f, fm::to_f32(t) - d.tt_f, d.bcriauti_f);
+      const float ea = exp2f(x * 3.32192809488736235f), r = fm::to_f32(rit);
+      near = open && !(fabsf(r - ea) > ea * 0x1p-12f);
+      if (open && r > ea) ice_high = true;
     }
-    const bool near = open && !gtd(rit, ea + ea * 0x1p-14) && !ltd(rit, ea - ea * 0x1p-14);
-    if (open && gtd(rit, ea + ea * 0x1p-14)) ice_high = true;
-    if (warp_any(near) && near) ice_high = gtd(rit, fm::fexp10(x));
+    if (warp_any(near) && near) ice_high = gtd(rit, fm::fexp10(c.ACRIAUTI * (t - c.TT) + c.BCRIAUTI));
   } else if (warp_any(aucv_ri != 0 || gtp(rit, c.I_RTMIN))) {
     criauti = dmin(c.CRIAUTI, fm::fexp10(c.ACRIAUTI * (t - c.TT) + c.BCRIAUTI));
   }
@@ -523,7 +535,8 @@ ICE3_HD void hard_rates(const Cst &c, const Derived &d, const double *__restrict
   // without cloud only; it is not formed for the other points
   const bool need_esw = gtp(t, c.TT) || (gtp(v[IRR], c.R_RTMIN) && !gtp(v[IRC], c.C_RTMIN));
   double lt, it, esi_f, esw = 0.0;
-  if (tt && tt->set && fm::bits_(tt->t) == fm::bits_(t)) {
+  const bool same_t = tt && tt->set && fm::bits_(tt->t) == fm::bits_(t);
+  if (same_t) {
     lt = tt->lt; it = tt->it; esi_f = tt->esi;
     if (tt->esw_set) esw = tt->esw;
     else if (need_esw) esw = esat_from(c.ALPW, c.BETAW, c.GAMW, it, lt);
@@ -533,7 +546,8 @@ ICE3_HD void hard_rates(const Cst &c, const Derived &d, const double *__restrict
     if (need_esw) esw = esat_from(c.ALPW, c.BETAW, c.GAMW, it, lt);
   }
   const double esi = O ? tiwmx_at(op->tw + TW_ESI * kTiwmxN, t) : esi_f;
-  R.ssi = fm::fdiv(v[IRV] * (pf.pres - esi), c.EPSILO * esi) - 1.0;
+  if (!O && same_t && tt->ssi_set && fm::bits_(tt->rv) == fm::bits_(v[IRV])) R.ssi = tt->ssi;
+  else R.ssi = fm::fdiv(v[IRV] * (pf.pres - esi), c.EPSILO * esi) - 1.0;
   const bool has_v = gtp(v[IRV], c.V_RTMIN), has_c = gtp(v[IRC], c.C_RTMIN), has_r = gtp(v[IRR], c.R_RTMIN);
   const bool has_i = gtp(v[IRI], c.I_RTMIN), has_s = gtp(v[IRS], c.S_RTMIN), has_g = gtp(v[IRG], c.G_RTMIN);
   const bool has_h = H && gtp(v[IRH], c.H_RTMIN);
@@ -601,8 +615,8 @@ ICE3_HD void hard_rates(const Cst &c, const Derived &d, const double *__restrict
   double heat_i = 0.0, heat_w = 0.0;
   if (has_s || has_g || has_h) {
     const double ev = fm::fdiv(v[IRV] * pf.pres, c.EPSILO + v[IRV]);
-    const double ei = c.LEVLIMIT != 0.0 ? dmin(ev, esi_f) : ev;
-    const double ew = c.LEVLIMIT != 0.0 ? dmin(ev, esw) : ev;
+    const double ei = d.levlimit ? dmin(ev, esi_f) : ev;
+    const double ew = d.levlimit ? dmin(ev, esw) : ev;
     const double kt = ka * (c.TT - t);
     const double dl = dv * (c.LVTT + d.cpv_cl * (t - c.TT));
     const double irt = it * d.irv;
@@ -650,7 +664,7 @@ ICE3_HD void hard_rates(const Cst &c, const Derived &d, const double *__restrict
   // ---- ICE4_FAST_RS rates (mode_ice4_fast_rs.F90) ----
   // collision-freezing denominator, shared with ICE4_FAST_RG
   const double den = (has_s || has_g || has_h) ? fm::frcp(rho * (c.LMTT - c.CL * (c.TT - t))) : 0.0;
-  const double freez2 = (rho * (c.LMTT + d.ci_cl * (c.TT - t))) * den;
+  const double freez2 = (has_s || has_g || has_h) ? (rho * (c.LMTT + d.ci_cl * (c.TT - t))) * den : 0.0;
   rs[RS_FREEZ1] = has_s ? heat_i * vent_s * den : 0.0;
   rs[RS_FREEZ2] = has_s ? freez2 : 0.0;
   if (has_c && has_s) {
@@ -910,7 +924,7 @@ ICE3_HD void soft_rates(const Cst &c, const Derived &d, double t, const double *
 // O (OCND2): the part of the graupel deposition given to snow
 // (mode_ice4_tendencies.F90:445-458) and the RVDEPI / RILARS rows.
 template <bool H = false, bool O = false>
-ICE3_HD void aggregate(const Cst &c, double t, const double *v, double lvfact, double lsfact, Rates &R,
+ICE3_HD void aggregate(const Cst &c, const Derived &d, double t, const double *v, double lvfact, double lsfact, Rates &R,
                        double *A, bool soft = false, HailRates *hr = nullptr, double *B = nullptr,
                        const OcndRates *orr = nullptr, const double *ext = nullptr)
 {
@@ -952,9 +966,9 @@ ICE3_HD void aggregate(const Cst &c, double t, const double *v, double lvfact, d
     const double wet = pmax0(rwetg_init - rg[RG_RIWETG] - rg[RG_RSWETG]);
     const double dry = pmax0(rdryg_init - rg[RG_RIDRYG] - rg[RG_RSDRYG]);
     ldwetg = !gtd(wet, dry);
-    if (c.LNULLWETG != 0.0) ldwetg = ldwetg && pos(rdryg_init);
+    if (d.lnullwetg) ldwetg = ldwetg && pos(rdryg_init);
     else ldwetg = ldwetg && pos(rwetg_init);
-    if (c.LWETGPOST == 0.0) ldwetg = ldwetg && cold;
+    if (!d.lwetgpost) ldwetg = ldwetg && cold;
     lldryg = cold && gtp(rdryg_init, 1.e-20) && gtd(wet, dry);
   }
   if (ldwetg) {
@@ -1194,11 +1208,11 @@ ICE3_HD void hard_adjust(const Cst &c, const Derived &d, const PointFix &pf, dou
     r = v[IRR];
     if (d.lfeedbackt) {
       // the IEEE quotients only where the limit can bind: (TT - 35)/exn
-      // estimated within 2^-22 and taken 2^-20 low, so that the estimated
+      // estimated within 2^-20 and taken 2^-18 low, so that the estimated
       // quotient is below the true one
-      const double zq = quot_est(d.tt_m35, pf.exn);
-      if (!quot_above(zq - fabs(zq) * 0x1p-20 - v[ITH], lsv, r))
-        r = dmin(r, pmax0((d.tt_m35 / pf.exn - v[ITH]) / lsv));
+      const double zq = fm::to_f64(quot_est(d.tt_m35, pf.exn));
+      if (!quot_above(zq - fabs(zq) * 0x1p-18 - v[ITH], lsv, r))
+        r = dmin(r, pmax0(fm::fdiv_rn(fm::fdiv_rn(d.tt_m35, pf.exn) - v[ITH], lsv)));
     }
   }
   b[B_RRHONG_MR] = r;
@@ -1215,7 +1229,7 @@ ICE3_HD void hard_adjust(const Cst &c, const Derived &d, const PointFix &pf, dou
     if (d.lfeedbackt) {
       // the IEEE quotient only where it can be below r
       const double num = v[ITH] - pf.zx;
-      if (!quot_above(num, lsv, r)) r = dmin(r, pmax0(num / lsv));
+      if (!quot_above(num, lsv, r)) r = dmin(r, pmax0(fm::fdiv_rn(num, lsv)));
     }
   }
   b[B_RIMLTC_MR] = r;
@@ -1254,14 +1268,15 @@ ICE3_HD void tendencies(const Cst &c, const Derived &d, const double *__restrict
   for (int k = 0; k < NVT; ++k) { v[k] = vart[k]; B[k] = 0.0; }
   double *b = R.bu;
   TTerms tt;
-  tt.set = tt.esw_set = false;
+  tt.set = tt.esw_set = tt.ssi_set = false;
   if (!soft) {
     hard_adjust<O>(c, d, pf, lvfact, lsfact, cit, t, v, b, B, op, &tt);
   } else {
     b[B_RVHENI_MR] = b[B_RRHONG_MR] = b[B_RIMLTC_MR] = 0.0;
   }
   double criauti;
-  const double zrainfr = compute_pdf(c, d, pf.rcrautc, v[IRC], v[IRI], pf.cf, t, pf.sigma_rc, hl, hi, criauti, soft);
+  const double zrainfr = compute_pdf(c, d, pf.rcrautc, v[IRC], v[IRI], pf.cf, t, pf.sigma_rc, pf.rc_lo, pf.rc_hi, hl, hi,
+                                     criauti, soft);
   const bool llrfr = d.llrfr;
   if (llrfr) {
     rainfr = dmax(rainfr, zrainfr);
@@ -1276,11 +1291,13 @@ ICE3_HD void tendencies(const Cst &c, const Derived &d, const double *__restrict
                                 orr, &tt);
   else soft_rates<SUBG, H, O>(c, d, t, v, cit, hl, hi, R, pf.cf, rainfr, hr, orr);
   if (SUR && !soft && sur) slow_rates_from(c, t, v, hi, sur, R);
-  aggregate<H, O>(c, t, v, lvfact, lsfact, R, A, soft, hr, B, orr, ext);
+  aggregate<H, O>(c, d, t, v, lvfact, lsfact, R, A, soft, hr, B, orr, ext);
 }
 
 // ICE4_STEPPING for one micro point (mode_ice4_stepping.F90:139-518).
 // Returns the pass key (outer << 16 | inner-of-last-outer), 0 if capped.
+// t_0, ls_0, lv_0, zdev_0: temperature, latent heats and cph of the state at
+// t, which the caller has formed and the first pass starts from.
 // TS: the MRSTEP / TSTEP_TS time splitting (mode_ice4_stepping.F90:191-197,
 // :387-453): per outer iteration (IITER) the state and time at its start; a
 // pass ends early when the TSTEP_TS sub-step is used up or a mixing ratio has
@@ -1289,8 +1306,8 @@ template <bool SUR = false, bool SUBG = false, bool H = false, bool O = false, b
 ICE3_HD unsigned int stepping(const Cst &c, const Derived &d, const double *__restrict__ lut, const PointFix &pf,
                               double dt, int max_passes, double *vart, const double *ext, double &cit,
                               double &rainfr, double &rrevav, double hl[4], double hi[4], bool &capped,
-                              const double *sur = nullptr, const double *__restrict__ hlut = nullptr,
-                              const OcndPt *op = nullptr)
+                              double t_0, double ls_0, double lv_0, double zdev_0, const double *sur = nullptr,
+                              const double *__restrict__ hlut = nullptr, const OcndPt *op = nullptr)
 {
   OcndRates OR{0.0, 1.0, 1.0, 0.0, 0.0};
   int nb_iter_max = 0;
@@ -1343,12 +1360,17 @@ ICE3_HD unsigned int stepping(const Cst &c, const Derived &d, const double *__re
       if (passes >= max_passes) { capped = true; return 0u; }
       ++passes;
       ++inner;
-      double zsum2 = vart[IRI] + vart[IRS] + vart[IRG];
-      if (H) zsum2 += vart[IRH];
-      const double zdev = (c.CPD + c.CPV * vart[IRV] + c.CL * (vart[IRC] + vart[IRR]) + c.CI * zsum2) * pf.exn;
-      const double zzt = vart[ITH] * pf.exn;
-      double lsfact, lvfact;     // the IEEE quotients (fdiv_rn2: one reciprocal, checked)
-      fm::fdiv_rn2(c.LSTT + d.cpv_ci * (zzt - c.TT), c.LVTT + d.cpv_cl * (zzt - c.TT), zdev, lsfact, lvfact);
+      double zzt = t_0, ls_num = ls_0, lv_num = lv_0, zdev = zdev_0;
+      if (passes > 1) {
+        double zsum2 = vart[IRI] + vart[IRS] + vart[IRG];
+        if (H) zsum2 += vart[IRH];
+        zdev = c.CPD + c.CPV * vart[IRV] + c.CL * (vart[IRC] + vart[IRR]) + c.CI * zsum2;
+        zzt = vart[ITH] * pf.exn;
+        ls_num = c.LSTT + d.cpv_ci * (zzt - c.TT);
+        lv_num = c.LVTT + d.cpv_cl * (zzt - c.TT);
+      }
+      double lsfact, lvfact;     // the IEEE quotients
+      fm::fdiv_rn2(ls_num, lv_num, zdev * pf.exn, lsfact, lvfact);
       double A[NVT], B[NVT];
       tendencies<SUR, SUBG, H, O>(c, d, lut, soft, pf, lvfact, lsfact, cit, zzt, vart, R, rainfr, hl, hi, A, B, sur,
                                   &HR, hlut, op, &OR, ext);    // A includes the external tendencies
@@ -1357,12 +1379,18 @@ ICE3_HD unsigned int stepping(const Cst &c, const Derived &d, const double *__re
       // B (the instantaneous changes) is zero on soft passes: no theta jump
       // across TT/exn, no B in the depletion limits and the state update
       if (d.lfeedbackt) {
-        if (!soft && negd((vart[ITH] - zx) * (vart[ITH] + B[ITH] - zx))) maxtime = 0.;
+        // (th - zx) (th + B - zx) < 0: the two on different sides of zx
+        double num = zx;
+        if (!soft) {
+          const double tb = vart[ITH] + B[ITH];
+          if ((gtd(vart[ITH], zx) && ltd(tb, zx)) || (ltd(vart[ITH], zx) && gtd(tb, zx))) maxtime = 0.;
+          num = zx - B[ITH];
+        }
         if (abs_gtp(A[ITH], 1.e-20)) {
           // the IEEE quotient only where it can be positive and below maxtime
-          const double num = zx - B[ITH] - vart[ITH];
-          const double e = quot_est(num, A[ITH]);
-          if (!negd(e) && !est_above(e, maxtime)) {
+          num -= vart[ITH];
+          const float e = quot_est(num, A[ITH]);
+          if (!(e < 0.0f) && !est_above(e, maxtime)) {
             const double thr = fm::fdiv_rn(num, A[ITH]);
             if (pos(thr)) maxtime = dmin(maxtime, thr);
           }
@@ -1372,16 +1400,12 @@ ICE3_HD unsigned int stepping(const Cst &c, const Derived &d, const double *__re
       // MAX(MIN over all of them, MNH_TINY); a species' IEEE quotient is only
       // formed where it can be below the running minimum
       bool limited = false;
-      double mt_hi = maxtime + fabs(maxtime) * 0x1p-18;   // est_above's bound, updated with maxtime
 #pragma unroll
       for (int v = 1; v < NVT; ++v) {
         if (ltd(A[v], -1.e-20) && gtp(vart[v], rsmin[v])) {
           limited = true;
-          const double num = -(B[v] + vart[v]);
-          if (!gtd(quot_est(num, A[v]), mt_hi)) {
-            maxtime = dmin(maxtime, fm::fdiv_rn(num, A[v]));
-            mt_hi = maxtime + fabs(maxtime) * 0x1p-18;
-          }
+          const double num = soft ? -vart[v] : -(B[v] + vart[v]);
+          if (!est_above(quot_est(num, A[v]), maxtime)) maxtime = dmin(maxtime, fm::fdiv_rn(num, A[v]));
         }
       }
       if (limited) maxtime = dmax(maxtime, c.MNH_TINY);
@@ -1459,7 +1483,7 @@ ICE3_HD unsigned int rain_ice_point(const Cst &c, const Derived &d, const double
                                     const double *oconc = nullptr)
 {
   constexpr int NVT = H ? NVH : NV;
-  const double inv_dt = 1.0 / dt;
+  const double inv_dt = fm::frcp(dt);   // 1 / dt, correctly rounded
   const bool lwarm = d.lwarm;
   const bool sigm = d.aucv_rc == 1 && d.prpdf == 0;
   const bool adju = d.aucv_rc == 2 || d.aucv_ri == 2;
@@ -1518,6 +1542,8 @@ ICE3_HD unsigned int rain_ice_point(const Cst &c, const Derived &d, const double
     pf.rcrautc = c.CRIAUTC * irho;
     pf.cf = ldp(f.cldfr, p);
     pf.sigma_rc = sigm ? 2.0 * ldp(f.sigs, p) : 0.0;
+    pf.rc_lo = pf.rcrautc - pf.sigma_rc;
+    pf.rc_hi = pf.rcrautc + pf.sigma_rc;
     double vart[NVT], ext[NVT];
     vart[ITH] = th; vart[IRV] = rv; vart[IRC] = rc; vart[IRR] = rr; vart[IRI] = ri; vart[IRS] = rs; vart[IRG] = rg;
     ext[ITH] = ths - th * inv_dt; ext[IRV] = rvs - rv * inv_dt; ext[IRC] = rcs - rc * inv_dt;
@@ -1537,7 +1563,7 @@ ICE3_HD unsigned int rain_ice_point(const Cst &c, const Derived &d, const double
     }
     double rrevav;
     key = stepping<SUR, SUBG, H, O, TS>(c, d, lut, pf, dt, max_passes, vart, ext, cit, rainfr, rrevav, hl, hi,
-                                        capped, sur, hlut, &op);
+                                        capped, t, ls_num, lv_num, zdev, sur, hlut, &op);
 #pragma unroll
     for (int v = 0; v < NVT; ++v) vart[v] -= ext[v] * dt;
     evap = lwarm ? rrevav : 0.0;
@@ -1553,12 +1579,19 @@ ICE3_HD unsigned int rain_ice_point(const Cst &c, const Derived &d, const double
     const double wr = (vart[IRR] - rr0) * inv_dt, wi = (vart[IRI] - ri0) * inv_dt;
     const double ws = (vart[IRS] - rs0) * inv_dt, wg = (vart[IRG] - rg0) * inv_dt;
     const double wh = H ? (vart[NVT - 1] - ldp(f.rht, p)) * inv_dt : 0.0;
-    ths += (wc + wr) * lvx + (H ? wi + ws + wg + wh : wi + ws + wg) * lsx + zrvheni * lsx;
+    // (zrvheni = MIN(rvs, 0) here: 0 but for a negative vapour source)
+    double dth = (wc + wr) * lvx + (H ? wi + ws + wg + wh : wi + ws + wg) * lsx, dv = wv, di = wi;
+    if (warp_any(nz(zrvheni))) {
+      dth += zrvheni * lsx;
+      dv -= zrvheni;
+      di += zrvheni;
+    }
+    ths += dth;
     if (H) rhs += wh;
-    rvs += wv - zrvheni;
+    rvs += dv;
     rcs += wc;
     rrs += wr;
-    ris += wi + zrvheni;
+    ris += di;
     rss += ws;
     rgs += wg;
   } else {
@@ -1634,9 +1667,10 @@ ICE3_HD void prfr_column(const Cst &c, const Ice3gbRainIceFields &f, long nij, i
     double rf = 0.0;
     if (micro) {
       const double sig = sigm ? ldp(f.sigs, p) : 0.0;
-      const double rho = ldp(f.rhodref, p);
+      const double rcrautc = c.CRIAUTC / ldp(f.rhodref, p), sig2 = sig * sig;
       double criauti;
-      rf = compute_pdf(c, d, c.CRIAUTC / rho, rc, ri, cf, ldp(f.tht, p) * ldp(f.exn, p), sig * sig, hl, hi, criauti);
+      rf = compute_pdf(c, d, rcrautc, rc, ri, cf, ldp(f.tht, p) * ldp(f.exn, p), sig2, rcrautc - sig2, rcrautc + sig2,
+                       hl, hi, criauti);
     } else {
       if (aucv_rc != 2) hl[0] = 0.0;
       hl[2] = 0.0;

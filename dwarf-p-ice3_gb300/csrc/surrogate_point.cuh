@@ -42,6 +42,8 @@ ICE3_HD void point_fix(const Cst &c, const Ice3gbRainIceFields &f, long p, Point
   pf.rcrautc = c.CRIAUTC * irho;
   pf.cf = ldp(f.cldfr, p);
   pf.sigma_rc = sigm ? 2.0 * ldp(f.sigs, p) : 0.0;
+  pf.rc_lo = pf.rcrautc - pf.sigma_rc;
+  pf.rc_hi = pf.rcrautc + pf.sigma_rc;
 }
 
 // The 16 features of grid point p from its state at the start of the step,
