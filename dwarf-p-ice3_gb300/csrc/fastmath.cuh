@@ -47,6 +47,7 @@
 //          y0^2| < 2^-21, exact in integers), y0 (1 + eps/2 + 3 eps^2/8), the
 //          series of (1 - eps)^(-1/2) to its quadratic term (remainder below
 //          2^-64), rounded once: within 0.51 ulp, no FP64 operation.
+//          fsqrt_rn: sqrt(d), the IEEE result bit for bit, from it.
 //   fatan  reduction to [0, 1] by atan(x) = pi/2 - atan(1/x), then
 //          atan(y) = atan(c) + atan(r), c = j/64 the nearest table point,
 //          r = (y - c)/(1 + y c) (|r| <= 1/128; for y = 1/|x| numerator and
@@ -446,7 +447,8 @@ FM_NI void fdiv_rn2(double a1, double a2, double b, double &q1, double &q2)
   q2 = quot_(ch, cl, bh, bl, y, ec - eb + 1023u);
 }
 
-// The IEEE 1/sqrt(d), out of line (the rare fallback).
+// The IEEE square root and its reciprocal, out of line (the rare fallbacks).
+FM_NI double sqrt_ieee_(double d) { return sqrt(d); }
 FM_NI double rsqrt_ieee_(double d) { return 1.0 / sqrt(d); }
 
 // x = X 2^-52 in [1, 4) and d = x 4^k for a positive normal d.
@@ -490,6 +492,25 @@ FM_NI double frsqrt(double d)
   const uint64_t q = (rsqrt_fixed_(X, odd) + 256u) >> 9;          // [2^52, 2^53]
   const uint32_t k2 = (h >> 20) - odd;                            // 2 k + 1023
   return from_bits_((int64_t)(q + ((uint64_t)(1021u + 511u - (k2 >> 1)) << 52)));
+}
+
+// sqrt(d), the IEEE result bit for bit: X times 1/sqrt(x), rounded to 53
+// bits q, settled by the exact X - q^2 (nearest iff -q < X - q^2 <= q).
+FM_NI double fsqrt_rn(double d)
+{
+  if (!frsqrt_ok(d)) return sqrt_ieee_(d);
+  const uint32_t h = hi_(d);
+  uint64_t X;
+  uint32_t odd;
+  sqrt_split_(h, lo_(d), X, odd);
+  // sqrt(x) 2^62 in [2^62, 2^63): x 2^62 times Y, high half, doubled twice
+  const uint64_t r = mulhi64_(X << 10, rsqrt_fixed_(X, odd)) << 2;
+  uint64_t q = (r + 512u) >> 10;                                  // [2^52, 2^53]
+  const int64_t rem = (int64_t)((X << 52) - q * q);               // modulo 2^64
+  if (rem > (int64_t)q) ++q;
+  else if (rem <= -(int64_t)q) --q;
+  const uint32_t k2 = (h >> 20) - odd;
+  return from_bits_((int64_t)(q + ((uint64_t)((k2 >> 1) + 511u) << 52)));
 }
 
 // Arc tangent (see the header).

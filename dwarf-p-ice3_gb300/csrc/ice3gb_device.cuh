@@ -166,5 +166,11 @@ ICE3_HD double tiwmx_at(const double *tab, double t)
 }
 
 #if defined(__CUDACC__)
+// p mod nij, in 32 bits where p allows it (a 64-bit remainder is a call of
+// ~100 instructions).
+__device__ __forceinline__ long column_of(long p, int nij)
+{
+  return p <= 0xffffffffL ? (long)((unsigned)p % (unsigned)nij) : p % nij;
+}
 __device__ __forceinline__ double ld1(const double *p, long i) { return __ldg(p + i); }
 #endif

@@ -176,6 +176,7 @@ void tiwmx_tables(const Ice3gbConstants &c, double *tab);
 cudaError_t launch_ice_adjust(const Ice3gbConstants &c, const IaKernelFields &kf, int nij, int nk, double dt,
                               int num_sms, cudaStream_t s);
 cudaError_t launch_sedimentation(const Ice3gbConstants &c, const SedArgs &a, cudaStream_t s);
+cudaError_t launch_sedimentation_fluxes(const Ice3gbConstants &c, const SedArgs &a, cudaStream_t s);
 cudaError_t launch_fog_deposition(const Ice3gbConstants &c, const FogArgs &a, cudaStream_t s);
 cudaError_t launch_rain_ice_points(const Ice3gbConstants &c, const RainIceArgs &a, int num_sms, cudaStream_t s);
 cudaError_t launch_rain_ice_evap_fixup(const RainIceArgs &a, cudaStream_t s);

@@ -12,13 +12,6 @@
 namespace {
 using namespace ice3ia;
 
-// p mod nij, in 32 bits where p allows it (a 64-bit remainder is a call of
-// ~100 instructions).
-__device__ __forceinline__ long column_of(long p, int nij)
-{
-  return p <= 0xffffffffL ? (long)((unsigned)p % (unsigned)nij) : p % nij;
-}
-
 // One point per thread.  ADV: the state adjusted is adv_dt times the sources
 // (th = dt*ths, r = dt*rs, the state after the microphysics in the chained
 // physics step) instead of th/rv/.../rg, which are then not read; rrs/rss/rgs

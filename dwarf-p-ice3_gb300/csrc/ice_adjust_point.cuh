@@ -402,7 +402,7 @@ ICE3_HD void triangle_pdf_vjp(double w_dt, double crit, double cf_mf, double g_h
     b_crit += -b_u + (-6.0 * w_dt * crit + 3.0 * crit * crit) * b_P;
   }
   b_cf += hcf0 * g_hcf;
-  if (!w_const) b_w += -2.0 * inv_w2 / wmax * b_inv_w2;
+  if (!w_const) b_w += fm::fdiv(-2.0 * inv_w2, wmax) * b_inv_w2;
 }
 
 // Reverse-mode derivative of ia_point (hand-written): from the cotangents g
@@ -418,8 +418,8 @@ ICE3_HD void ia_point_vjp(const Cst &c, const IaDerived &d, double dt, double in
   // ---- forward, keeping what the reverse pass needs ----
   const int nrr = d.nrr;
   const double t0 = x.th * x.exn;
-  const double lv = c.LVTT + (c.CPV - c.CL) * (t0 - c.TT);
-  const double ls = c.LSTT + (c.CPV - c.CI) * (t0 - c.TT);
+  const double lv = c.LVTT + d.cpv_cl * (t0 - c.TT);
+  const double ls = c.LSTT + d.cpv_ci * (t0 - c.TT);
   double cph;
   if (nrr == 5) cph = c.CPD + c.CPV * x.rv + c.CL * (x.rc + x.rr) + c.CI * (x.ri + x.rs);
   else if (nrr == 4) cph = c.CPD + c.CPV * x.rv + c.CL * (x.rc + x.rr);
@@ -437,24 +437,30 @@ ICE3_HD void ia_point_vjp(const Cst &c, const IaDerived &d, double dt, double in
     rt = x.rv + x.rc + x.ri;
     lt = fm::flog(t0);
     it = fm::frcp(t0);
-    ew = fm::fexp(c.ALPW - c.BETAW * it - c.GAMW * lt);
-    ei = fm::fexp(c.ALPI - c.BETAI * it - c.GAMI * lt);
-    pv = nmin_sel(ew, 0.99 * x.pabs, pv_first);
-    piv = nmin_sel(ei, 0.99 * x.pabs, piv_first);
     frac_div = fgt(x.rc + x.ri, 1e-20);
     frac = frac_div ? fm::fdiv(x.rc, x.rc + x.ri) : 0.0;
     if (fmode == 3) {
       frac_pass = clip01_pass(frac);
       frac = nclip01(frac);
     } else if (fmode == 0) {
-      const double f0 = fm::fdiv(c.TMAXMIX - t0, c.TMAXMIX - c.TMINMIX);
+      const double f0 = fm::mul_(c.TMAXMIX - t0, d.imix);
       frac_pass = clip01_pass(f0);
       frac = nclip01(f0);
     } else {
       frac_pass = true;
     }
-    qsl0 = fm::fdiv(d.rdrv * pv, x.pabs - pv);
-    qsi = fm::fdiv(d.rdrv * piv, x.pabs - piv);
+    // the saturation over water / ice where it has a weight, or where the
+    // weight's own derivative reads it (FRAC_ICE_ADJUST 0 within its range)
+    if (fmode != 0 || frac_pass || fm::bits_(frac) != fm::bits_(1.0)) {
+      ew = fm::fexp(c.ALPW - c.BETAW * it - c.GAMW * lt);
+      pv = nmin_sel(ew, 0.99 * x.pabs, pv_first);
+      qsl0 = fm::fdiv(d.rdrv * pv, x.pabs - pv);
+    }
+    if (fmode != 0 || frac_pass || !zerod_(frac)) {
+      ei = fm::fexp(c.ALPI - c.BETAI * it - c.GAMI * lt);
+      piv = nmin_sel(ei, 0.99 * x.pabs, piv_first);
+      qsi = fm::fdiv(d.rdrv * piv, x.pabs - piv);
+    }
     qsl = (1.0 - frac) * qsl0 + frac * qsi;
     lvs = (1.0 - frac) * lv + frac * ls;
     ah = lvs * qsl * (it * it * d.irv) * (1.0 + qsl * d.rvrd);
@@ -463,7 +469,7 @@ ICE3_HD void ia_point_vjp(const Cst &c, const IaDerived &d, double dt, double in
     const double sbar = a * G;
     if (d.sig_full) {
       sig_sqrt = !(fge(x.sigqsat, 0.0) && fge(0.0, x.sigqsat));
-      sigma0 = sig_sqrt ? sqrt(sq(2.0 * x.sigs) + sq(x.sigqsat * qsl * a)) : 2.0 * x.sigs;
+      sigma0 = sig_sqrt ? fm::fsqrt_rn(sq(2.0 * x.sigs) + sq(x.sigqsat * qsl * a)) : 2.0 * x.sigs;
     } else {
       sigma0 = 2.0 * x.sigs;
     }
@@ -522,7 +528,9 @@ ICE3_HD void ia_point_vjp(const Cst &c, const IaDerived &d, double dt, double in
     nmin_sel(1.0, cldfr0 + x.cf_mf, cld1_const);
     double b_w1m = 0.0, b_w2m = 0.0, b_cf = 0.0;
     const int mfpdf = d.mfpdf;
-    if (mfpdf == 0 || mfpdf == 1) {
+    // (a warp without mass-flux clouds has zero contents on the flat part of
+    // the PDF: nothing flows back)
+    if ((mfpdf == 0 || mfpdf == 1) && warp_any(nz(x.cf_mf) || nz(w1m) || nz(w2m))) {
       const double criaut = fm::fdiv(c.CRIAUTC, x.rho);
       const double p10 = fm::fexp10(c.ACRIAUTI * (t - c.TT) + c.BCRIAUTI);
       bool ci_const;
@@ -557,7 +565,7 @@ ICE3_HD void ia_point_vjp(const Cst &c, const IaDerived &d, double dt, double in
         b_criaut_i += x.cf_mf * b_crit;
         b_cf += criaut_i * b_crit;
       }
-      b.rho += -criaut / x.rho * b_criaut;
+      b.rho += fm::fdiv(-criaut, x.rho) * b_criaut;
       if (!ci_const) b_t += c.ACRIAUTI * 2.302585092994045684 * p10 * b_criaut_i;
     }
     // ths = ths2 + (w1m lv + w2m ls) inv_cphex; rvs = rvs2 - w1m - w2m; ris = ris1 + w2m; rcs = rcs1 + w1m
@@ -575,10 +583,10 @@ ICE3_HD void ia_point_vjp(const Cst &c, const IaDerived &d, double dt, double in
     double b_w1m0 = scale * b_w1m, b_w2m0 = scale * b_w2m;
     const double b_scale = w1m0 * b_w1m + w2m0 * b_w2m;
     if (sc_div) {
-      const double b_tot = -scale / tot * b_scale;
+      const double b_tot = fm::fdiv(-scale, tot) * b_scale;
       b_w1m0 += b_tot;
       b_w2m0 += b_tot;
-      b_rvs += b_scale / tot;
+      b_rvs += fm::fdiv(b_scale, tot);
     }
     b.rc_mf += inv_dt * b_w1m0;
     b.ri_mf += inv_dt * b_w2m0;
@@ -611,8 +619,10 @@ ICE3_HD void ia_point_vjp(const Cst &c, const IaDerived &d, double dt, double in
   b_ri_out += inv_dt * b_w2r;
   b.ri -= inv_dt * b_w2r;
   // inv_cphex = inv_cph / exn_ref
-  b_inv_cph += b_inv_cphex / x.exn_ref;
-  b.exn_ref += -inv_cphex / x.exn_ref * b_inv_cphex;
+  double bq, iq;
+  fm::fdiv_rn2(b_inv_cphex, -inv_cphex, x.exn_ref, bq, iq);
+  b_inv_cph += bq;
+  b.exn_ref += iq * b_inv_cphex;
   double b_t0 = 0.0;
   if (subg) {
     // rv_out = rt - rc_out - ri_out
@@ -637,7 +647,7 @@ ICE3_HD void ia_point_vjp(const Cst &c, const IaDerived &d, double dt, double in
     double b_q1 = 0.0;
     if (cld_on && cld_pass) {
       const double z = 1.55 * q1;
-      b_q1 += 0.36 * 1.55 / (1.0 + z * z) * b_cldfr0;
+      b_q1 += fm::fdiv(0.36 * 1.55, 1.0 + z * z) * b_cldfr0;
     }
     // cond1 = cond0 sigma
     const double b_cond0 = sigma * b_cond1;
@@ -646,13 +656,16 @@ ICE3_HD void ia_point_vjp(const Cst &c, const IaDerived &d, double dt, double in
     else if (cond_poly) { if (poly_pass) b_q1 += (0.66 + 0.172 * q1) * b_cond0; }
     else b_q1 += b_cond0;
     // q1 = sbar / sigma
-    const double b_sbar = b_q1 / sigma;
-    b_sigma += -q1 / sigma * b_q1;
+    double b_sbar, qs;
+    fm::fdiv_rn2(b_q1, -q1, sigma, b_sbar, qs);
+    b_sigma += qs * b_q1;
     const double b_sigma0 = sig_const ? 0.0 : b_sigma;
     double b_qsl = 0.0, b_a = 0.0;
     if (sig_sqrt) {
       const double u = 2.0 * x.sigs, v = x.sigqsat * qsl * a;
-      const double b_u = u / sigma0 * b_sigma0, b_v = v / sigma0 * b_sigma0;
+      double us, vs;
+      fm::fdiv_rn2(u, v, sigma0, us, vs);
+      const double b_u = us * b_sigma0, b_v = vs * b_sigma0;
       b.sigs += 2.0 * b_u;
       b.sigqsat += qsl * a * b_v;
       b_qsl += x.sigqsat * a * b_v;
@@ -690,21 +703,32 @@ ICE3_HD void ia_point_vjp(const Cst &c, const IaDerived &d, double dt, double in
     b_frac += (qsi - qsl0) * b_qsl;
     // qsi = rdrv piv / (pabs - piv), qsl0 = rdrv pv / (pabs - pv)
     const double di = x.pabs - piv, dw = x.pabs - pv;
-    const double b_piv = d.rdrv * x.pabs / (di * di) * b_qsi;
-    const double b_pv = d.rdrv * x.pabs / (dw * dw) * b_qsl0;
-    b.pabs += -d.rdrv * piv / (di * di) * b_qsi - d.rdrv * pv / (dw * dw) * b_qsl0;
+    double b_piv = 0.0, b_pv = 0.0;
+    if (nz(piv)) {
+      double ki, kip;
+      fm::fdiv_rn2(d.rdrv * x.pabs, -d.rdrv * piv, di * di, ki, kip);
+      b_piv = ki * b_qsi;
+      b.pabs += kip * b_qsi;
+    }
+    if (nz(pv)) {
+      double kw, kwp;
+      fm::fdiv_rn2(d.rdrv * x.pabs, d.rdrv * pv, dw * dw, kw, kwp);
+      b_pv = kw * b_qsl0;
+      b.pabs -= kwp * b_qsl0;
+    }
     // frac
     if (fmode == 0) {
-      if (frac_pass) b_t0 += -b_frac / (c.TMAXMIX - c.TMINMIX);
+      if (frac_pass) b_t0 += fm::mul_(-b_frac, d.imix);
     } else if (frac_div && frac_pass) {
       const double s2 = rcri * rcri;
-      b.rc += x.ri / s2 * b_frac;
-      b.ri += -x.rc / s2 * b_frac;
+      b.rc += fm::fdiv(x.ri, s2) * b_frac;
+      b.ri += fm::fdiv(-x.rc, s2) * b_frac;
     }
-    // pv = min(ew, 0.99 pabs), piv = min(ei, 0.99 pabs)
+    // pv = min(ew, 0.99 pabs), piv = min(ei, 0.99 pabs) (b_pv, b_piv are 0
+    // where the pressure was not formed)
     double b_ew = 0.0, b_ei = 0.0;
-    if (pv_first) b_ew = b_pv; else b.pabs += 0.99 * b_pv;
-    if (piv_first) b_ei = b_piv; else b.pabs += 0.99 * b_piv;
+    if (pv_first) b_ew = b_pv; else if (warp_any(nz(b_pv))) b.pabs += 0.99 * b_pv;
+    if (piv_first) b_ei = b_piv; else if (warp_any(nz(b_piv))) b.pabs += 0.99 * b_piv;
     // ew = exp(ALPW - BETAW it - GAMW lt), ei likewise
     b_it += -c.BETAW * ew * b_ew - c.BETAI * ei * b_ei;
     const double b_lt = -c.GAMW * ew * b_ew - c.GAMI * ei * b_ei;
@@ -729,7 +753,7 @@ ICE3_HD void ia_point_vjp(const Cst &c, const IaDerived &d, double dt, double in
     b.ri += c.CI * b_cph; b.rs += c.CI * b_cph; b.rg += c.CI * b_cph;
   }
   // lv, ls, t0 = th exn
-  b_t0 += (c.CPV - c.CL) * b_lv + (c.CPV - c.CI) * b_ls;
+  b_t0 += d.cpv_cl * b_lv + d.cpv_ci * b_ls;
   b.th += x.exn * b_t0;
   b.exn += x.th * b_t0;
 }

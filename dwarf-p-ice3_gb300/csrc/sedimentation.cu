@@ -49,6 +49,9 @@ __device__ __forceinline__ SpeciesPar species_par(const Cst &c, int s)
           ex - c.CEXVT - 1.0};
 }
 
+// FLUX_ONLY: the fluxes alone (the adjoint's recomputed forward sweep); the
+// sources and the surface precipitation are not written.
+template <bool FLUX_ONLY>
 __global__ void __launch_bounds__(32 * 6) sedimentation_kernel(const __grid_constant__ Cst c,
                                                                const __grid_constant__ SedArgs a)
 {
@@ -134,7 +137,7 @@ __global__ void __launch_bounds__(32 * 6) sedimentation_kernel(const __grid_cons
       if (!zerod_(w2)) flux += pmax0(1.0 - l[LV_DZ_IDT][lane] * fm::frcp(w2)) * fabove;
       if (valid) {
         const double idiv = l[LV_IDIV][lane];
-        src[p] = a.fortran ? sr + idiv * (fabove - flux) : sr + fm::fdiv(fabove - flux, idiv);
+        if (!FLUX_ONLY) src[p] = a.fortran ? sr + idiv * (fabove - flux) : sr + fm::fdiv(fabove - flux, idiv);
         if (fpr) fpr[p] = flux;
       }
       fabove = flux;
@@ -143,7 +146,7 @@ __global__ void __launch_bounds__(32 * 6) sedimentation_kernel(const __grid_cons
   if (!valid) return;
   if (!moves && fpr)
     for (int k = 0; k < a.nk; ++k) fpr[(long)k * nij + col] = 0.0;
-  if (inpr) inpr[col] = moves ? fabove / c.RHOLW : 0.0;
+  if (!FLUX_ONLY && inpr) inpr[col] = moves ? fabove / c.RHOLW : 0.0;
 }
 
 // SEDIM = SPLI: one column per thread (sed_split_column).
@@ -198,7 +201,13 @@ __global__ void fog_deposition_kernel(const __grid_constant__ Cst c, FogArgs a)
 cudaError_t launch_sedimentation(const Cst &c, const SedArgs &a, cudaStream_t s)
 {
   const int warps = a.hsrc ? 6 : 5;
-  sedimentation_kernel<<<(unsigned)(((long)a.nij + 31) / 32), 32 * warps, 0, s>>>(c, a);
+  sedimentation_kernel<false><<<(unsigned)(((long)a.nij + 31) / 32), 32 * warps, 0, s>>>(c, a);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_sedimentation_fluxes(const Cst &c, const SedArgs &a, cudaStream_t s)
+{
+  sedimentation_kernel<true><<<(unsigned)(((long)a.nij + 31) / 32), 32 * 5, 0, s>>>(c, a);
   return cudaGetLastError();
 }
 

@@ -104,7 +104,7 @@ ICE3_HD double fall_speed_d(const Cst &c, int s, double r, double lrho, double w
       first = gtd(0.05e6, arg);
       const double dmax_ = first ? 0.05e6 : arg;
       const double v = c.FSEDI * fm::fexp(-c.CEXVT * lrho + c.EXCSEDI * fm::flog(dmax_));
-      const double dld = first ? 0.0 : -0.021454e6 / dmax_;
+      const double dld = first ? 0.0 : fm::fdiv(-0.021454e6, dmax_);
       d_lr = v * c.EXCSEDI * dld;
       d_lrho = v * (-c.CEXVT + c.EXCSEDI * dld);
       return v;
@@ -243,51 +243,109 @@ struct SedGradients {
   double *rhodref, *dzz, *pabs, *tht;
 };
 
+// What the species share at a level of the reverse sweep, and the cotangents
+// of it that a species adds to.
+struct SedLevel {
+  double rho, dz, rhodz, tso, lrho, wlbda;   // tso = dt / (rho dz); wlbda: cloud only
+};
+struct SedLevelCot {
+  double rho, dz, rhodz, tso, lrho, wlbda;
+};
+
+// One species at one level of the reverse sweep: the source and the fluxes
+// entering (fa) and leaving (fk) the level, the cotangents gS of the updated
+// source and bF of fk.  Returns the cotangent of fa; b_src receives that of
+// the source and b the level's.  Derivatives of the branch the forward took at
+// the kinks (the min of the two flux bounds, the max(0, .) of the transfer
+// factor, the thresholds rt, qp > XRTMIN).
+ICE3_HD double sed_vjp_species(const Cst &c, int s, bool fortran, const CloudPar &cp, double dt, double inv_dt,
+                               const SedLevel &l, double src, double rtmin, double fa, double fk, double gS, double bF,
+                               double &b_src, SedLevelCot &b)
+{
+  const double rt = src * dt, qp = fa * l.tso;
+  const bool c1 = gtp(rt, rtmin), c2 = gtp(qp, rtmin);
+  double d1_lr = 0.0, d1_lrho = 0.0, d1_wl = 0.0, d2_lr = 0.0, d2_lrho = 0.0, d2_wl = 0.0;
+  const double w1 = c1 ? fall_speed_d(c, s, rt, l.lrho, l.wlbda, cp, d1_lr, d1_lrho, d1_wl) : 0.0;
+  const double w2 = c2 ? fall_speed_d(c, s, qp, l.lrho, l.wlbda, cp, d2_lr, d2_lrho, d2_wl) : 0.0;
+  const double a1 = l.rhodz * rt * inv_dt, a2 = w1 * l.rho * rt;
+  const bool sel1 = !gtd(a1, a2);
+  double Bv = 0.0, u = 0.0, idw = 0.0;               // idw = 1 / (dt w2)
+  const bool nz2 = !zerod_(w2);
+  if (nz2) {
+    idw = fm::frcp(dt * w2);
+    u = 1.0 - l.dz * idw;
+    Bv = pmax0(u);
+  }
+  // source update
+  double b_fa, bFt;
+  if (fortran) {
+    const double coef = l.tso * inv_dt;
+    b_fa = coef * gS;
+    bFt = bF - coef * gS;
+    b.tso += (fa - fk) * inv_dt * gS;
+  } else {
+    const double iden = fm::frcp(l.rhodz * dt);
+    b_fa = gS * iden;
+    bFt = bF - gS * iden;
+    b.rhodz += -(fa - fk) * dt * (iden * iden) * gS;
+  }
+  // F_k = min(a1, a2) + Bv F_{k+1}
+  b_fa += Bv * bFt;
+  double b_rt = 0.0;
+  if (sel1) {
+    b_rt = l.rhodz * inv_dt * bFt;
+    b.rhodz += rt * inv_dt * bFt;
+  } else {
+    const double b_w1 = l.rho * rt * bFt;
+    b.rho += w1 * rt * bFt;
+    b_rt = w1 * l.rho * bFt;
+    if (c1) {
+      b_rt += fm::fdiv(d1_lr, rt) * b_w1;
+      b.lrho += d1_lrho * b_w1;
+      b.wlbda += d1_wl * b_w1;
+    }
+  }
+  if (nz2 && pos(u)) {
+    const double b_B = fa * bFt, g2 = idw * b_B;
+    const double b_w2 = fm::fdiv(l.dz * g2, w2);      // dz / (dt w2^2) b_B
+    b.dz -= g2;
+    if (c2) {
+      const double b_qp = fm::fdiv(d2_lr, qp) * b_w2;
+      b.lrho += d2_lrho * b_w2;
+      b.wlbda += d2_wl * b_w2;
+      b_fa += l.tso * b_qp;
+      b.tso += fa * b_qp;
+    }
+  }
+  b_src = gS + dt * b_rt;
+  return b_fa;
+}
+
 // Reverse sweep of one column (hand-written adjoint of sed_column_forward):
 // bottom-up, carrying the cotangent of the flux entering each level from
 // above.  `flux` holds the forward fluxes F_k of the column (io.fpr layout),
-// recomputed by sed_column_forward just before.  Derivatives of the branch
-// the forward took at the kinks (the min of the two flux bounds, the
-// max(0, .) of the transfer factor, the thresholds rt, qp > XRTMIN).
+// recomputed by sed_column_forward just before.
 ICE3_HD void sed_column_vjp(const Cst &c, bool fortran, bool skip_c, const CloudPar &cp, double dt,
                             const SedColumnIO &io, double *const flux[5], const SedCotangents &g,
                             const SedGradients &gx, long col)
 {
   const double inv_dt = 1.0 / dt;
   double rtmin[5];
-#pragma unroll
   for (int s = 0; s < 5; ++s) rtmin[s] = sed_rtmin(c, s);
   // cotangent of F_k (flux leaving level k downward), starting at the surface
   double bF[5];
-#pragma unroll
   for (int s = 0; s < 5; ++s) bF[s] = (g.inpr[s] && !(s == 0 && skip_c)) ? g.inpr[s][col] / c.RHOLW : 0.0;
   for (int k = 0; k < io.nk; ++k) {
     const long p = (long)k * io.nij + col;
-    const long pa = p + io.nij;                    // level above
-    const double rho = sed_load(io.rhodref, p), dz = sed_load(io.dzz, p);
-    const double rhodz = rho * dz;
-    const double tsorhodz = fm::fdiv(dt, rhodz);
-    double src[5], rt[5], qp[5], fa[5], fk[5];
-    bool c1[5], c2[5];
-    bool any = false;
-#pragma unroll
-    for (int s = 0; s < 5; ++s) {
-      if (s == 0 && skip_c) { c1[s] = c2[s] = false; src[s] = rt[s] = qp[s] = fa[s] = fk[s] = 0.0; continue; }
-      src[s] = io.src_in[s][p];
-      rt[s] = src[s] * dt;
-      fa[s] = (k + 1 < io.nk) ? flux[s][pa] : 0.0;
-      fk[s] = flux[s][p];
-      qp[s] = fa[s] * tsorhodz;
-      c1[s] = gtp(rt[s], rtmin[s]);
-      c2[s] = gtp(qp[s], rtmin[s]);
-      any = any || c1[s] || c2[s];
-    }
-    const double lrho = any ? fm::flog(rho) : 0.0;
-    const bool cloud = c1[0] || c2[0];
-    const double pabs = cloud ? sed_load(io.pabs, p) : 1.0, tht = cloud ? sed_load(io.tht, p) : 0.0;
-    const double wlbda = cloud ? 6.6e-8 * fm::fdiv(101325.0, pabs) * (tht * (1.0 / 293.15)) : 0.0;
-    double b_rho = 0.0, b_dz = 0.0, b_rhodz = 0.0, b_tso = 0.0, b_lrho = 0.0, b_wl = 0.0;
-#pragma unroll
+    SedLevel l;
+    l.rho = sed_load(io.rhodref, p);
+    l.dz = sed_load(io.dzz, p);
+    l.rhodz = l.rho * l.dz;
+    l.tso = fm::fdiv(dt, l.rhodz);
+    l.lrho = fm::flog(l.rho);
+    const double pabs = sed_load(io.pabs, p), tht = sed_load(io.tht, p);
+    l.wlbda = 6.6e-8 * fm::fdiv(101325.0, pabs) * (tht * (1.0 / 293.15));
+    SedLevelCot b = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
     for (int s = 0; s < 5; ++s) {
       const double gS = g.src[s] ? g.src[s][p] : 0.0;
       if (s == 0 && skip_c) {                       // sources passed through unchanged
@@ -295,70 +353,18 @@ ICE3_HD void sed_column_vjp(const Cst &c, bool fortran, bool skip_c, const Cloud
         continue;
       }
       if (g.fpr[s]) bF[s] += g.fpr[s][p];
-      double d1_lr = 0.0, d1_lrho = 0.0, d1_wl = 0.0, d2_lr = 0.0, d2_lrho = 0.0, d2_wl = 0.0;
-      const double w1 = c1[s] ? fall_speed_d(c, s, rt[s], lrho, wlbda, cp, d1_lr, d1_lrho, d1_wl) : 0.0;
-      const double w2 = c2[s] ? fall_speed_d(c, s, qp[s], lrho, wlbda, cp, d2_lr, d2_lrho, d2_wl) : 0.0;
-      const double a1 = rhodz * rt[s] * inv_dt, a2 = w1 * rho * rt[s];
-      const bool sel1 = !gtd(a1, a2);
-      double Bv = 0.0, u = 0.0;
-      const bool nz2 = !zerod_(w2);
-      if (nz2) {
-        u = 1.0 - fm::fdiv(dz, dt * w2);
-        Bv = pmax0(u);
-      }
-      // source update
-      double b_src = gS, b_fa = 0.0, bFt;
-      if (fortran) {
-        const double coef = tsorhodz * inv_dt;
-        b_fa += coef * gS;
-        bFt = bF[s] - coef * gS;
-        b_tso += (fa[s] - fk[s]) * inv_dt * gS;
-      } else {
-        const double den = rhodz * dt;
-        b_fa += gS / den;
-        bFt = bF[s] - gS / den;
-        b_rhodz += -(fa[s] - fk[s]) * dt / (den * den) * gS;
-      }
-      // F_k = min(a1, a2) + Bv F_{k+1}
-      b_fa += Bv * bFt;
-      const double b_B = fa[s] * bFt;
-      double b_rt = 0.0;
-      if (sel1) {
-        b_rt += rhodz * inv_dt * bFt;
-        b_rhodz += rt[s] * inv_dt * bFt;
-      } else {
-        const double b_w1 = rho * rt[s] * bFt;
-        b_rho += w1 * rt[s] * bFt;
-        b_rt += w1 * rho * bFt;
-        if (c1[s]) {
-          b_rt += d1_lr / rt[s] * b_w1;
-          b_lrho += d1_lrho * b_w1;
-          b_wl += d1_wl * b_w1;
-        }
-      }
-      if (nz2 && pos(u)) {
-        const double b_w2 = dz / (dt * w2 * w2) * b_B;
-        b_dz += -1.0 / (dt * w2) * b_B;
-        if (c2[s]) {
-          const double b_qp = d2_lr / qp[s] * b_w2;
-          b_lrho += d2_lrho * b_w2;
-          b_wl += d2_wl * b_w2;
-          b_fa += tsorhodz * b_qp;
-          b_tso += fa[s] * b_qp;
-        }
-      }
-      b_src += dt * b_rt;
+      const double fa = (k + 1 < io.nk) ? flux[s][p + io.nij] : 0.0;
+      double b_src;
+      bF[s] = sed_vjp_species(c, s, fortran, cp, dt, inv_dt, l, io.src_in[s][p], rtmin[s], fa, flux[s][p], gS, bF[s],
+                              b_src, b);
       if (gx.src[s]) gx.src[s][p] = b_src;
-      bF[s] = b_fa;                                 // cotangent of F_{k+1}, used at level k + 1
     }
     // level quantities shared by the species
-    b_rhodz += -tsorhodz / rhodz * b_tso;
-    b_rho += dz * b_rhodz + (any ? b_lrho / rho : 0.0);
-    b_dz += rho * b_rhodz;
-    if (gx.rhodref) gx.rhodref[p] = b_rho;
-    if (gx.dzz) gx.dzz[p] = b_dz;
-    if (gx.pabs) gx.pabs[p] = cloud ? -wlbda / pabs * b_wl : 0.0;
-    if (gx.tht) gx.tht[p] = cloud ? wlbda / tht * b_wl : 0.0;
+    b.rhodz += -fm::fdiv(l.tso, l.rhodz) * b.tso;
+    if (gx.rhodref) gx.rhodref[p] = b.rho + l.dz * b.rhodz + fm::fdiv(b.lrho, l.rho);
+    if (gx.dzz) gx.dzz[p] = b.dz + l.rho * b.rhodz;
+    if (gx.pabs) gx.pabs[p] = -fm::fdiv(l.wlbda, pabs) * b.wlbda;
+    if (gx.tht) gx.tht[p] = fm::fdiv(l.wlbda, tht) * b.wlbda;
   }
 }
 
