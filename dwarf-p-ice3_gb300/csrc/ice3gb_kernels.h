@@ -142,6 +142,9 @@ struct TcGemmArgs {
   long ldz;
   __nv_bfloat16 *H;         // EPI_BIAS_GELU, EPI_DGELU
   long ldh;
+  __nv_bfloat16 *HT;        // H transposed [N][ldht] (optional), ldht >= M rounded up to 128
+  long ldht;
+  int padded;               // A and B rows hold zeros from K to the next multiple of 8
   int *err;
 };
 cudaError_t launch_tc_gemm(const TcGemmArgs &a, cudaStream_t s);
@@ -160,11 +163,14 @@ cudaError_t launch_mlp_pack(const float *p, long w1, long w2, long w3, long w4, 
                             cudaStream_t s);
 cudaError_t launch_mlp_fused(const MlpFusedArgs &a, int num_sms, cudaStream_t s);
 cudaError_t launch_sum_splits(const float *part, float *out, long n, int splits, cudaStream_t s);
-cudaError_t launch_col_sum(const float *x, float *out, int rows, int cols, long ld, cudaStream_t s);
-cudaError_t launch_surrogate_loss(const float *y, const float *tgt, int rows, int nrates, __nv_bfloat16 *dy, float *dyf,
-                                  float *loss, cudaStream_t s);
-cudaError_t launch_adam(float *w, const float *g, float *m1, float *m2, __nv_bfloat16 *w16, long n, float lr, float b1,
-                        float b2, float eps, int step, cudaStream_t s);
+constexpr int COL_SUM_BLOCKS = 64;   // row ranges of a column sum: part holds that many rows of partials
+cudaError_t launch_col_sum(const float *x, float *part, float *out, int rows, int cols, long ld, cudaStream_t s);
+cudaError_t launch_surrogate_loss(const float *y, const float *tgt, int rows, int nrates, __nv_bfloat16 *dy,
+                                  __nv_bfloat16 *dyt, long ldt, float *dyf, float *loss, cudaStream_t s);
+cudaError_t launch_adam(float *w, const float *g, float *m1, float *m2, __nv_bfloat16 *w16, __nv_bfloat16 *w16t, int din,
+                        long ldt, long n, float lr, float b1, float b2, float eps, int step, cudaStream_t s);
+cudaError_t launch_to_bf16_t(const float *x, __nv_bfloat16 *y, __nv_bfloat16 *yt, long rows, int cols, long pad_rows,
+                             long ldt, cudaStream_t s);
 cudaError_t launch_to_bf16(const float *x, __nv_bfloat16 *y, long n, cudaStream_t s);
 
 // OCND2 TIWMX tables (micro/mode_ini_tiwmx.F90), filled on the host: six

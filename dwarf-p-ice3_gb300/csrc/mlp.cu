@@ -2,19 +2,27 @@
 // per-point MLP of the slow-process surrogate built on it (forward,
 // hand-written backward, Adam).
 //
-// tc_gemm_kernel: one CTA (4 warps) computes a 128 x N tile (N <= 256) of
+// tc_gemm_kernel: one CTA (8 warps) computes a 128 x N tile (N <= 256) of
 //   C[m][n] = sum_k A(m, k) B(n, k),  A(m, k) = A[m*sam + k*sak],  B(n, k) = B[n*sbn + k*sbk]
-// in FP32 in TMEM.  K is walked in chunks of 64: the CTA stages the A and B
-// chunks into shared memory in the K-major core-matrix layout (16-byte
-// vector loads when K is the contiguous index, element loads otherwise,
-// which also transposes), one thread issues the K/16 tcgen05.mma and commits
-// to an mbarrier, and all threads wait (bounded) before the next chunk.
-// Rows >= M and k >= K are staged as zeros.  The epilogue reads the tile
-// back with tcgen05.ld (warp w: rows 32w..32w+31) and applies:
+// in FP32 in TMEM.  K is walked in chunks of 64 through a ring of G_NST
+// shared-memory stages in the K-major core-matrix layout, filled with 16-byte
+// asynchronous copies where K is the contiguous index (element loads
+// otherwise, which also transpose); one thread issues the K/16 tcgen05.mma of
+// a chunk and commits them to the stage's mbarrier, and a stage is refilled
+// once its MMAs are done (bounded waits).  Rows >= M and k >= K are staged as
+// zeros.  The epilogue reads the tile back with tcgen05.ld (warp w: rows
+// 32 (w % 4) .. + 31, every second group of 16 columns) and applies:
 //   EPI_STORE     C -> f32 (split-K partials at C + split * M * ldc)
 //   EPI_BIAS_GELU Z = C + bias -> f32 Zout (optional), H = GELU(Z) -> bf16
 //   EPI_BIAS      Y = C + bias -> f32
 //   EPI_DGELU     dZ = C * GELU'(Zin) -> bf16 H and f32 C
+// H also goes to HT, transposed ([n][m], zeros up to the tile's last row),
+// where the caller wants it: the weight gradients contract over m, and with
+// HT their operands have m contiguous too.
+// Bound: at the training batch (16,384 rows) the latency of filling the ring
+// and the epilogue's stores; four warps, one stage and element-wise transposing
+// took 122 us per hidden layer forward, 299 us backward and 776 us per weight
+// gradient.
 // On a barrier timeout the kernel sets *err, stops issuing and frees its
 // TMEM after a second bounded wait.
 #include <cuda_bf16.h>
@@ -52,12 +60,53 @@ __device__ __forceinline__ float dgelu(float z)
   return 0.5f * (1.0f + th) + 0.5f * z * (1.0f - th * th) * du;
 }
 
-__global__ void __launch_bounds__(128) tc_gemm_kernel(const TcGemmArgs a)
+constexpr int G_THREADS = 256, G_NST = 4;
+constexpr int G_A = 128 * KC, G_STAGE = (128 + 256) * KC;         // elements of a stage (A, then B)
+
+// 16 bytes global -> shared, or zeros
+__device__ __forceinline__ void copy16(__nv_bfloat16 *dst, const __nv_bfloat16 *src, bool in)
+{
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(tc::smem_u32(dst)), "l"(src), "r"(in ? 16 : 0)
+               : "memory");
+}
+
+// Rows r0 .. r0 + nrows - 1 (those below `rows`) and k0 .. k0 + KC - 1 (below
+// K) of an operand with strides sr, sk into a stage's tile.
+__device__ __forceinline__ void stage_tile(__nv_bfloat16 *tile, const __nv_bfloat16 *x, long sr, long sk, long r0, int nrows,
+                                           long rows, int k0, int K, bool vec, int tid)
+{
+  if (vec) {
+    for (int i = tid; i < nrows * (KC / 8); i += G_THREADS) {
+      const int r = i / (KC / 8), q = i % (KC / 8), k = k0 + 8 * q;
+      const bool in = r0 + r < rows && k < K;
+      copy16(tile + tc::core_off(r, 8 * q, KC), in ? x + (r0 + r) * sr + k : x, in);
+    }
+  } else {
+    for (int i = tid; i < nrows * KC; i += G_THREADS) {
+      int r, kk;
+      if (sr == 1) { r = i % nrows; kk = i / nrows; } else { r = i / KC; kk = i % KC; }
+      __nv_bfloat16 v = __float2bfloat16(0.0f);
+      if (r0 + r < rows && k0 + kk < K) v = x[(r0 + r) * sr + (long)(k0 + kk) * sk];
+      tile[tc::core_off(r, kk, KC)] = v;
+    }
+  }
+}
+
+__device__ __forceinline__ uint32_t bf16x2_bits(float a, float b)
+{
+  const __nv_bfloat162 v = __floats2bfloat162_rn(a, b);
+  return *reinterpret_cast<const uint32_t *>(&v);
+}
+__device__ __forceinline__ bool aligned_rows(const void *p, long ld, int elem)
+{
+  return (((uintptr_t)p | (uintptr_t)(ld * elem)) & 15) == 0;
+}
+
+__global__ void __launch_bounds__(G_THREADS) tc_gemm_kernel(const TcGemmArgs a)
 {
   extern __shared__ __align__(1024) unsigned char smem_raw[];
-  __nv_bfloat16 *sA = reinterpret_cast<__nv_bfloat16 *>(smem_raw);               // 128 x KC
-  __nv_bfloat16 *sB = sA + 128 * KC;                                            // 256 x KC
-  __shared__ __align__(8) uint64_t mbar;
+  __nv_bfloat16 *const ring = reinterpret_cast<__nv_bfloat16 *>(smem_raw);
+  __shared__ __align__(8) uint64_t mbar[G_NST];
   __shared__ uint32_t tmem_base;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int np = (a.N + 15) & ~15;
@@ -68,116 +117,136 @@ __global__ void __launch_bounds__(128) tc_gemm_kernel(const TcGemmArgs a)
   const int ksplit = ((kpad / 16 + a.k_split - 1) / a.k_split) * 16;
   const int kbeg = blockIdx.y * ksplit;
   const int kend = min(kpad, kbeg + ksplit);
-  if (tid == 0) tc::mbar_init(&mbar, 1);
+  const int nch = kend > kbeg ? (kend - kbeg + KC - 1) / KC : 0;
+  if (tid == 0) {
+    for (int i = 0; i < G_NST; ++i) tc::mbar_init(&mbar[i], 1);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
   if (warp == 0) tc::tmem_alloc(&tmem_base, ncols);
   tc::fence_before();
   __syncthreads();
   tc::fence_after();
   const uint32_t tmem = tmem_base;
   const uint32_t idesc = tc::idesc_bf16_f32(128, np);
-  const bool a_vec = a.sak == 1 && (a.sam % 8) == 0 && (((uintptr_t)a.A) & 15) == 0;
-  const bool b_vec = a.sbk == 1 && (a.sbn % 8) == 0 && (((uintptr_t)a.B) & 15) == 0;
-  bool ok = true, issued = false;
-  uint32_t phase = 0;
-  for (int k0 = kbeg; k0 < kend && ok; k0 += KC) {
-    const int kc = min(KC, kend - k0);
-    // ---- stage A (128 x kc) and B (np x kc)
-    if (a_vec && (a.K % 8) == 0) {
-      for (int i = tid; i < 128 * (kc >> 3); i += 128) {
-        const int r = i / (kc >> 3), q = i % (kc >> 3);
-        const long m = m0 + r;
-        const int k = k0 + 8 * q;
-        uint4 v = make_uint4(0, 0, 0, 0);
-        if (m < a.M && k < a.K) v = __ldg(reinterpret_cast<const uint4 *>(a.A + m * a.sam + k));
-        *reinterpret_cast<uint4 *>(sA + tc::core_off(r, 8 * q, kc)) = v;
-      }
-    } else {
-      for (int i = tid; i < 128 * kc; i += 128) {
-        int r, kk;
-        if (a.sam == 1) { r = i % 128; kk = i / 128; } else { r = i / kc; kk = i % kc; }
-        const long m = m0 + r;
-        const int k = k0 + kk;
-        __nv_bfloat16 v = __float2bfloat16(0.0f);
-        if (m < a.M && k < a.K) v = a.A[m * a.sam + (long)k * a.sak];
-        sA[tc::core_off(r, kk, kc)] = v;
-      }
-    }
-    if (b_vec && (a.K % 8) == 0) {
-      for (int i = tid; i < np * (kc >> 3); i += 128) {
-        const int r = i / (kc >> 3), q = i % (kc >> 3);
-        const int k = k0 + 8 * q;
-        uint4 v = make_uint4(0, 0, 0, 0);
-        if (r < a.N && k < a.K) v = __ldg(reinterpret_cast<const uint4 *>(a.B + (long)r * a.sbn + k));
-        *reinterpret_cast<uint4 *>(sB + tc::core_off(r, 8 * q, kc)) = v;
-      }
-    } else {
-      for (int i = tid; i < np * kc; i += 128) {
-        int r, kk;
-        if (a.sbn == 1) { r = i % np; kk = i / np; } else { r = i / kc; kk = i % kc; }
-        const int k = k0 + kk;
-        __nv_bfloat16 v = __float2bfloat16(0.0f);
-        if (r < a.N && k < a.K) v = a.B[(long)r * a.sbn + (long)k * a.sbk];
-        sB[tc::core_off(r, kk, kc)] = v;
-      }
-    }
+  // (a padded operand holds zeros from K to the next multiple of 8)
+  const bool k8 = a.padded || (a.K % 8) == 0;
+  const bool a_vec = k8 && a.sak == 1 && aligned_rows(a.A, a.sam, 2);
+  const bool b_vec = k8 && a.sbk == 1 && aligned_rows(a.B, a.sbn, 2);
+  auto fill = [&](int ch) {
+    __nv_bfloat16 *sA = ring + (ch % G_NST) * G_STAGE;
+    // (nothing past this split's range is read: its chunk count ends there)
+    const int k0 = kbeg + ch * KC, K = min(a.K, kend);
+    stage_tile(sA, a.A, a.sam, a.sak, m0, 128, a.M, k0, K, a_vec, tid);
+    stage_tile(sA + G_A, a.B, a.sbn, a.sbk, 0, np, a.N, k0, K, b_vec, tid);
+  };
+  for (int ch = 0; ch < G_NST - 1; ++ch) {
+    if (ch < nch) fill(ch);
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  }
+  bool ok = true;
+  int issued = 0;
+  for (int ch = 0; ch < nch; ++ch) {
+    asm volatile("cp.async.wait_group %0;" ::"n"(G_NST - 2) : "memory");   // this thread's copies of chunk ch
     tc::fence_async_smem();
-    __syncthreads();
-    // ---- MMAs of the chunk
+    ok = __syncthreads_and(ok) != 0;                   // block-uniform
+    if (!ok) break;
     if (tid == 0) {
       tc::fence_after();
-      const uint32_t sbo = (uint32_t)(kc >> 3) * 128u;
-      for (int ks = 0; ks < kc / 16; ++ks) {
-        const uint64_t da = tc::desc(tc::smem_u32(sA) + ks * 256, 128u, sbo);
-        const uint64_t db = tc::desc(tc::smem_u32(sB) + ks * 256, 128u, sbo);
-        tc::mma_bf16(tmem, da, db, idesc, issued || ks > 0);
-      }
-      issued = true;
-      tc::commit(&mbar);
+      const uint32_t sA = tc::smem_u32(ring + (ch % G_NST) * G_STAGE), sB = sA + G_A * 2;
+      const int steps = min(KC, kend - kbeg - ch * KC) / 16;
+      for (int ks = 0; ks < steps; ++ks)
+        tc::mma_bf16(tmem, tc::desc(sA + ks * 256, 128u, (KC / 8) * 128u), tc::desc(sB + ks * 256, 128u, (KC / 8) * 128u),
+                     idesc, ch > 0 || ks > 0);
+      tc::commit(&mbar[ch % G_NST]);
     }
-    issued = true;
-    // block-uniform: every warp must take the same path into tcgen05.ld
-    ok = __syncthreads_and(tc::mbar_wait(&mbar, phase, WAIT_ITERS) ? 1 : 0) != 0;
-    phase ^= 1u;
-    tc::fence_after();
+    issued = ch + 1;
+    // refill the stage of chunk ch - 1 once its MMAs are done
+    if (ch + G_NST - 1 < nch) {
+      if (ch > 0) ok = tc::mbar_wait(&mbar[(ch - 1) % G_NST], (uint32_t)(((ch - 1) / G_NST) & 1), WAIT_ITERS);
+      if (ok) fill(ch + G_NST - 1);
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
   }
+  // every MMA of the tile is done when the last commit is
+  if (ok && issued > 0)
+    ok = tc::mbar_wait(&mbar[(issued - 1) % G_NST], (uint32_t)(((issued - 1) / G_NST) & 1), WAIT_ITERS);
+  ok = __syncthreads_and(ok) != 0;
+  tc::fence_after();
   if (!ok) {
     if (tid == 0) atomicExch(a.err, 1);
-    tc::mbar_wait(&mbar, phase ^ 1u, WAIT_ITERS);     // let MMAs in flight finish before freeing TMEM
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    // let MMAs in flight finish before freeing TMEM
+    if (issued > 0) tc::mbar_wait(&mbar[(issued - 1) % G_NST], (uint32_t)(((issued - 1) / G_NST) & 1), WAIT_ITERS);
   }
   // ---- epilogue
   if (ok) {
-    const long m = m0 + warp * 32 + lane;
-    for (int c0 = 0; c0 < np; c0 += 16) {
+    const int row = (warp & 3) * 32 + lane;
+    const long m = m0 + row;
+    const bool in = m < a.M;
+    const bool c4 = aligned_rows(a.C, a.ldc, 4), z4 = aligned_rows(a.Zout ? a.Zout : a.Zin, a.ldz, 4);
+    const bool h8 = aligned_rows(a.H, a.ldh, 2);
+    for (int c0 = 16 * (warp >> 2); c0 < np; c0 += 32) {
       float v[16];
-      if (issued) tc::tmem_ld16(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)c0, v);
+      if (issued) tc::tmem_ld16(tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)c0, v);
       else
         for (int j = 0; j < 16; ++j) v[j] = 0.0f;
-      if (m >= a.M) continue;
+      const bool full = c0 + 16 <= a.N;
+      float h[16];                                     // what H takes
+      if (a.epi == EPI_DGELU) {
+        float z[16];
+        if (in && full && z4) {
 #pragma unroll
-      for (int j = 0; j < 16; ++j) {
-        const int n = c0 + j;
-        if (n >= a.N) continue;
-        float x = v[j];
-        switch (a.epi) {
-          case EPI_STORE:
-            a.C[(long)blockIdx.y * a.M * a.ldc + m * a.ldc + n] = x;
-            break;
-          case EPI_BIAS_GELU: {
-            const float z = x + a.bias[n];
-            if (a.Zout) a.Zout[m * a.ldz + n] = z;
-            a.H[m * a.ldh + n] = __float2bfloat16(gelu(z));
-            break;
+          for (int q = 0; q < 4; ++q) {
+            const float4 t = __ldg(reinterpret_cast<const float4 *>(a.Zin + m * a.ldz + c0) + q);
+            z[4 * q] = t.x; z[4 * q + 1] = t.y; z[4 * q + 2] = t.z; z[4 * q + 3] = t.w;
           }
-          case EPI_BIAS:
-            a.C[m * a.ldc + n] = x + a.bias[n];
-            break;
-          default: {  // EPI_DGELU
-            const float dz = x * dgelu(a.Zin[m * a.ldz + n]);
-            a.H[m * a.ldh + n] = __float2bfloat16(dz);
-            if (a.C) a.C[m * a.ldc + n] = dz;
-            break;
-          }
+        } else {
+#pragma unroll
+          for (int j = 0; j < 16; ++j) z[j] = (in && c0 + j < a.N) ? a.Zin[m * a.ldz + c0 + j] : 0.0f;
         }
+#pragma unroll
+        for (int j = 0; j < 16; ++j) h[j] = v[j] *= dgelu(z[j]);
+      } else if (a.epi != EPI_STORE) {
+#pragma unroll
+        for (int j = 0; j < 16; ++j) {
+          if (c0 + j < a.N) v[j] += a.bias[c0 + j];
+          h[j] = a.epi == EPI_BIAS_GELU ? gelu(v[j]) : 0.0f;
+        }
+      }
+      // FP32 result: Z of the forward, C of the others
+      float *const o = a.epi == EPI_BIAS_GELU ? a.Zout : a.C;
+      if (o && in) {
+        float *const d = a.epi == EPI_BIAS_GELU ? o + m * a.ldz + c0
+                                                : o + (a.epi == EPI_STORE ? (long)blockIdx.y * a.M * a.ldc : 0L) + m * a.ldc + c0;
+        if (full && (a.epi == EPI_BIAS_GELU ? z4 : (c4 && (a.epi != EPI_STORE || ((a.M * a.ldc) & 3) == 0)))) {
+#pragma unroll
+          for (int q = 0; q < 4; ++q)
+            reinterpret_cast<float4 *>(d)[q] = make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
+        } else {
+#pragma unroll
+          for (int j = 0; j < 16; ++j)
+            if (c0 + j < a.N) d[j] = v[j];
+        }
+      }
+      if (a.epi != EPI_BIAS_GELU && a.epi != EPI_DGELU) continue;
+      if (in) {
+        __nv_bfloat16 *const d = a.H + m * a.ldh + c0;
+        if (full && h8) {
+#pragma unroll
+          for (int q = 0; q < 2; ++q)
+            reinterpret_cast<uint4 *>(d)[q] =
+                make_uint4(bf16x2_bits(h[8 * q], h[8 * q + 1]), bf16x2_bits(h[8 * q + 2], h[8 * q + 3]),
+                           bf16x2_bits(h[8 * q + 4], h[8 * q + 5]), bf16x2_bits(h[8 * q + 6], h[8 * q + 7]));
+        } else {
+#pragma unroll
+          for (int j = 0; j < 16; ++j)
+            if (c0 + j < a.N) d[j] = __float2bfloat16(h[j]);
+        }
+      }
+      if (a.HT) {
+#pragma unroll
+        for (int j = 0; j < 16; ++j)
+          if (c0 + j < a.N) a.HT[(long)(c0 + j) * a.ldht + m] = __float2bfloat16(in ? h[j] : 0.0f);
       }
     }
   }
@@ -206,12 +275,6 @@ constexpr int FZ_OFF_H = 0, FZ_OFF_STAGE = 65536, FZ_OFF_W1 = FZ_OFF_STAGE + FZ_
 constexpr int FZ_OFF_W4 = FZ_OFF_W1 + 8192, FZ_OFF_X = FZ_OFF_W4 + 8192, FZ_OFF_B = FZ_OFF_X + 4096;
 constexpr int FZ_SMEM = FZ_OFF_B + (3 * 256 + 16) * 4;
 
-__device__ __forceinline__ uint32_t pack_bf16x2(float a, float b)
-{
-  const __nv_bfloat162 v = __floats2bfloat162_rn(a, b);
-  return *reinterpret_cast<const uint32_t *>(&v);
-}
-
 // Bias + GELU of 32 accumulator columns (from cb0) of one row into the
 // activation tile.  In an epilogue half h, warp w holds TMEM lanes
 // 32 (w % 4) .. + 31 (its rows) and the columns 128 h + 32 (w / 4) .. + 31;
@@ -230,7 +293,7 @@ __device__ __forceinline__ void fz_gelu_half(const uint32_t r[32], const float *
     uint32_t w[4];
 #pragma unroll
     for (int j = 0; j < 4; ++j)
-      w[j] = pack_bf16x2(gelu(__uint_as_float(r[8 * g + 2 * j]) + bb[2 * j]),
+      w[j] = bf16x2_bits(gelu(__uint_as_float(r[8 * g + 2 * j]) + bb[2 * j]),
                          gelu(__uint_as_float(r[8 * g + 2 * j + 1]) + bb[2 * j + 1]));
     *reinterpret_cast<uint4 *>(sH + tc::core_off(row, cb, 256)) = make_uint4(w[0], w[1], w[2], w[3]);
   }
@@ -364,10 +427,10 @@ __global__ void __launch_bounds__(FZ_THREADS, 1) mlp_fused_kernel(const MlpFused
         for (int q = 0; q < 16; ++q) x[q] = 0.0f;
       }
       *reinterpret_cast<uint4 *>(sX + tc::core_off(tid, 0, 16)) =
-          make_uint4(pack_bf16x2(x[0], x[1]), pack_bf16x2(x[2], x[3]), pack_bf16x2(x[4], x[5]), pack_bf16x2(x[6], x[7]));
+          make_uint4(bf16x2_bits(x[0], x[1]), bf16x2_bits(x[2], x[3]), bf16x2_bits(x[4], x[5]), bf16x2_bits(x[6], x[7]));
       *reinterpret_cast<uint4 *>(sX + tc::core_off(tid, 8, 16)) =
-          make_uint4(pack_bf16x2(x[8], x[9]), pack_bf16x2(x[10], x[11]), pack_bf16x2(x[12], x[13]),
-                     pack_bf16x2(x[14], x[15]));
+          make_uint4(bf16x2_bits(x[8], x[9]), bf16x2_bits(x[10], x[11]), bf16x2_bits(x[12], x[13]),
+                     bf16x2_bits(x[14], x[15]));
     }
     sync_async();
     // ---- layer 1: K = 16, one MMA into A
@@ -484,28 +547,44 @@ __global__ void sum_splits_kernel(const float *__restrict__ part, float *__restr
 {
   for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x) {
     float s = 0.0f;
+#pragma unroll 8
     for (int j = 0; j < splits; ++j) s += part[(long)j * n + i];
     out[i] = s;
   }
 }
 
-// Column sums (bias gradients): out[n] = sum_m x[m * ld + n], fixed order.
-__global__ void col_sum_kernel(const float *__restrict__ x, float *__restrict__ out, int rows, int cols, long ld)
+// Column sums (bias gradients) of a range of rows per block, in a fixed order:
+// part[b][n] = sum of x[m * ld + n] over the block's rows, eight rows side by
+// side for 32 columns; sum_splits_kernel adds the blocks.  (A thread per
+// column over all rows took 0.93 ms for 16,384 x 256.)
+__global__ void __launch_bounds__(256) col_sum_kernel(const float *__restrict__ x, float *__restrict__ part, int rows,
+                                                      int cols, long ld, int rows_per)
 {
-  const int n = blockIdx.x * blockDim.x + threadIdx.x;
-  if (n >= cols) return;
+  __shared__ float red[8][32];
+  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5, n = blockIdx.x * 32 + tx;
+  const int r1 = min(rows, (int)(blockIdx.y + 1) * rows_per);
   float s = 0.0f;
-  for (int m = 0; m < rows; ++m) s += x[(long)m * ld + n];
-  out[n] = s;
+  if (n < cols) {
+#pragma unroll 4
+    for (int m = blockIdx.y * rows_per + ty; m < r1; m += 8) s += x[(long)m * ld + n];
+  }
+  red[ty][tx] = s;
+  __syncthreads();
+  if (ty == 0 && n < cols) {
+#pragma unroll
+    for (int j = 1; j < 8; ++j) s += red[j][tx];
+    part[(long)blockIdx.y * cols + n] = s;
+  }
 }
 
 // Loss of the surrogate head: per rate r, y[2r] is the logit of "the rate is
 // nonzero" (binary cross-entropy against act), y[2r+1] the transformed rate
 // (squared error against val where the rate is nonzero).  Writes dY
-// ([rows][16], mean over the batch) in bf16 for the GEMMs and in f32 for the
-// output-bias gradient, and accumulates the loss.
+// ([rows][16], mean over the batch) in bf16 for the GEMMs (also transposed,
+// [16][ldt]) and in f32 for the output-bias gradient, and accumulates the loss.
 __global__ void surrogate_loss_kernel(const float *__restrict__ y, const float *__restrict__ tgt, int rows, int nrates,
-                                      __nv_bfloat16 *__restrict__ dy, float *__restrict__ dyf, float *__restrict__ loss)
+                                      __nv_bfloat16 *__restrict__ dy, __nv_bfloat16 *__restrict__ dyt, long ldt,
+                                      float *__restrict__ dyf, float *__restrict__ loss)
 {
   __shared__ float red[128];
   const int m = blockIdx.x * blockDim.x + threadIdx.x;
@@ -529,6 +608,9 @@ __global__ void surrogate_loss_kernel(const float *__restrict__ y, const float *
       dy[(long)m * 16 + j] = __float2bfloat16(0.0f);
       dyf[(long)m * 16 + j] = 0.0f;
     }
+    for (int j = 0; j < 16; ++j) dyt[j * ldt + m] = dy[(long)m * 16 + j];
+  } else {
+    for (int j = 0; j < 16; ++j) dyt[j * ldt + m] = __float2bfloat16(0.0f);   // zeros to the block's last row
   }
   red[threadIdx.x] = l;
   __syncthreads();
@@ -539,10 +621,11 @@ __global__ void surrogate_loss_kernel(const float *__restrict__ y, const float *
   if (threadIdx.x == 0) atomicAdd(loss, red[0] / (float)rows);
 }
 
-// Adam on FP32 master weights; refreshes the BF16 copy used by the GEMMs.
+// Adam on FP32 master weights; refreshes the BF16 copies used by the GEMMs
+// (w16 [out][din], w16t [din][ldt]).
 __global__ void adam_kernel(float *__restrict__ w, const float *__restrict__ g, float *__restrict__ m1,
-                            float *__restrict__ m2, __nv_bfloat16 *__restrict__ w16, long n, float lr, float b1,
-                            float b2, float eps, float c1, float c2)
+                            float *__restrict__ m2, __nv_bfloat16 *__restrict__ w16, __nv_bfloat16 *__restrict__ w16t,
+                            int din, long ldt, long n, float lr, float b1, float b2, float eps, float c1, float c2)
 {
   for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x) {
     const float gi = g[i];
@@ -552,6 +635,7 @@ __global__ void adam_kernel(float *__restrict__ w, const float *__restrict__ g, 
     const float wi = w[i] - lr * (a * c1) / (sqrtf(b * c2) + eps);
     w[i] = wi;
     if (w16) w16[i] = __float2bfloat16(wi);
+    if (w16t) w16t[(i % din) * ldt + i / din] = __float2bfloat16(wi);
   }
 }
 
@@ -561,12 +645,25 @@ __global__ void to_bf16_kernel(const float *__restrict__ x, __nv_bfloat16 *__res
     y[i] = __float2bfloat16(x[i]);
 }
 
+// x [rows][cols] (f32) -> y (BF16, [rows][cols], or NULL) and yt (BF16,
+// [cols][ldt]), the transpose with zeros for rows .. pad_rows - 1.
+__global__ void to_bf16_t_kernel(const float *__restrict__ x, __nv_bfloat16 *__restrict__ y, __nv_bfloat16 *__restrict__ yt,
+                                 long rows, int cols, long pad_rows, long ldt)
+{
+  for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < pad_rows * cols; i += (long)gridDim.x * blockDim.x) {
+    const long r = i / cols;
+    const int k = (int)(i - r * cols);
+    const __nv_bfloat16 v = __float2bfloat16(r < rows ? x[i] : 0.0f);
+    if (y && r < rows) y[i] = v;
+    yt[k * ldt + r] = v;
+  }
+}
+
 }  // namespace
 
-// Operand staging needs (128 + 256) x KC BF16 = 48 KB; the request is
-// padded to 96 KB so that at most two CTAs (2 x 256 TMEM columns, the SM's
-// 512) are resident per SM and no tcgen05.alloc has to wait for columns.
-size_t tc_gemm_smem_bytes() { return (size_t)96 * 1024; }
+// The stage ring takes 192 KB, so one CTA is resident per SM and no
+// tcgen05.alloc has to wait for columns.
+size_t tc_gemm_smem_bytes() { return (size_t)G_NST * G_STAGE * sizeof(__nv_bfloat16); }
 
 cudaError_t launch_tc_gemm(const TcGemmArgs &a, cudaStream_t s)
 {
@@ -575,7 +672,7 @@ cudaError_t launch_tc_gemm(const TcGemmArgs &a, cudaStream_t s)
                                        (int)tc_gemm_smem_bytes());
   if (e != cudaSuccess) return e;
   dim3 grid((unsigned)((a.M + 127) / 128), (unsigned)a.k_split);
-  tc_gemm_kernel<<<grid, 128, tc_gemm_smem_bytes(), s>>>(a);
+  tc_gemm_kernel<<<grid, G_THREADS, tc_gemm_smem_bytes(), s>>>(a);
   return cudaGetLastError();
 }
 
@@ -606,26 +703,37 @@ cudaError_t launch_sum_splits(const float *part, float *out, long n, int splits,
   return cudaGetLastError();
 }
 
-cudaError_t launch_col_sum(const float *x, float *out, int rows, int cols, long ld, cudaStream_t s)
+cudaError_t launch_col_sum(const float *x, float *part, float *out, int rows, int cols, long ld, cudaStream_t s)
 {
-  col_sum_kernel<<<(unsigned)((cols + 127) / 128), 128, 0, s>>>(x, out, rows, cols, ld);
-  return cudaGetLastError();
+  const int rows_per = (rows + COL_SUM_BLOCKS - 1) / COL_SUM_BLOCKS, blocks = (rows + rows_per - 1) / rows_per;
+  col_sum_kernel<<<dim3((unsigned)((cols + 31) / 32), (unsigned)blocks), 256, 0, s>>>(x, part, rows, cols, ld, rows_per);
+  cudaError_t e = cudaGetLastError();
+  return e != cudaSuccess ? e : launch_sum_splits(part, out, cols, blocks, s);
 }
 
 cudaError_t launch_surrogate_loss(const float *y, const float *tgt, int rows, int nrates, __nv_bfloat16 *dy,
-                                  float *dyf, float *loss, cudaStream_t s)
+                                  __nv_bfloat16 *dyt, long ldt, float *dyf, float *loss, cudaStream_t s)
 {
-  surrogate_loss_kernel<<<(unsigned)((rows + 127) / 128), 128, 0, s>>>(y, tgt, rows, nrates, dy, dyf, loss);
+  surrogate_loss_kernel<<<(unsigned)((rows + 127) / 128), 128, 0, s>>>(y, tgt, rows, nrates, dy, dyt, ldt, dyf, loss);
   return cudaGetLastError();
 }
 
-cudaError_t launch_adam(float *w, const float *g, float *m1, float *m2, __nv_bfloat16 *w16, long n, float lr, float b1,
-                        float b2, float eps, int step, cudaStream_t s)
+cudaError_t launch_adam(float *w, const float *g, float *m1, float *m2, __nv_bfloat16 *w16, __nv_bfloat16 *w16t, int din,
+                        long ldt, long n, float lr, float b1, float b2, float eps, int step, cudaStream_t s)
 {
   const float c1 = 1.0f / (1.0f - powf(b1, (float)step)), c2 = 1.0f / (1.0f - powf(b2, (float)step));
   long blocks = (n + 255) / 256;
   if (blocks > 4096) blocks = 4096;
-  adam_kernel<<<(unsigned)blocks, 256, 0, s>>>(w, g, m1, m2, w16, n, lr, b1, b2, eps, c1, c2);
+  adam_kernel<<<(unsigned)blocks, 256, 0, s>>>(w, g, m1, m2, w16, w16t, din, ldt, n, lr, b1, b2, eps, c1, c2);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_to_bf16_t(const float *x, __nv_bfloat16 *y, __nv_bfloat16 *yt, long rows, int cols, long pad_rows,
+                             long ldt, cudaStream_t s)
+{
+  long blocks = (pad_rows * cols + 255) / 256;
+  if (blocks > 4096) blocks = 4096;
+  to_bf16_t_kernel<<<(unsigned)blocks, 256, 0, s>>>(x, y, yt, rows, cols, pad_rows, ldt);
   return cudaGetLastError();
 }
 

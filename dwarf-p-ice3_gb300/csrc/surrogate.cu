@@ -30,11 +30,20 @@ struct Mlp {
   long nparam = 0;
   float *p = nullptr, *g = nullptr, *m1 = nullptr, *m2 = nullptr;  // [nparam]
   std::vector<__nv_bfloat16 *> w16;   // BF16 copies of W
+  // the transposes [din][ldt(l)], zero from dout to ldt, of the layers the
+  // backward pass contracts with (1 ..), valid for version t_version
+  std::vector<__nv_bfloat16 *> w16t;
+  long t_version = -1;
+  long ldt(int l) const { return (dout[l] + 15) / 16 * 16; }
   int *err = nullptr;
   float *loss = nullptr;
   // activation buffers for `cap` rows
   long cap = 0;
   __nv_bfloat16 *xb = nullptr, *dyb = nullptr, *dzb[2] = {nullptr, nullptr};
+  // transposes [columns][cap] for the weight gradients, zero from the batch's
+  // rows to the next multiple of 128
+  __nv_bfloat16 *xbt = nullptr, *dybt = nullptr, *dzt = nullptr;
+  std::vector<__nv_bfloat16 *> HT;    // [n_layers] [n_hid][cap]
   std::vector<__nv_bfloat16 *> H;     // [n_layers] [cap][n_hid]
   std::vector<float *> Z;             // [n_layers] [cap][n_hid]
   float *y = nullptr, *dyf = nullptr, *dzf = nullptr, *part = nullptr;
@@ -62,8 +71,11 @@ void free_acts(Mlp *m)
   cudaFree(m->xb); cudaFree(m->dyb); cudaFree(m->dzb[0]); cudaFree(m->dzb[1]);
   for (auto *h : m->H) cudaFree(h);
   for (auto *z : m->Z) cudaFree(z);
+  for (auto *h : m->HT) cudaFree(h);
+  cudaFree(m->xbt); cudaFree(m->dybt); cudaFree(m->dzt);
   cudaFree(m->y); cudaFree(m->dyf); cudaFree(m->dzf);
-  m->H.clear(); m->Z.clear();
+  m->H.clear(); m->Z.clear(); m->HT.clear();
+  m->xbt = m->dybt = m->dzt = nullptr;
   m->xb = m->dyb = m->dzb[0] = m->dzb[1] = nullptr;
   m->y = m->dyf = m->dzf = nullptr;
   m->cap = 0;
@@ -77,11 +89,16 @@ cudaError_t ensure_acts(Mlp *m, long n)
   cudaError_t e = cudaMalloc(&m->xb, sizeof(__nv_bfloat16) * c * m->n_in);
   if (e == cudaSuccess) e = cudaMalloc(&m->dyb, sizeof(__nv_bfloat16) * c * 16);
   for (int i = 0; i < 2 && e == cudaSuccess; ++i) e = cudaMalloc(&m->dzb[i], sizeof(__nv_bfloat16) * c * m->n_hid);
+  if (e == cudaSuccess) e = cudaMalloc(&m->xbt, sizeof(__nv_bfloat16) * c * m->n_in);
+  if (e == cudaSuccess) e = cudaMalloc(&m->dybt, sizeof(__nv_bfloat16) * c * 16);
+  if (e == cudaSuccess) e = cudaMalloc(&m->dzt, sizeof(__nv_bfloat16) * c * m->n_hid);
   m->H.assign(m->n_layers, nullptr);
   m->Z.assign(m->n_layers, nullptr);
+  m->HT.assign(m->n_layers, nullptr);
   for (int l = 0; l < m->n_layers && e == cudaSuccess; ++l) {
     e = cudaMalloc(&m->H[l], sizeof(__nv_bfloat16) * c * m->n_hid);
     if (e == cudaSuccess) e = cudaMalloc(&m->Z[l], sizeof(float) * c * m->n_hid);
+    if (e == cudaSuccess) e = cudaMalloc(&m->HT[l], sizeof(__nv_bfloat16) * c * m->n_hid);
   }
   if (e == cudaSuccess) e = cudaMalloc(&m->y, sizeof(float) * c * 16);
   if (e == cudaSuccess) e = cudaMalloc(&m->dyf, sizeof(float) * c * 16);
@@ -118,7 +135,7 @@ TcGemmArgs gemm(const __nv_bfloat16 *A, long sam, long sak, const __nv_bfloat16 
   return a;
 }
 
-// Forward of n rows already in m->xb; keeps Z and H of the hidden layers.
+// Forward of n rows already in m->xb; keeps Z, H and H transposed of the hidden layers.
 cudaError_t mlp_forward_dev(Mlp *m, int n, float *y_out, long ldy, cudaStream_t s)
 {
   cudaError_t e = cudaSuccess;
@@ -129,6 +146,7 @@ cudaError_t mlp_forward_dev(Mlp *m, int n, float *y_out, long ldy, cudaStream_t 
     a.bias = m->p + m->boff[l];
     a.Zout = m->Z[l]; a.ldz = m->n_hid;
     a.H = m->H[l]; a.ldh = m->n_hid;
+    a.HT = m->HT[l]; a.ldht = m->cap;
     e = launch_tc_gemm(a, s);
     in = m->H[l];
     ldin = m->n_hid;
@@ -200,7 +218,9 @@ cudaError_t mlp_infer_dev(Mlp *m, long n, const float *x, float *y, cudaStream_t
   return mlp_infer_layered(m, n, x, y, s);
 }
 
-int split_for(int n) { int sp = n / 512; return sp < 1 ? 1 : (sp > 32 ? 32 : sp); }
+// Batch ranges of a weight gradient: 256 rows each, so that a batch of 16,384
+// gives 64 x 2 tiles of a 256-wide layer for the 152 SMs.
+int split_for(int n) { int sp = n / 256; return sp < 1 ? 1 : (sp > 64 ? 64 : sp); }
 
 cudaError_t ensure_part(Mlp *m, long words)
 {
@@ -213,18 +233,34 @@ cudaError_t ensure_part(Mlp *m, long words)
   return e;
 }
 
-// dW (dout x din) = dZ^T (dout x n) * X (n x din), split over n, into g.
-cudaError_t weight_grad(Mlp *m, const __nv_bfloat16 *dz, long lddz, const __nv_bfloat16 *x, long ldx, int n, int dout,
-                        int din, float *gw, cudaStream_t s)
+// dW (dout x din) = dZ^T (dout x n) * X (n x din), split over n, into g, from
+// the transposes [dout][cap] and [din][cap].
+cudaError_t weight_grad(Mlp *m, const __nv_bfloat16 *dzt, const __nv_bfloat16 *xt, int n, int dout, int din, float *gw,
+                        cudaStream_t s)
 {
   const int sp = split_for(n);
-  cudaError_t e = ensure_part(m, (long)sp * dout * din);
-  if (e != cudaSuccess) return e;
-  TcGemmArgs a = gemm(dz, 1, lddz, x, 1, ldx, dout, din, n, EPI_STORE, m->err);
+  TcGemmArgs a = gemm(dzt, m->cap, 1, xt, m->cap, 1, dout, din, n, EPI_STORE, m->err);
+  a.padded = 1;
   a.k_split = sp;
   a.C = m->part; a.ldc = din;
-  e = launch_tc_gemm(a, s);
+  cudaError_t e = launch_tc_gemm(a, s);
   if (e == cudaSuccess) e = launch_sum_splits(m->part, gw, (long)dout * din, sp, s);
+  return e;
+}
+
+// The transposed BF16 weights, refreshed when the parameters were set from
+// outside (a training step keeps them in step itself).
+cudaError_t ensure_transposes(Mlp *m, cudaStream_t s)
+{
+  if (m->t_version == m->version) return cudaSuccess;
+  cudaError_t e = cudaSuccess;
+  m->w16t.resize(m->nl, nullptr);
+  for (int l = 1; l < m->nl && e == cudaSuccess; ++l) {
+    if (!m->w16t[l]) e = cudaMalloc(&m->w16t[l], sizeof(__nv_bfloat16) * (size_t)m->din[l] * m->ldt(l));
+    if (e == cudaSuccess)
+      e = launch_to_bf16_t(m->p + m->woff[l], nullptr, m->w16t[l], m->dout[l], m->din[l], m->ldt(l), m->ldt(l), s);
+  }
+  if (e == cudaSuccess) m->t_version = m->version;
   return e;
 }
 
@@ -232,15 +268,19 @@ cudaError_t weight_grad(Mlp *m, const __nv_bfloat16 *dz, long lddz, const __nv_b
 cudaError_t mlp_loss_grad(Mlp *m, int n, const float *x, const float *tgt, cudaStream_t s)
 {
   cudaError_t e = ensure_acts(m, n);
-  if (e == cudaSuccess) e = launch_to_bf16(x, m->xb, (long)n * m->n_in, s);
+  if (e == cudaSuccess) e = ensure_transposes(m, s);
+  const int n_max = m->n_hid > m->n_in ? m->n_hid : m->n_in;
+  if (e == cudaSuccess) e = ensure_part(m, (long)(split_for(n) * n_max > COL_SUM_BLOCKS ? split_for(n) * n_max : COL_SUM_BLOCKS) * m->n_hid);
+  const long pad = ((long)n + 127) / 128 * 128;
+  if (e == cudaSuccess) e = launch_to_bf16_t(x, m->xb, m->xbt, n, m->n_in, pad, m->cap, s);
   if (e == cudaSuccess) e = cudaMemsetAsync(m->loss, 0, sizeof(float), s);
   if (e == cudaSuccess) e = mlp_forward_dev(m, n, m->y, 16, s);
-  if (e == cudaSuccess) e = launch_surrogate_loss(m->y, tgt, n, m->n_out / 2, m->dyb, m->dyf, m->loss, s);
+  if (e == cudaSuccess) e = launch_surrogate_loss(m->y, tgt, n, m->n_out / 2, m->dyb, m->dybt, m->cap, m->dyf, m->loss, s);
   if (e != cudaSuccess) return e;
   // output layer: dW = dY^T H_last, db = column sums of dY
   const int L = m->nl - 1;
-  e = weight_grad(m, m->dyb, 16, m->H[m->n_layers - 1], m->n_hid, n, m->dout[L], m->din[L], m->g + m->woff[L], s);
-  if (e == cudaSuccess) e = launch_col_sum(m->dyf, m->g + m->boff[L], n, m->dout[L], 16, s);
+  e = weight_grad(m, m->dybt, m->HT[m->n_layers - 1], n, m->dout[L], m->din[L], m->g + m->woff[L], s);
+  if (e == cudaSuccess) e = launch_col_sum(m->dyf, m->part, m->g + m->boff[L], n, m->dout[L], 16, s);
   if (e != cudaSuccess) return e;
   int cur = 0;
   const __nv_bfloat16 *dnext = m->dyb;
@@ -248,15 +288,18 @@ cudaError_t mlp_loss_grad(Mlp *m, int n, const float *x, const float *tgt, cudaS
   for (int l = m->n_layers - 1; l >= 0 && e == cudaSuccess; --l) {
     // dZ_l = (dZ_{l+1} W_{l+1}) * GELU'(Z_l)
     const int lw = l + 1;  // weight layer consuming H_l
-    TcGemmArgs a = gemm(dnext, ldnext, 1, m->w16[lw], 1, m->din[lw], n, m->dout[l], m->dout[lw], EPI_DGELU, m->err);
+    TcGemmArgs a = gemm(dnext, ldnext, 1, m->w16t[lw], m->ldt(lw), 1, n, m->dout[l], m->dout[lw], EPI_DGELU, m->err);
+    // zeros past K: dY's columns and W^T's are padded to 16; a hidden layer's
+    // dZ has dout columns and nothing behind them
+    a.padded = lw == L;
     a.Zin = m->Z[l]; a.ldz = m->n_hid;
     a.H = m->dzb[cur]; a.ldh = m->n_hid;
+    a.HT = m->dzt; a.ldht = m->cap;
     a.C = m->dzf; a.ldc = m->n_hid;
     e = launch_tc_gemm(a, s);
-    if (e == cudaSuccess) e = launch_col_sum(m->dzf, m->g + m->boff[l], n, m->dout[l], m->n_hid, s);
-    const __nv_bfloat16 *xin = l > 0 ? m->H[l - 1] : m->xb;
-    const long ldx = l > 0 ? m->n_hid : m->n_in;
-    if (e == cudaSuccess) e = weight_grad(m, m->dzb[cur], m->n_hid, xin, ldx, n, m->dout[l], m->din[l], m->g + m->woff[l], s);
+    if (e == cudaSuccess) e = launch_col_sum(m->dzf, m->part, m->g + m->boff[l], n, m->dout[l], m->n_hid, s);
+    if (e == cudaSuccess)
+      e = weight_grad(m, m->dzt, l > 0 ? m->HT[l - 1] : m->xbt, n, m->dout[l], m->din[l], m->g + m->woff[l], s);
     dnext = m->dzb[cur];
     ldnext = m->n_hid;
     cur ^= 1;
@@ -365,6 +408,7 @@ int ice3gb_mlp_destroy(void *mlp)
   cudaFree(m->p); cudaFree(m->g); cudaFree(m->m1); cudaFree(m->m2); cudaFree(m->err); cudaFree(m->loss);
   cudaFree(m->part);
   for (auto *w : m->w16) cudaFree(w);
+  for (auto *w : m->w16t) cudaFree(w);
   m->magic = 0;
   delete m;
   return ICE3GB_OK;
@@ -447,13 +491,14 @@ int ice3gb_mlp_train_step(void *mlp, int n, const float *x, const float *tgt, fl
   cudaError_t e = mlp_loss_grad(m, n, x, tgt, s);
   m->step += 1;
   m->version += 1;
+  if (e == cudaSuccess) m->t_version = m->version;     // adam_kernel writes the transposes too
   for (int l = 0; l < m->nl && e == cudaSuccess; ++l) {
     const long nw = (long)m->din[l] * m->dout[l];
-    e = launch_adam(m->p + m->woff[l], m->g + m->woff[l], m->m1 + m->woff[l], m->m2 + m->woff[l], m->w16[l], nw, lr,
-                    0.9f, 0.999f, 1e-8f, m->step, s);
+    e = launch_adam(m->p + m->woff[l], m->g + m->woff[l], m->m1 + m->woff[l], m->m2 + m->woff[l], m->w16[l],
+                    l > 0 ? m->w16t[l] : nullptr, m->din[l], m->ldt(l), nw, lr, 0.9f, 0.999f, 1e-8f, m->step, s);
     if (e == cudaSuccess)
-      e = launch_adam(m->p + m->boff[l], m->g + m->boff[l], m->m1 + m->boff[l], m->m2 + m->boff[l], nullptr,
-                      m->dout[l], lr, 0.9f, 0.999f, 1e-8f, m->step, s);
+      e = launch_adam(m->p + m->boff[l], m->g + m->boff[l], m->m1 + m->boff[l], m->m2 + m->boff[l], nullptr, nullptr,
+                      1, 0, m->dout[l], lr, 0.9f, 0.999f, 1e-8f, m->step, s);
   }
   if (e == cudaSuccess && loss) e = cudaMemcpyAsync(loss, m->loss, sizeof(float), cudaMemcpyDeviceToDevice, s);
   return e == cudaSuccess ? ICE3GB_OK : ICE3GB_ERR_CUDA;
