@@ -242,8 +242,8 @@ FM_HD uint64_t exp_reduce_(uint32_t h, uint32_t l, uint64_t bias, uint32_t kb, u
 // 2^(k/512) e^r for r = R 2^-70 in (0, 2^-8.8), k = kb - 2^20: T + T (e^r - 1)
 // with T = 2^(j/512) 2^62 from the table and
 // e^r - 1 = r + r^2/2 + r^3 (1/6 + r/24 + r^2/120), all terms positive, each
-// held to 2^-60 or better of the result; rounded once to 53 bits.
-FM_HD double exp_core_(uint64_t R, uint32_t kb)
+// held to 2^-60 or better of the result; rounded once to 53 bits: q 2^(m - 52).
+FM_HD void exp_core_(uint64_t R, uint32_t kb, uint64_t &q, int32_t &m)
 {
   const uint64_t r2 = sqr70_(R);
   const uint32_t r40 = (uint32_t)(R >> 30);                       // r 2^40
@@ -254,8 +254,13 @@ FM_HD double exp_core_(uint64_t R, uint32_t kb)
   const uint64_t T = exp_entry(kb & 511u);
   const uint64_t y = T + mulhi64_(T, p);                          // [2^62, 2^63.004)
   const uint32_t ov = (uint32_t)(y >> 63);
-  const int32_t m = (int32_t)(kb >> 9) - 2048 + (int32_t)ov;
-  const uint64_t q = (y + (512u << ov)) >> (10u + ov);            // 53 bits
+  m = (int32_t)(kb >> 9) - 2048 + (int32_t)ov;
+  q = (y + (512u << ov)) >> (10u + ov);                           // 53 bits
+}
+
+// q 2^(m - 52), rounded once more only where it is subnormal.
+FM_HD double exp_scale_(uint64_t q, int32_t m)
+{
   if (m >= -1022 && m <= 1022) return from_bits_((int64_t)(q + ((uint64_t)(uint32_t)(m + 1022) << 52)));
   // gradual underflow / overflow edges: scale in two steps
   const double d = from_bits_((int64_t)(q + ((uint64_t)(uint32_t)(m / 2 + 1022) << 52)));
@@ -270,6 +275,12 @@ FM_HD uint32_t exp_index_(float x, float s)
   return (uint32_t)(fbits_(fmaf_(x, s, sh)) - fbits_(sh)) + 1048575u;
 }
 
+FM_HD void exp_parts_(double x, uint64_t &q, int32_t &m)
+{
+  const uint32_t kb = exp_index_(to_f32(x), FM_INV_L512_F);
+  exp_core_(exp_reduce_(hi_(x), lo_(x), FM_L512_BIAS, kb, FM_L512_HI, FM_L512_LO), kb, q, m);
+}
+
 // e^x.
 FM_NI double fexp(double x)
 {
@@ -279,8 +290,10 @@ FM_NI double fexp(double x)
     if (x > 709.782712893384) return from_bits_(0x7ff0000000000000LL);
     if (x < -745.1332191019412) return 0.0;
   }
-  const uint32_t kb = exp_index_(to_f32(x), FM_INV_L512_F);
-  return exp_core_(exp_reduce_(h, lo_(x), FM_L512_BIAS, kb, FM_L512_HI, FM_L512_LO), kb);
+  uint64_t q;
+  int32_t m;
+  exp_parts_(x, q, m);
+  return exp_scale_(q, m);
 }
 
 // 10^x.
@@ -294,7 +307,10 @@ FM_NI double fexp10(double x)
   }
   const uint32_t kb = exp_index_(to_f32(x), FM_INV_LG512_F);
   const uint64_t r10 = exp_reduce_(h, lo_(x), FM_LG512_BIAS, kb, FM_LG512_HI, FM_LG512_LO);
-  return exp_core_(mulhi64_(r10, FM_LN10_62) << 2, kb);
+  uint64_t q;
+  int32_t m;
+  exp_core_(mulhi64_(r10, FM_LN10_62) << 2, kb, q, m);
+  return exp_scale_(q, m);
 }
 
 // log1p(r) for |r| <= 2^-8 (exact r = x - 1): r + r^2 q, q to r in FP64 and
@@ -312,22 +328,10 @@ FM_NI double log_near1_(double x)
   return fma_(mul_(r, r), q, r);
 }
 
-// Natural logarithm.
-FM_NI double flog(double x)
+// log of a positive x = h : l outside log_near1_'s range, ebias = 1100 - 1023
+// (less 54 for a subnormal scaled by 2^54).
+FM_HD double log_core_(uint32_t h, uint32_t l, uint32_t ebias)
 {
-  uint32_t h = hi_(x), l = lo_(x);
-  uint32_t ebias = 77u;                                           // 1100 - 1023
-  if (h - 0x3fefe000u < 0x3000u) return log_near1_(x);            // 1 - 2^-8 <= x < 1 + 2^-8
-  if (h - 0x00100000u >= 0x7fe00000u) {                           // <= 0, subnormal, inf, NaN
-    if (x != x) return x;
-    if (x < 0.0) return from_bits_(0x7ff8000000000000LL);
-    if (x == 0.0) return from_bits_((int64_t)0xfff0000000000000ULL);
-    if (h >= 0x7ff00000u) return x;                               // +inf
-    x = mul_(x, 18014398509481984.0);                             // subnormal: * 2^54
-    h = hi_(x);
-    l = lo_(x);
-    ebias = 77u - 54u;
-  }
   const LogEntry t = log_entry((h >> 11) & 511u);
   const uint32_t eb = (h >> 20) + ebias;                          // e + 1100
   // r 2^70 = (z c / 2048 - 1) 2^70, exact
@@ -354,6 +358,53 @@ FM_NI double flog(double x)
   const uint64_t top = ((uint64_t)funnel_l_(v1, v2, lz) << 32) | funnel_l_(v0, v1, lz);
   const uint64_t q = (top >> 11) + ((uint32_t)(top >> 10) & 1u);
   return from_bits_((int64_t)(q + ((uint64_t)(1045u - lz) << 52) + ((uint64_t)(sg & 0x80000000u) << 32)));
+}
+
+// Natural logarithm.
+FM_NI double flog(double x)
+{
+  uint32_t h = hi_(x), l = lo_(x);
+  uint32_t ebias = 77u;                                           // 1100 - 1023
+  if (h - 0x3fefe000u < 0x3000u) return log_near1_(x);            // 1 - 2^-8 <= x < 1 + 2^-8
+  if (h - 0x00100000u >= 0x7fe00000u) {                           // <= 0, subnormal, inf, NaN
+    if (x != x) return x;
+    if (x < 0.0) return from_bits_(0x7ff8000000000000LL);
+    if (x == 0.0) return from_bits_((int64_t)0xfff0000000000000ULL);
+    if (h >= 0x7ff00000u) return x;                               // +inf
+    x = mul_(x, 18014398509481984.0);                             // subnormal: * 2^54
+    h = hi_(x);
+    l = lo_(x);
+    ebias = 77u - 54u;
+  }
+  return log_core_(h, l, ebias);
+}
+
+// Two logarithms / exponentials at once: the two dependent chains of integer
+// operations overlap, where a single one leaves a warp waiting for its own
+// results (used where a warp needs pairs and its latency counts).
+struct Pair { double a, b; };
+FM_HD bool log_plain_(double x)                                   // normal, positive, not next to 1
+{
+  const uint32_t h = hi_(x);
+  return h - 0x00100000u < 0x7fe00000u && h - 0x3fefe000u >= 0x3000u;
+}
+FM_NI Pair flog2(double a, double b)
+{
+  if (log_plain_(a) && log_plain_(b)) return {log_core_(hi_(a), lo_(a), 77u), log_core_(hi_(b), lo_(b), 77u)};
+  return {flog(a), flog(b)};
+}
+FM_NI Pair fexp2(double a, double b)
+{
+  // (|x| < 700: no overflow, no subnormal result)
+  if ((hi_(a) & 0x7fffffffu) < 0x4085e000u && (hi_(b) & 0x7fffffffu) < 0x4085e000u) {
+    uint64_t qa, qb;
+    int32_t ma, mb;
+    exp_parts_(a, qa, ma);
+    exp_parts_(b, qb, mb);
+    return {from_bits_((int64_t)(qa + ((uint64_t)(uint32_t)(ma + 1022) << 52))),
+            from_bits_((int64_t)(qb + ((uint64_t)(uint32_t)(mb + 1022) << 52)))};
+  }
+  return {fexp(a), fexp(b)};
 }
 
 // the IEEE division, out of line (the rare fallback of the paths below)
