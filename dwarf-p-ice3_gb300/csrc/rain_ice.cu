@@ -193,11 +193,12 @@ cudaError_t launch_rain_ice_points(const Cst &c, const RainIceArgs &a, int num_s
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rain_ice_smem_bytes());
   if (e != cudaSuccess) return e;
   const long n = (long)a.nij * a.nk;
-  long chunks = (n + RI_THREADS - 1) / RI_THREADS;
+  const int threads = ri_threads(n, num_sms);
+  long chunks = (n + threads - 1) / threads;
   long blocks = (long)num_sms * RI_BLOCKS_PER_SM;
   if (blocks > chunks) blocks = chunks;
   if (blocks < 1) blocks = 1;
-  kern<<<(unsigned)blocks, RI_THREADS, rain_ice_smem_bytes(), s>>>(c, a);
+  kern<<<(unsigned)blocks, threads, rain_ice_smem_bytes(), s>>>(c, a);
   return cudaGetLastError();
 }
 

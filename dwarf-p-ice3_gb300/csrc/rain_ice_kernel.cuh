@@ -22,6 +22,27 @@
 namespace ice3ri {
 using namespace ice3pt;
 
+// The lookup tables into shared memory, 16 bytes a load, eight in flight (a
+// block of one warp stages all 78.7 KB too).
+__device__ __forceinline__ void stage_luts(double *lut, const double *src)
+{
+  static_assert(LUT_N % 2 == 0, "16-byte loads");
+  double2 *d = reinterpret_cast<double2 *>(lut);
+  const double2 *g = reinterpret_cast<const double2 *>(src);
+#pragma unroll 8
+  for (int i = threadIdx.x; i < LUT_N / 2; i += blockDim.x) d[i] = __ldg(g + i);
+}
+
+// Threads per block: RI_THREADS where that fills the SMs; a smaller call is
+// spread over them in blocks of as few warps as cover it (2,880 points: 6
+// blocks of 512 threads take 140 us, the FP64 pipes of 6 SMs shared by 16
+// warps each).
+inline int ri_threads(long n, int num_sms)
+{
+  const long per_sm = (n + num_sms - 1) / num_sms, warps = (per_sm + 31) / 32;
+  return warps >= RI_THREADS / 32 ? RI_THREADS : (int)(warps < 1 ? 32 : 32 * warps);
+}
+
 __device__ __forceinline__ void warp_key_max(unsigned int *key_max, unsigned int key)
 {
   const unsigned int m = __reduce_max_sync(0xffffffffu, key);
@@ -37,9 +58,9 @@ template <bool SUBG, bool H = false, bool O = false, bool TS = false>
 __global__ void __launch_bounds__(RI_THREADS, RI_BLOCKS_PER_SM) rain_ice_points_kernel(const __grid_constant__ Cst c,
                                                                          const __grid_constant__ RainIceArgs a)
 {
-  extern __shared__ double lut[];
+  extern __shared__ __align__(16) double lut[];
   __shared__ Derived dsh;
-  for (int i = threadIdx.x; i < LUT_N; i += blockDim.x) lut[i] = a.luts[i];
+  stage_luts(lut, a.luts);
   if (threadIdx.x == 0) make_derived(c, dsh);
   __shared__ unsigned int chunk;
   __syncthreads();

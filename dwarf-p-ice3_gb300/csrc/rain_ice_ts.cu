@@ -22,10 +22,11 @@ cudaError_t launch_rain_ice_points_ts(const Cst &c, const RainIceArgs &a, int nu
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
   const long n = (long)a.nij * a.nk;
-  long chunks = (n + RI_THREADS - 1) / RI_THREADS;
+  const int threads = ice3ri::ri_threads(n, num_sms);
+  long chunks = (n + threads - 1) / threads;
   long blocks = (long)num_sms * RI_BLOCKS_PER_SM;
   if (blocks > chunks) blocks = chunks;
   if (blocks < 1) blocks = 1;
-  kern<<<(unsigned)blocks, RI_THREADS, smem, s>>>(c, a);
+  kern<<<(unsigned)blocks, threads, smem, s>>>(c, a);
   return cudaGetLastError();
 }

@@ -16,6 +16,7 @@
 //   points without a row.
 #include "ice3gb_device.cuh"
 #include "ice3gb_kernels.h"
+#include "rain_ice_kernel.cuh"
 #include "surrogate_point.cuh"
 
 // One block of RI_THREADS per SM, as the plain rain_ice kernel.
@@ -41,10 +42,10 @@ template <bool RATES>
 __global__ void __launch_bounds__(SAMPLE_THREADS) surrogate_sample_kernel(const __grid_constant__ Cst c,
                                                                           const __grid_constant__ SurSampleArgs a)
 {
-  extern __shared__ double lut[];
+  extern __shared__ __align__(16) double lut[];
   __shared__ Derived dsh;
   if (RATES)
-    for (int i = threadIdx.x; i < LUT_N; i += blockDim.x) lut[i] = a.luts[i];
+    ice3ri::stage_luts(lut, a.luts);
   if (threadIdx.x == 0) make_derived(c, dsh);
   __syncthreads();
   const long n = (long)a.nij * a.nk;
@@ -122,7 +123,7 @@ __device__ __forceinline__ bool finite_(double x) { return (fm::bits_(x) & 0x7ff
 __global__ void __launch_bounds__(RI_THREADS, RI_BLOCKS_PER_SM)
     rain_ice_surrogate_kernel(const __grid_constant__ Cst c, const __grid_constant__ SurRainIceArgs sa)
 {
-  extern __shared__ double lut[];
+  extern __shared__ __align__(16) double lut[];
   __shared__ Derived dsh;
   // the in-out fields a point starts from, for the fall-back to the plain
   // path: kept in shared memory rather than in registers across the point
@@ -130,7 +131,7 @@ __global__ void __launch_bounds__(RI_THREADS, RI_BLOCKS_PER_SM)
   __shared__ double s_in[8][RI_THREADS];
   __shared__ double s_sur[RI_THREADS][NRATE];          // the decoded learned rates of a thread's point
   const RainIceArgs &a = sa.ri;
-  for (int i = threadIdx.x; i < LUT_N; i += blockDim.x) lut[i] = a.luts[i];
+  ice3ri::stage_luts(lut, a.luts);
   if (threadIdx.x == 0) make_derived(c, dsh);
   __shared__ unsigned int chunk;
   __syncthreads();
@@ -217,10 +218,11 @@ cudaError_t launch_rain_ice_surrogate(const Cst &c, const SurRainIceArgs &a, int
                                        (int)lut_smem_bytes());
   if (e != cudaSuccess) return e;
   const long n = (long)a.ri.nij * a.ri.nk;
-  long chunks = (n + RI_THREADS - 1) / RI_THREADS;
+  const int threads = ice3ri::ri_threads(n, num_sms);
+  long chunks = (n + threads - 1) / threads;
   long blocks = (long)num_sms * RI_BLOCKS_PER_SM;
   if (blocks > chunks) blocks = chunks;
   if (blocks < 1) blocks = 1;
-  rain_ice_surrogate_kernel<<<(unsigned)blocks, RI_THREADS, lut_smem_bytes(), s>>>(c, a);
+  rain_ice_surrogate_kernel<<<(unsigned)blocks, threads, lut_smem_bytes(), s>>>(c, a);
   return cudaGetLastError();
 }
