@@ -67,8 +67,27 @@ class Ice3Handle:
         return bits.value
 
 
+def _copies(fields):
+    """Copies of what a call updates in place, each with its own storage; on
+    the device in one launch (a copy each is most of a small call's time)."""
+    if not all(type(f) is torch.Tensor and f.is_cuda and f.dtype is torch.float64 and not f.requires_grad
+               and f.device == fields[0].device for f in fields):
+        return [f.clone() for f in fields]
+    out = [torch.empty_like(f, memory_format=torch.contiguous_format) for f in fields]
+    torch._foreach_copy_(out, fields)
+    return out
+
+
+def _struct(cls, tensors: Mapping[str, Optional[torch.Tensor]]):
+    """The ABI structure of pointers: one constructor call instead of a
+    descriptor access per field; members without a tensor are NULL."""
+    return cls(*[0 if (t := tensors.get(k)) is None else t.data_ptr() for k, _ in cls._fields_])
+
+
 def _as_device_f64(x, like: Optional[torch.Tensor] = None) -> torch.Tensor:
     if isinstance(x, torch.Tensor):
+        if like is not None and x.dtype is torch.float64 and x.device == like.device:
+            return x.contiguous()
         t = x
     else:
         t = torch.as_tensor(np.asarray(x, dtype=np.float64))
@@ -127,23 +146,17 @@ class IceAdjust:
         shape = tuple(ref.shape)
         dev = {k: _as_device_f64(v, ref) for k, v in args.items()}
         for k, v in dev.items():
-            if k not in ("sigqsat", "ice_cld_wgt") and tuple(v.shape) != shape:
+            if v.shape != ref.shape and k not in ("sigqsat", "ice_cld_wgt"):
                 raise ValueError(f"{k} has shape {tuple(v.shape)}, expected {shape}")
         nij, nk, sig3d = self._geometry(shape, tuple(dev["sigqsat"].shape))
         outs = {k: torch.empty(shape, dtype=torch.float64, device=ref.device) for k in IA_OUTPUTS}
-        io = {k: dev[k].clone() for k in IA_INOUT}
-        f = _abi.IceAdjustFields()
-        for k in IA_INPUTS:
-            setattr(f, k, _ptr(dev[k]))
-        for k, v in {**io, **outs}.items():
-            setattr(f, k, _ptr(v))
-        f.sigqsat_3d = sig3d
+        io = dict(zip(IA_INOUT, _copies([dev[k] for k in IA_INOUT])))
         srcs = torch.empty(shape, dtype=torch.float64, device=ref.device) if return_srcs else None
-        f.srcs = _ptr(srcs)
+        f = _struct(_abi.IceAdjustFields, {**dev, **io, **outs, "srcs": srcs})
+        f.sigqsat_3d = sig3d
         extra = ()
         if self.ocnd2:
             self._check_ocnd2(shape, nij, tuple(dev["ice_cld_wgt"].shape))
-            f.zz, f.ice_cld_wgt = _ptr(dev["zz"]), _ptr(dev["ice_cld_wgt"])
             extra = tuple(torch.empty(shape, dtype=torch.float64, device=ref.device) for _ in _abi.OCND2_OUTPUTS)
             for k, v in zip(_abi.OCND2_OUTPUTS, extra):
                 setattr(f, k, _ptr(v))
@@ -295,12 +308,13 @@ class RainIce:
                     raise KeyError(f"state is missing {key!r}")
             fields[abi] = self._to_kij(v)
         nk, nij = fields["tht"].shape[0], int(np.prod(fields["tht"].shape[1:]))
-        for key, abi in RI_STATE_INOUT.items():
+        inout = []
+        for key in RI_STATE_INOUT:
             v = get(key)
             if v is None:
-                if key.startswith("hl") or key == "ci_t" or key.endswith("s"):
-                    v = torch.zeros(shape, dtype=torch.float64, device=ref_t.device)
-            fields[abi] = self._to_kij(v).clone()
+                v = torch.zeros(shape, dtype=torch.float64, device=ref_t.device)
+            inout.append(self._to_kij(v))
+        fields.update(zip(RI_STATE_INOUT.values(), _copies(inout)))
         hail = self.table.values["NRR"] == 7.0
         if hail:
             # NRR = 7: hail at t and its source (RainIceJAX's state has no hail;
@@ -335,12 +349,7 @@ class RainIce:
             diag["inprh"] = torch.empty((nij,), dtype=torch.float64, device=dev)
             if with_fluxes:
                 diag["fpr_h"] = torch.empty((nk, nij), dtype=torch.float64, device=dev)
-        f = _abi.RainIceFields()
-        for k, v in fields.items():
-            setattr(f, k, _ptr(v))
-        for k, v in diag.items():
-            setattr(f, k, _ptr(v))
-        f.sea, f.town = _ptr(sea), _ptr(town)
+        f = _struct(_abi.RainIceFields, {**fields, **diag, "sea": sea, "town": town})
         return {"f": f, "fields": fields, "diag": diag, "sea": sea, "town": town, "nij": nij, "nk": nk,
                 "shape": shape, "host": host}
 
