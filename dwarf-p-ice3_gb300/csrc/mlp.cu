@@ -257,32 +257,37 @@ __global__ void __launch_bounds__(G_THREADS) tc_gemm_kernel(const TcGemmArgs a)
 
 // ---------------------------------------------------------------------------
 // Fused inference of the surrogate's MLP shape (16 -> 256 -> 256 -> 256 ->
-// n_out <= 16, GELU): one persistent CTA per SM walks 128-row tiles.  Per
-// tile the 128 x 256 FP32 accumulators of consecutive layers alternate
-// between the two halves of TMEM (columns 0-255 and 256-511), the BF16
-// activations sit in shared memory (64 KB, K-major core matrices), W1 and
-// the output layer stay resident in shared memory, and W2 / W3 stream from
-// L2 as eight 32 KB K-chunks (pre-packed in the core-matrix layout) through
-// a four-stage ring filled by bulk asynchronous copies.  Thread 0 issues the
-// copies and the tcgen05.mma; all 16 warps run the epilogues (tcgen05.ld,
-// bias, GELU, BF16 pack into the activation tile) in two halves of 128
-// columns: the MMAs of the next layer's first two K-chunks (the first
-// half's activations) run while the warps form the second half.
-constexpr int FZ_NST = 4;                               // weight ring stages (3: 5.14, 4: 4.98 ms on 8.4 M rows)
-constexpr int FZ_THREADS = 512;                         // 16 warps: 4 row groups x 4 column quarters
-constexpr uint32_t FZ_CHUNK_BYTES = 256 * 64 * 2;       // one K-chunk of W2 / W3
-constexpr int FZ_OFF_H = 0, FZ_OFF_STAGE = 65536, FZ_OFF_W1 = FZ_OFF_STAGE + FZ_NST * 32768;
-constexpr int FZ_OFF_W4 = FZ_OFF_W1 + 8192, FZ_OFF_X = FZ_OFF_W4 + 8192, FZ_OFF_B = FZ_OFF_X + 4096;
+// n_out <= 16, GELU): one persistent CTA per SM walks 128-row tiles, two of
+// them in flight (slots 0 and 1).  Each slot has a 128 x 256 FP32 accumulator
+// in TMEM (all 512 columns together) and a BF16 activation tile in shared
+// memory (64 KB, K-major core matrices); W1 and the output layer stay
+// resident in shared memory, and W2 / W3 stream from L2 in 16 KB K-chunks
+// (pre-packed in the core-matrix layout) through a four-stage ring of bulk
+// asynchronous copies.  The warps have roles:
+//   0-15   bias + GELU of a hidden layer's accumulator into the activation
+//          tile (warp w: rows 32 (w % 4) .. + 31, columns 64 (w / 4) .. + 63)
+//   16-19  the input rows -> BF16, and the output rows
+//   20     one thread issues the tcgen05.mma: layer by layer, slot 0 then 1
+//   21     one thread issues the weight copies
+// so that the MMAs of one slot run while the other slot's GELU does.
+// Bound: the GELU warps (32,768 hardware tanh per layer and tile at 16 per
+// clock, and the FP32 operations around them, 1.2 us) - the MMAs (1.4 us per
+// hidden layer and tile) are behind them.  2 M rows take 0.84 ms (684
+// TFLOP/s); with one tile in flight and all warps in step, MMAs and GELU
+// largely in turn, they took 1.21 ms.
+constexpr int FZ_NST = 4;                               // weight ring stages
+constexpr int FZ_KC = 32;                               // K of a weight chunk
+constexpr int FZ_GELU_WARPS = 16, FZ_IO_WARP = 16, FZ_MMA_WARP = 20, FZ_COPY_WARP = 21, FZ_THREADS = 32 * 22;
+constexpr uint32_t FZ_CHUNK_BYTES = 256 * FZ_KC * 2;
+constexpr int FZ_CHUNKS = 256 / FZ_KC;                  // per hidden layer
+constexpr int FZ_OFF_H = 0, FZ_OFF_STAGE = 2 * 65536, FZ_OFF_W1 = FZ_OFF_STAGE + FZ_NST * FZ_CHUNK_BYTES;
+constexpr int FZ_OFF_W4 = FZ_OFF_W1 + 8192, FZ_OFF_X = FZ_OFF_W4 + 8192, FZ_OFF_B = FZ_OFF_X + 2 * 4096;
 constexpr int FZ_SMEM = FZ_OFF_B + (3 * 256 + 16) * 4;
 
 // Bias + GELU of 32 accumulator columns (from cb0) of one row into the
-// activation tile.  In an epilogue half h, warp w holds TMEM lanes
-// 32 (w % 4) .. + 31 (its rows) and the columns 128 h + 32 (w / 4) .. + 31;
-// the load of the second half is in flight while the first half's GELU runs
-// (the MUFU tanh is the epilogue's bound); the biases are read four at a
-// time (the same address for the whole warp).
-__device__ __forceinline__ void fz_gelu_half(const uint32_t r[32], const float *bias, int cb0, int row,
-                                             __nv_bfloat16 *sH)
+// activation tile (the MUFU tanh is the epilogue's bound); the biases are read
+// four at a time (the same address for the whole warp).
+__device__ __forceinline__ void fz_gelu32(const uint32_t r[32], const float *bias, int cb0, int row, __nv_bfloat16 *sH)
 {
 #pragma unroll
   for (int g = 0; g < 4; ++g) {
@@ -302,21 +307,21 @@ __device__ __forceinline__ void fz_gelu_half(const uint32_t r[32], const float *
 __global__ void __launch_bounds__(FZ_THREADS, 1) mlp_fused_kernel(const MlpFusedArgs a)
 {
   extern __shared__ __align__(1024) unsigned char smem[];
-  __nv_bfloat16 *sH = reinterpret_cast<__nv_bfloat16 *>(smem + FZ_OFF_H);
-  __nv_bfloat16 *sW1 = reinterpret_cast<__nv_bfloat16 *>(smem + FZ_OFF_W1);
-  __nv_bfloat16 *sW4 = reinterpret_cast<__nv_bfloat16 *>(smem + FZ_OFF_W4);
-  __nv_bfloat16 *sX = reinterpret_cast<__nv_bfloat16 *>(smem + FZ_OFF_X);
   float *sB = reinterpret_cast<float *>(smem + FZ_OFF_B);
-  __shared__ __align__(8) uint64_t bar_mma, bar_full[FZ_NST], bar_free[FZ_NST];
+  // acc: a hidden layer's accumulator is ready; out: the output layer's; in:
+  // the input tile is written (and the slot's last output read); act: the
+  // activation tile is written (and the accumulator read)
+  __shared__ __align__(8) uint64_t bar_acc[2], bar_out[2], bar_in[2], bar_act[2], bar_full[FZ_NST], bar_free[FZ_NST],
+      bar_end;
   __shared__ uint32_t tmem_base;
-  const int tid = threadIdx.x, warp = tid >> 5;
+  __shared__ int failed;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const long ntiles = (a.n + 127) / 128;
   const long my_tiles = blockIdx.x < ntiles ? (ntiles - 1 - blockIdx.x) / gridDim.x + 1 : 0;
-  const long total_chunks = 8 * my_tiles;
   // resident operands: W1 (256 x 16), output layer (16 x 256), biases
   for (int i = tid; i < 4096 / 8; i += FZ_THREADS) {
-    reinterpret_cast<uint4 *>(sW1)[i] = __ldg(reinterpret_cast<const uint4 *>(a.w1) + i);
-    reinterpret_cast<uint4 *>(sW4)[i] = __ldg(reinterpret_cast<const uint4 *>(a.w4) + i);
+    reinterpret_cast<uint4 *>(smem + FZ_OFF_W1)[i] = __ldg(reinterpret_cast<const uint4 *>(a.w1) + i);
+    reinterpret_cast<uint4 *>(smem + FZ_OFF_W4)[i] = __ldg(reinterpret_cast<const uint4 *>(a.w4) + i);
   }
   for (int i = tid; i < 256; i += FZ_THREADS) {
     sB[i] = a.b1[i];
@@ -325,11 +330,18 @@ __global__ void __launch_bounds__(FZ_THREADS, 1) mlp_fused_kernel(const MlpFused
   }
   if (tid < 16) sB[768 + tid] = tid < a.n_out ? a.b4[tid] : 0.0f;
   if (tid == 0) {
-    tc::mbar_init(&bar_mma, 1);
+    for (int s = 0; s < 2; ++s) {
+      tc::mbar_init(&bar_acc[s], 1);
+      tc::mbar_init(&bar_out[s], 1);
+      tc::mbar_init(&bar_in[s], 4);
+      tc::mbar_init(&bar_act[s], FZ_GELU_WARPS);
+    }
     for (int s = 0; s < FZ_NST; ++s) {
       tc::mbar_init(&bar_full[s], 1);
       tc::mbar_init(&bar_free[s], 1);
     }
+    tc::mbar_init(&bar_end, 1);
+    failed = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 0) tc::tmem_alloc(&tmem_base, 512);
@@ -338,183 +350,152 @@ __global__ void __launch_bounds__(FZ_THREADS, 1) mlp_fused_kernel(const MlpFused
   __syncthreads();
   tc::fence_after();
   const uint32_t tmem = tmem_base;
-  const uint32_t id256 = tc::idesc_bf16_f32(128, 256), id16 = tc::idesc_bf16_f32(128, 16);
-  const uint32_t aH = tc::smem_u32(sH), aX = tc::smem_u32(sX), aW1 = tc::smem_u32(sW1), aW4 = tc::smem_u32(sW4);
-  long issued = 0, consumed = 0;       // weight chunks (thread 0's bookkeeping)
-  uint32_t mma_phase = 0;
   bool ok = true;
-  // chunk g of the stream: W2 chunks 0..3, then W3 chunks 0..3, per tile
-  auto issue = [&](long g) -> bool {
-    const int s = (int)(g % FZ_NST);
-    if (g >= FZ_NST && !tc::mbar_wait(&bar_free[s], (uint32_t)((g / FZ_NST - 1) & 1), WAIT_ITERS)) return false;
-    const int j = (int)(g % 8);
-    const __nv_bfloat16 *src = (j < 4 ? a.w2 : a.w3) + (long)(j & 3) * (256 * 64);
-    tc::mbar_expect_tx(&bar_full[s], FZ_CHUNK_BYTES);
-    tc::bulk_g2s(smem + FZ_OFF_STAGE + s * 32768, src, FZ_CHUNK_BYTES, &bar_full[s]);
-    ++issued;
-    return true;
-  };
-  if (tid == 0)
-    for (long g = 0; g < FZ_NST - 1 && g < total_chunks && ok; ++g) ok = issue(g);
-  // Accumulators: the layers alternate between TMEM columns 0-255 (A) and
-  // 256-511 (B), so that the MMAs of a layer's first K half (activation
-  // columns 0-127, written by the first half of the previous epilogue) run
-  // while the warps form the second half of that epilogue.
-  const uint32_t tA = tmem, tB = tmem + 256u;
-  const int lane = tid & 31, q4 = warp & 3, row = 32 * q4 + lane;
-  auto ld_half = [&](uint32_t tacc, int h, uint32_t r[32]) {
-    tc::tmem_ld32_nowait(tacc + ((uint32_t)(32 * q4) << 16) + (uint32_t)(128 * h + 32 * (warp >> 2)), r);
-  };
-  auto gelu_half = [&](const uint32_t r[32], const float *bias, int h) {
-    fz_gelu_half(r, bias, 128 * h + 32 * (warp >> 2), row, sH);
-  };
-  auto sync_async = [&]() {     // activation writes visible to the tensor core; TMEM accesses ordered
+  // this warp's writes to shared memory and reads of TMEM are done
+  auto warp_arrive = [&](uint64_t *bar) {
     tc::fence_async_smem();
     tc::fence_before();
-    __syncthreads();
-    tc::fence_after();
+    __syncwarp();
+    if (lane == 0) tc::mbar_arrive(bar);
   };
-  long n_commit = 0;            // commits to bar_mma (thread 0)
-  bool uncommitted = false;     // MMAs issued after the last commit to bar_mma (thread 0)
-  // thread 0: the MMAs of K-chunks c0, c0 + 1 of a hidden layer into tacc
-  auto mma_chunks = [&](uint32_t tacc, int c0) -> bool {
-    for (int c = c0; c < c0 + 2; ++c) {
-      const long g = consumed;
-      const int s = (int)(g % FZ_NST);
-      if (!tc::mbar_wait(&bar_full[s], (uint32_t)((g / FZ_NST) & 1), WAIT_ITERS)) return false;
-      tc::fence_after();
-      const uint32_t aS = tc::smem_u32(smem + FZ_OFF_STAGE + s * 32768);
-#pragma unroll
-      for (int j = 0; j < 4; ++j)
-        tc::mma_bf16(tacc, tc::desc(aH + (uint32_t)(c * 8 + 2 * j) * 128u, 128u, 4096u),
-                     tc::desc(aS + (uint32_t)(2 * j) * 128u, 128u, 1024u), id256, c > 0 || j > 0);
-      uncommitted = true;
-      tc::commit(&bar_free[s]);
-      ++consumed;
-      const long gn = g + FZ_NST - 1;
-      if (gn < total_chunks && gn >= issued && !issue(gn)) return false;
-    }
-    return true;
-  };
-  auto commit_mma = [&]() {
-    tc::commit(&bar_mma);
-    ++n_commit;
-    uncommitted = false;
-  };
-  // all threads: wait for the last commit to bar_mma
-  auto wait_mma = [&]() -> bool {
-    ok = __syncthreads_and(ok && tc::mbar_wait(&bar_mma, mma_phase, WAIT_ITERS)) != 0;
-    mma_phase ^= 1u;
-    tc::fence_after();
-    return ok;
-  };
-  long tile = blockIdx.x;
-  for (long it = 0; it < my_tiles; ++it, tile += gridDim.x) {
-    const long r0 = tile * 128;
-    // ---- input rows -> BF16 tile (threads 0..127, one row each)
-    if (tid < 128) {
-      const long rw = r0 + tid;
-      float x[16];
-      if (rw < a.n) {
-        const float4 *xp = reinterpret_cast<const float4 *>(a.x + rw * 16);
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          const float4 v = __ldg(xp + q);
-          x[4 * q] = v.x; x[4 * q + 1] = v.y; x[4 * q + 2] = v.z; x[4 * q + 3] = v.w;
+  if (warp < FZ_GELU_WARPS) {
+    const int row = 32 * (warp & 3) + lane, c0 = 64 * (warp >> 2);
+    const uint32_t lanes = (uint32_t)(32 * (warp & 3)) << 16;
+    uint32_t phase[2] = {0u, 0u};
+    for (long t0 = 0; t0 < my_tiles && ok; t0 += 2)
+      for (int layer = 0; layer < 3 && ok; ++layer)
+        for (int s = 0; s < 2 && t0 + s < my_tiles; ++s) {
+          ok = tc::mbar_wait(&bar_acc[s], phase[s], WAIT_ITERS);
+          if (!__all_sync(0xffffffffu, ok)) { ok = false; break; }
+          phase[s] ^= 1u;
+          tc::fence_after();
+          const uint32_t acc = tmem + 256u * s + lanes + (uint32_t)c0;
+          __nv_bfloat16 *sH = reinterpret_cast<__nv_bfloat16 *>(smem + FZ_OFF_H + 65536 * s);
+          uint32_t r0[32], r1[32];
+          tc::tmem_ld32_nowait(acc, r0);
+          tc::tmem_wait_ld();
+          tc::tmem_ld32_nowait(acc + 32u, r1);       // in flight during the first half
+          fz_gelu32(r0, sB + 256 * layer, c0, row, sH);
+          tc::tmem_wait_ld();
+          fz_gelu32(r1, sB + 256 * layer, c0 + 32, row, sH);
+          warp_arrive(&bar_act[s]);
         }
-      } else {
+  } else if (warp < FZ_MMA_WARP) {
+    // ---- input and output rows (thread = row of the tile)
+    const int row = 32 * (warp & 3) + lane;
+    const uint32_t lanes = (uint32_t)(32 * (warp & 3)) << 16;
+    float4 x[4];
+    auto load = [&](long t) {
+      const long rw = ((long)blockIdx.x + t * gridDim.x) * 128 + row;
 #pragma unroll
-        for (int q = 0; q < 16; ++q) x[q] = 0.0f;
-      }
-      *reinterpret_cast<uint4 *>(sX + tc::core_off(tid, 0, 16)) =
-          make_uint4(bf16x2_bits(x[0], x[1]), bf16x2_bits(x[2], x[3]), bf16x2_bits(x[4], x[5]), bf16x2_bits(x[6], x[7]));
-      *reinterpret_cast<uint4 *>(sX + tc::core_off(tid, 8, 16)) =
-          make_uint4(bf16x2_bits(x[8], x[9]), bf16x2_bits(x[10], x[11]), bf16x2_bits(x[12], x[13]),
-                     bf16x2_bits(x[14], x[15]));
-    }
-    sync_async();
-    // ---- layer 1: K = 16, one MMA into A
-    if (tid == 0) {
-      tc::mma_bf16(tA, tc::desc(aX, 128u, 256u), tc::desc(aW1, 128u, 256u), id256, false);
-      commit_mma();
-    }
-    if (!wait_mma()) break;
-    // ---- layers 2 (into B) and 3 (into A): K = 256 in four chunks; the
-    // first two chunks start after the first half of the previous epilogue
-    for (int layer = 0; layer < 2 && ok; ++layer) {
-      const uint32_t tprev = layer == 0 ? tA : tB, tcur = layer == 0 ? tB : tA;
-      const float *bprev = sB + 256 * layer;
-      uint32_t rh0[32], rh1[32];
-      ld_half(tprev, 0, rh0);
-      tc::tmem_wait_ld();
-      ld_half(tprev, 1, rh1);                   // in flight during the first half
-      gelu_half(rh0, bprev, 0);
-      sync_async();
-      if (tid == 0) ok = mma_chunks(tcur, 0);
-      tc::tmem_wait_ld();
-      gelu_half(rh1, bprev, 1);
-      sync_async();
-      if (tid == 0) {
-        if (ok) ok = mma_chunks(tcur, 2);
-        commit_mma();
-      }
-      if (!wait_mma()) break;
-    }
-    if (!ok) break;
-    // ---- epilogue of layer 3 (A), both halves, then the output layer
-    // (N = 16, K = 256) into B
-    {
-      uint32_t rh0[32], rh1[32];
-      ld_half(tA, 0, rh0);
-      tc::tmem_wait_ld();
-      ld_half(tA, 1, rh1);
-      gelu_half(rh0, sB + 512, 0);
-      tc::tmem_wait_ld();
-      gelu_half(rh1, sB + 512, 1);
-    }
-    sync_async();
-    if (tid == 0) {
+      for (int q = 0; q < 4; ++q)
+        x[q] = rw < a.n ? __ldg(reinterpret_cast<const float4 *>(a.x + rw * 16) + q) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    };
+    auto put = [&](int s) {
+      __nv_bfloat16 *sX = reinterpret_cast<__nv_bfloat16 *>(smem + FZ_OFF_X + 4096 * s);
 #pragma unroll
-      for (int j = 0; j < 16; ++j)
-        tc::mma_bf16(tB, tc::desc(aH + (uint32_t)(2 * j) * 128u, 128u, 4096u),
-                     tc::desc(aW4 + (uint32_t)(2 * j) * 128u, 128u, 4096u), id16, j > 0);
-      commit_mma();
+      for (int q = 0; q < 2; ++q)
+        *reinterpret_cast<uint4 *>(sX + tc::core_off(row, 8 * q, 16)) =
+            make_uint4(bf16x2_bits(x[2 * q].x, x[2 * q].y), bf16x2_bits(x[2 * q].z, x[2 * q].w),
+                       bf16x2_bits(x[2 * q + 1].x, x[2 * q + 1].y), bf16x2_bits(x[2 * q + 1].z, x[2 * q + 1].w));
+      warp_arrive(&bar_in[s]);
+    };
+    for (long t = 0; t < 2 && t < my_tiles; ++t) {
+      load(t);
+      put((int)t);
     }
-    if (!wait_mma()) break;
-    if (warp < 4) {                  // output columns 0..15: the first column quarter's warps
+    for (long t = 0; t < my_tiles && ok; ++t) {
+      const int s = (int)(t & 1);
+      if (t + 2 < my_tiles) load(t + 2);               // in flight while the tile is computed
+      ok = tc::mbar_wait(&bar_out[s], (uint32_t)((t >> 1) & 1), WAIT_ITERS);
+      if (!__all_sync(0xffffffffu, ok)) { ok = false; break; }
+      tc::fence_after();
       float v[16];
-      tc::tmem_ld16(tB + ((uint32_t)(warp * 32) << 16), v);
-      const long rw = r0 + tid;
+      tc::tmem_ld16(tmem + 256u * s + lanes, v);
+      const long rw = ((long)blockIdx.x + t * gridDim.x) * 128 + row;
       if (rw < a.n) {
 #pragma unroll
         for (int j = 0; j < 16; ++j)
           if (j < a.n_out) a.y[rw * a.n_out + j] = v[j] + sB[768 + j];
       }
+      if (t + 2 < my_tiles) put(s);
     }
-    tc::fence_before();
-    __syncthreads();
-    tc::fence_after();
-  }
-  if (!ok) {
-    if (tid == 0) atomicExch(a.err, 1);
-    // let the tensor core and the copies in flight finish before the
-    // shared memory and TMEM are released: one more commit covers every MMA
-    // issued so far; its phase is the parity of the commit count
-    if (tid == 0) {
-      if (uncommitted) commit_mma();
-      if (n_commit > 0) tc::mbar_wait(&bar_mma, (uint32_t)((n_commit - 1) & 1), WAIT_ITERS);
-      for (long g = consumed; g < issued; ++g)
-        tc::mbar_wait(&bar_full[g % FZ_NST], (uint32_t)((g / FZ_NST) & 1), WAIT_ITERS);
+  } else if (warp == FZ_MMA_WARP) {
+    if (lane == 0) {
+      const uint32_t id256 = tc::idesc_bf16_f32(128, 256), id16 = tc::idesc_bf16_f32(128, 16);
+      const uint32_t aW1 = tc::smem_u32(smem + FZ_OFF_W1), aW4 = tc::smem_u32(smem + FZ_OFF_W4);
+      uint32_t ph_act[2] = {0u, 0u};
+      long g = 0;                                      // weight chunks consumed
+      for (long t0 = 0; t0 < my_tiles && ok; t0 += 2)
+        for (int layer = 0; layer < 4 && ok; ++layer)
+          for (int s = 0; s < 2 && t0 + s < my_tiles && ok; ++s) {
+            const uint32_t acc = tmem + 256u * s, aH = tc::smem_u32(smem + FZ_OFF_H + 65536 * s);
+            if (layer == 0) {
+              ok = tc::mbar_wait(&bar_in[s], (uint32_t)((t0 >> 1) & 1), WAIT_ITERS);
+            } else {
+              ok = tc::mbar_wait(&bar_act[s], ph_act[s], WAIT_ITERS);
+              ph_act[s] ^= 1u;
+            }
+            if (!ok) break;
+            tc::fence_after();
+            if (layer == 0) {
+              tc::mma_bf16(acc, tc::desc(tc::smem_u32(smem + FZ_OFF_X + 4096 * s), 128u, 256u), tc::desc(aW1, 128u, 256u),
+                           id256, false);
+            } else if (layer < 3) {
+              for (int c = 0; c < FZ_CHUNKS; ++c, ++g) {
+                const int st = (int)(g % FZ_NST);
+                if (!(ok = tc::mbar_wait(&bar_full[st], (uint32_t)((g / FZ_NST) & 1), WAIT_ITERS))) break;
+                tc::fence_after();
+                const uint32_t aS = tc::smem_u32(smem + FZ_OFF_STAGE + st * FZ_CHUNK_BYTES);
+#pragma unroll
+                for (int j = 0; j < FZ_KC / 16; ++j)
+                  tc::mma_bf16(acc, tc::desc(aH + (uint32_t)(c * (FZ_KC / 8) + 2 * j) * 128u, 128u, 4096u),
+                               tc::desc(aS + (uint32_t)(2 * j) * 128u, 128u, (FZ_KC / 8) * 128u), id256, c > 0 || j > 0);
+                tc::commit(&bar_free[st]);
+              }
+              if (!ok) break;
+            } else {
+#pragma unroll
+              for (int j = 0; j < 16; ++j)
+                tc::mma_bf16(acc, tc::desc(aH + (uint32_t)(2 * j) * 128u, 128u, 4096u),
+                             tc::desc(aW4 + (uint32_t)(2 * j) * 128u, 128u, 4096u), id16, j > 0);
+            }
+            tc::commit(layer < 3 ? &bar_acc[s] : &bar_out[s]);
+          }
+      // every MMA issued is done before the shared memory and TMEM are released
+      tc::commit(&bar_end);
+      if (!tc::mbar_wait(&bar_end, 0u, WAIT_ITERS)) ok = false;
     }
+  } else if (lane == 0) {
+    // ---- weight chunks in the order of the MMAs: per pair of tiles W2 for
+    // slot 0, for slot 1, then W3 likewise
+    long g = 0;
+    auto copy = [&](const __nv_bfloat16 *w, int c) -> bool {
+      const int st = (int)(g % FZ_NST);
+      if (g >= FZ_NST && !tc::mbar_wait(&bar_free[st], (uint32_t)((g / FZ_NST - 1) & 1), WAIT_ITERS)) return false;
+      tc::mbar_expect_tx(&bar_full[st], FZ_CHUNK_BYTES);
+      tc::bulk_g2s(smem + FZ_OFF_STAGE + st * FZ_CHUNK_BYTES, w + (long)c * (256 * FZ_KC), FZ_CHUNK_BYTES, &bar_full[st]);
+      ++g;
+      return true;
+    };
+    for (long t0 = 0; t0 < my_tiles && ok; t0 += 2)
+      for (int layer = 0; layer < 2 && ok; ++layer)
+        for (int s = 0; s < 2 && t0 + s < my_tiles && ok; ++s)
+          for (int c = 0; c < FZ_CHUNKS && ok; ++c) ok = copy(layer == 0 ? a.w2 : a.w3, c);
+    // the copies in flight land before the shared memory is released
+    for (long i = g > FZ_NST ? g - FZ_NST : 0; i < g; ++i)
+      if (!tc::mbar_wait(&bar_full[i % FZ_NST], (uint32_t)((i / FZ_NST) & 1), WAIT_ITERS)) ok = false;
   }
+  if (!ok) failed = 1;
   tc::fence_before();
   __syncthreads();
+  if (tid == 0 && failed) atomicExch(a.err, 1);
   if (warp == 0) tc::tmem_dealloc(tmem, 512);
 }
 
 // FP32 master weights -> the fused kernel's BF16 layouts: W1 [256][16] and
 // the output layer [16][256] (rows >= n_out zero) as K-major core-matrix
-// tiles, W2 / W3 [256][256] as four K-chunks of 256 x 64 each.
+// tiles, W2 / W3 [256][256] as K-chunks of 256 x FZ_KC each.
 __global__ void mlp_pack_kernel(const float *__restrict__ p, long w1, long w2, long w3, long w4, int n_out,
                                 __nv_bfloat16 *__restrict__ out)
 {
@@ -531,7 +512,7 @@ __global__ void mlp_pack_kernel(const float *__restrict__ p, long w1, long w2, l
       const int l = (int)(j / 65536);
       const int n = (int)((j % 65536) / 256), k = (int)(j % 256);
       v = p[(l == 0 ? w2 : w3) + (long)n * 256 + k];
-      dst = 4096 + (long)l * 65536 + (long)(k / 64) * (256 * 64) + tc::core_off(n, k % 64, 64);
+      dst = 4096 + (long)l * 65536 + (long)(k / FZ_KC) * (256 * FZ_KC) + tc::core_off(n, k % FZ_KC, FZ_KC);
     } else {                                          // output layer: n < 16, k < 256
       const long j = i - 4096 - 131072;
       const int n = (int)(j / 256), k = (int)(j % 256);
