@@ -48,12 +48,12 @@
 //          series of (1 - eps)^(-1/2) to its quadratic term (remainder below
 //          2^-64), rounded once: within 0.51 ulp, no FP64 operation.
 //          fsqrt_rn: sqrt(d), the IEEE result bit for bit, from it.
-//   fatan  reduction to [0, 1] by atan(x) = pi/2 - atan(1/x), then
+//   fatan  reduction to y in (0, 1] by atan(x) = pi/2 - atan(1/x), then
 //          atan(y) = atan(c) + atan(r), c = j/64 the nearest table point,
-//          r = (y - c)/(1 + y c) (|r| <= 1/128; for y = 1/|x| numerator and
-//          denominator times |x|, so that one division serves), atan(r) by
-//          its Taylor series (r^3 in FP64, r^5 .. r^9 in FP32); atan(c) and
-//          pi/2 - atan(c) tabulated.  8 FP64 ops.
+//          r = (y - c)/(1 + y c) (|r| <= 1/128), atan(r) by its Taylor series
+//          to r^7; atan(c) and pi/2 - atan(c) tabulated; in 64-bit fixed point
+//          to 2^-60, rounded once, no FP64 operation.  Below 2^-7 the series
+//          in FP64.
 //
 // Accuracy: within 2 ulp (tests compare the host build of this code with
 // 200-bit mpmath values).  Every FP64 and FP32 operation is an explicit fma or
@@ -87,19 +87,17 @@
 
 namespace fm {
 
-struct AtanEntry { double hi; float lo; int pad; };
+struct alignas(16) AtanEntry { uint64_t at, co; };   // atan(j/64), pi/2 - atan(j/64), 2^-62
 struct alignas(16) LogEntry { uint32_t c, n0, n1, n2; };
 
 #if defined(__CUDA_ARCH__)
 __device__ const uint64_t kExpTable[512] = FM_EXP_TABLE_INIT;
 __device__ const LogEntry kLogTable[512] = FM_LOG_TABLE_INIT;
 __device__ const AtanEntry kAtanTable[65] = FM_ATAN_TABLE_INIT;
-__device__ const AtanEntry kAtanCTable[65] = FM_ATANC_TABLE_INIT;
-__device__ __forceinline__ void atan_entry(bool comp, int j, double &hi, float &lo)
+__device__ __forceinline__ AtanEntry atan_entry(uint32_t j)
 {
-  const double2 v = __ldg(reinterpret_cast<const double2 *>(comp ? kAtanCTable : kAtanTable) + j);
-  hi = v.x;
-  lo = __int_as_float((int)(uint32_t)__double_as_longlong(v.y));
+  const ulonglong2 v = __ldg(reinterpret_cast<const ulonglong2 *>(kAtanTable) + j);
+  return {v.x, v.y};
 }
 __device__ __forceinline__ float rcpf_(float x) { return __frcp_rn(x); }
 __device__ __forceinline__ float sqrtf_(float x) { return __fsqrt_rn(x); }
@@ -138,12 +136,7 @@ __device__ __forceinline__ float rcp_seed_(float x)
 static const uint64_t kExpTable[512] = FM_EXP_TABLE_INIT;
 static const LogEntry kLogTable[512] = FM_LOG_TABLE_INIT;
 static const AtanEntry kAtanTable[65] = FM_ATAN_TABLE_INIT;
-static const AtanEntry kAtanCTable[65] = FM_ATANC_TABLE_INIT;
-inline void atan_entry(bool comp, int j, double &hi, float &lo)
-{
-  const AtanEntry &e = comp ? kAtanCTable[j] : kAtanTable[j];
-  hi = e.hi; lo = e.lo;
-}
+inline AtanEntry atan_entry(uint32_t j) { return kAtanTable[j]; }
 inline float rcpf_(float x) { volatile float r = 1.0f / x; return r; }
 inline float sqrtf_(float x) { volatile float r = std::sqrt(x); return r; }
 inline uint64_t exp_entry(uint32_t j) { return kExpTable[j]; }
@@ -410,16 +403,16 @@ FM_NI Pair fexp2(double a, double b)
 // the IEEE division, out of line (the rare fallback of the paths below)
 FM_NI double div_ieee_(double a, double b) { return a / b; }
 
-// 1/x to within 2^-62 for x in [1, 2) as a fixed-point fraction, Y 2^-63;
-// mh : ml the 53-bit significand of x.
-FM_HD uint64_t rcp_fixed_(uint32_t mh, uint32_t ml)
+// 1/x to within 2^-62 for x = X 2^-60 in [1, 2) as a fixed-point fraction,
+// Y 2^-63.
+FM_HD uint64_t rcp_fixed60_(uint64_t X)
 {
-  const float xf = ffrom_bits_((int32_t)(0x3f800000u | ((mh & 0xfffffu) << 3) | (ml >> 29)));   // x truncated
+  const uint32_t xh = (uint32_t)(X >> 32), xl = (uint32_t)X;
+  const float xf = ffrom_bits_((int32_t)(0x3f800000u | ((uint32_t)(X >> 37) & 0x7fffffu)));   // x truncated
   // y0 2^24, below 2^24 (y0 = 1 is taken one unit lower)
   const uint32_t yb = (uint32_t)fbits_(rcp_seed_(xf));
   const uint32_t y0 = ((yb < 0x3f7fffffu ? yb : 0x3f7fffffu) & 0x7fffffu) | 0x800000u;
   // eps 2^84 = 2^84 - (x 2^60) (y0 2^24), modulo 2^64 (|eps| < 2^-21)
-  const uint32_t xl = ml << 8, xh = (mh << 8) | (ml >> 24);
   const uint64_t p = (uint64_t)xl * y0 + ((uint64_t)(xh * y0) << 32);
   const int64_t e = (int64_t)(0u - p);
   const int32_t eh = (int32_t)(e >> 32);
@@ -428,6 +421,8 @@ FM_HD uint64_t rcp_fixed_(uint32_t mh, uint32_t ml)
   const int64_t t = (int64_t)(int32_t)(w >> 32) * (int32_t)y0 + (int64_t)mulhi_((uint32_t)w, y0);   // y0 w 2^76
   return ((uint64_t)y0 << 39) + (uint64_t)(t >> 13);
 }
+// the same from x's 53-bit significand mh : ml
+FM_HD uint64_t rcp_fixed_(uint32_t mh, uint32_t ml) { return rcp_fixed60_((((uint64_t)mh << 32) | ml) << 8); }
 
 // The 53-bit quotient settled by its exact remainder r = a - q b (|r| far
 // below 2^63, so its low 64 bits tell it): q is the rounded quotient iff
@@ -564,34 +559,48 @@ FM_NI double fsqrt_rn(double d)
   return from_bits_((int64_t)(q + ((uint64_t)((k2 >> 1) + 511u) << 52)));
 }
 
+// atan x for |x| < 2^-7 (|x| >= 2^-30): the Taylor series, r^5 and beyond in FP32.
+FM_NI double atan_small_(double x)
+{
+  const double x2 = mul_(x, x);
+  const float f = to_f32(x2), s = fmaf_(f, fmaf_(f, 1.0f / 9.0f, -1.0f / 7.0f), 1.0f / 5.0f);
+  return fma_(mul_(x2, x), fma_(x2, to_f64(s), -1.0 / 3.0), x);
+}
+
 // Arc tangent (see the header).
 FM_NI double fatan(double x)
 {
-  const int64_t b = bits_(x), ab = b & 0x7fffffffffffffffLL;
-  if (ab < 0x3e10000000000000LL) return x;                        // |x| < 2^-30: atan x = x (1 - x^2/3), +-0
-  if (ab > 0x43b0000000000000LL) {                                // |x| > 2^60, inf, NaN
-    if (ab > 0x7ff0000000000000LL) return x;
-    return b < 0 ? -FM_PIO2 : FM_PIO2;
+  const uint32_t h = hi_(x), l = lo_(x), ah = h & 0x7fffffffu, e = ah >> 20;
+  if (e - 1016u >= 67u) {                                         // |x| < 2^-7 or >= 2^60, inf, NaN
+    if (ah >= 0x7ff00000u && x != x) return x;
+    if (e >= 1083u) return (int32_t)h < 0 ? -FM_PIO2 : FM_PIO2;
+    if (e < 993u) return x;                                       // |x| < 2^-30: atan x = x (1 - x^2/3), +-0
+    return atan_small_(x);
   }
-  const bool comp = ab > 0x3ff0000000000000LL;                    // |x| > 1: pi/2 - atan(1/|x|)
-  const double ax = from_bits_(ab);
-  const float xf = to_f32(ax);
-  const int32_t j = rint_f32(mulf_(comp ? rcpf_(xf) : xf, 64.0f));   // 0..64
-  const double c = j == 0 ? 0.0 : from_bits_(bits_(i2d(j)) - ((int64_t)6 << 52));   // j/64, exact
-  // r = (y - c) / (1 + y c), y = |x| or 1/|x| (then numerator and denominator times |x|)
-  const double num = comp ? fma_(-c, ax, 1.0) : add_(ax, -c);
-  const double r = fdiv_rn(num, comp ? add_(ax, c) : fma_(ax, c, 1.0));
-  const double r2 = mul_(r, r);
-  const float r2f = to_f32(r2);
-  // (atan r - r) / r^3 = -1/3 + r^2 (1/5 - r^2/7 + r^4/9)
-  const float s = fmaf_(r2f, fmaf_(r2f, 1.0f / 9.0f, -1.0f / 7.0f), 1.0f / 5.0f);
-  const double q = fma_(r2, to_f64(s), -1.0 / 3.0);
-  const double at = fma_(mul_(r2, r), q, r);
-  double hi;
-  float lo;
-  atan_entry(comp, j, hi, lo);
-  const double res = comp ? add_(hi, add_(to_f64(lo), -at)) : add_(hi, add_(to_f64(lo), at));
-  return b < 0 ? -res : res;
+  const uint32_t mh = (h & 0xfffffu) | 0x100000u;
+  const bool comp = e >= 1023u;                                   // |x| >= 1: pi/2 - atan(1/|x|)
+  // y = |x| or 1/|x| in (0, 1], 2^-63
+  const uint64_t y = comp ? rcp_fixed_(mh, l) >> (e - 1023u) : ((((uint64_t)mh << 32) | l) << 11) >> (1023u - e);
+  const uint32_t j = (uint32_t)((y + (1ull << 56)) >> 57);        // nearest multiple of 1/64
+  const uint64_t c = (uint64_t)j << 57;
+  // r = (y - c) / (1 + y c), |r| <= 2^-7: the magnitude 2^-69
+  const bool neg = y < c;
+  const uint64_t d = neg ? c - y : y - c;
+  const uint64_t den = (1ull << 60) + (mulhi64_(y, c) >> 2);      // [1, 2], 2^-60
+  const uint64_t q = rcp_fixed60_(den < (2ull << 60) ? den : (2ull << 60) - 1u);
+  const uint64_t r = mulhi64_(d << 7, q);
+  // atan r = r - r r^2 (1/3 - r^2/5 + r^4/7)
+  const uint64_t r2 = sqr70_(r << 1);                             // 2^-76
+  const uint32_t r46 = (uint32_t)(r2 >> 30);
+  const uint32_t v = 858993459u - mulhi_(r46 >> 14, 613566757u); // (1/5 - r^2/7) 2^32
+  const uint64_t w = 0x5555555555555555ull - (((uint64_t)r46 * v) >> 14);   // 2^-64
+  const uint64_t at = (r >> 7) - (mulhi64_(r << 1, mulhi64_(r2, w)) >> 20);   // 2^-62
+  const AtanEntry t = atan_entry(j);
+  const uint64_t res = (comp ? t.co : t.at) + ((comp != neg) ? 0u - at : at);   // (0, pi/2), 2^-62
+  const uint32_t lz = (uint32_t)clz32_((uint32_t)(res >> 32));
+  const uint64_t top = res << lz;
+  const uint64_t m = (top >> 11) + ((uint32_t)(top >> 10) & 1u);
+  return from_bits_((int64_t)(m + ((uint64_t)(1023u - lz) << 52) + ((uint64_t)(h & 0x80000000u) << 32)));
 }
 
 // x^a = e^(a log x) for x > 0 (relative error ~|a log x| ulp).

@@ -1033,142 +1033,73 @@
   {1026u, 0xa467ea69u, 0xb33b13a3u, 0xfffd063au}, \
 }
 
-// atan(j/64): {hi (double), lo (float)}, j = 0..64
+// {atan(j/64), pi/2 - atan(j/64)} 2^62, j = 0..64
 #define FM_ATAN_TABLE_INIT { \
-  {0x0.0p+0, 0.0f, 0}, \
-  {0x1.fff555bbb729bp-7, -0x1.220c3a0000000p-61f, 0}, \
-  {0x1.ffd55bba97625p-6, -0x1.5ec4320000000p-60f, 0}, \
-  {0x1.7fb818430da2ap-5, -0x1.86ef900000000p-63f, 0}, \
-  {0x1.ff55bb72cfdeap-5, -0x1.c934d80000000p-60f, 0}, \
-  {0x1.3f59f0e7c559dp-4, 0x1.ac4ce20000000p-58f, 0}, \
-  {0x1.7ee182602f10fp-4, -0x1.cfb6540000000p-58f, 0}, \
-  {0x1.be39ebe6f07c3p-4, 0x1.f7b8f20000000p-58f, 0}, \
-  {0x1.fd5ba9aac2f6ep-4, -0x1.cd37680000000p-59f, 0}, \
-  {0x1.1e1fafb043727p-3, -0x1.b485920000000p-59f, 0}, \
-  {0x1.3d6eee8c6626cp-3, 0x1.61a3b00000000p-57f, 0}, \
-  {0x1.5c9811e3ec26ap-3, -0x1.054ab20000000p-58f, 0}, \
-  {0x1.7b97b4bce5b02p-3, 0x1.347b0c0000000p-58f, 0}, \
-  {0x1.9a6a8e96c8626p-3, 0x1.cf601e0000000p-59f, 0}, \
-  {0x1.b90d7529260a2p-3, 0x1.17b10e0000000p-61f, 0}, \
-  {0x1.d77d5df205736p-3, 0x1.c648d20000000p-57f, 0}, \
-  {0x1.f5b75f92c80ddp-3, 0x1.8ab6e40000000p-57f, 0}, \
-  {0x1.09dc597d86362p-2, 0x1.62e4740000000p-56f, 0}, \
-  {0x1.18bf5a30bf178p-2, 0x1.30ca480000000p-57f, 0}, \
-  {0x1.278372057ef46p-2, -0x1.077cde0000000p-56f, 0}, \
-  {0x1.362773707ebccp-2, -0x1.963a540000000p-57f, 0}, \
-  {0x1.44aa436c2af0ap-2, -0x1.5d5e440000000p-56f, 0}, \
-  {0x1.530ad9951cd4ap-2, -0x1.2566480000000p-57f, 0}, \
-  {0x1.614840309cfe2p-2, -0x1.a725720000000p-56f, 0}, \
-  {0x1.6f61941e4def1p-2, -0x1.c63aae0000000p-56f, 0}, \
-  {0x1.7d5604b63b3f7p-2, 0x1.69c8860000000p-56f, 0}, \
-  {0x1.8b24d394a1b25p-2, 0x1.b6d0ba0000000p-56f, 0}, \
-  {0x1.98cd5454d6b18p-2, 0x1.9e6c980000000p-56f, 0}, \
-  {0x1.a64eec3cc23fdp-2, -0x1.24dec20000000p-56f, 0}, \
-  {0x1.b3a911da65c6cp-2, 0x1.ae187c0000000p-56f, 0}, \
-  {0x1.c0db4c94ec9f0p-2, -0x1.cc1ce80000000p-56f, 0}, \
-  {0x1.cde53432c1351p-2, -0x1.a2cfa40000000p-56f, 0}, \
-  {0x1.dac670561bb4fp-2, 0x1.a2b7f20000000p-56f, 0}, \
-  {0x1.e77eb7f175a34p-2, 0x1.0e53dc0000000p-56f, 0}, \
-  {0x1.f40dd0b541418p-2, -0x1.a3992e0000000p-57f, 0}, \
-  {0x1.0039c73c1a40cp-1, -0x1.b32c940000000p-55f, 0}, \
-  {0x1.0657e94db30d0p-1, -0x1.d5b4960000000p-56f, 0}, \
-  {0x1.0c6145b5b43dap-1, 0x1.974fa20000000p-58f, 0}, \
-  {0x1.1255d9bfbd2a9p-1, -0x1.2bdaee0000000p-58f, 0}, \
-  {0x1.1835a88be7c13p-1, 0x1.c621ce0000000p-55f, 0}, \
-  {0x1.1e00babdefeb4p-1, -0x1.928df20000000p-58f, 0}, \
-  {0x1.23b71e2cc9e6ap-1, 0x1.c421ca0000000p-57f, 0}, \
-  {0x1.2958e59308e31p-1, -0x1.09e73c0000000p-56f, 0}, \
-  {0x1.2ee628406cbcap-1, 0x1.c5d5ea0000000p-55f, 0}, \
-  {0x1.345f01cce37bbp-1, 0x1.1021140000000p-55f, 0}, \
-  {0x1.39c391cd4171ap-1, -0x1.2304340000000p-55f, 0}, \
-  {0x1.3f13fb89e96f4p-1, 0x1.ecf8b40000000p-56f, 0}, \
-  {0x1.445065b795b56p-1, -0x1.f76d020000000p-56f, 0}, \
-  {0x1.4978fa3269ee1p-1, 0x1.2419a80000000p-56f, 0}, \
-  {0x1.4e8de5bb6ec04p-1, 0x1.4a33dc0000000p-55f, 0}, \
-  {0x1.538f57b89061fp-1, -0x1.1bb74a0000000p-55f, 0}, \
-  {0x1.587d81f732fbbp-1, -0x1.5e5c9e0000000p-56f, 0}, \
-  {0x1.5d58987169b18p-1, 0x1.0028e40000000p-57f, 0}, \
-  {0x1.6220d115d7b8ep-1, -0x1.2b78540000000p-57f, 0}, \
-  {0x1.66d663923e087p-1, -0x1.6ea6fe0000000p-56f, 0}, \
-  {0x1.6b798920b3d99p-1, -0x1.a803860000000p-55f, 0}, \
-  {0x1.700a7c5784634p-1, -0x1.8c34d20000000p-56f, 0}, \
-  {0x1.748978fba8e0fp-1, 0x1.7b2a620000000p-59f, 0}, \
-  {0x1.78f6bbd5d315ep-1, 0x1.406a080000000p-55f, 0}, \
-  {0x1.7d528289fa093p-1, 0x1.5608220000000p-55f, 0}, \
-  {0x1.819d0b7158a4dp-1, -0x1.bf76220000000p-56f, 0}, \
-  {0x1.85d69576cc2c5p-1, 0x1.6b66e80000000p-57f, 0}, \
-  {0x1.89ff5ff57f1f8p-1, -0x1.55b9a60000000p-55f, 0}, \
-  {0x1.8e17aa99cc05ep-1, -0x1.ec182a0000000p-56f, 0}, \
-  {0x1.921fb54442d18p-1, 0x1.1a62640000000p-55f, 0}, \
-}
-
-// pi/2 - atan(j/64): {hi (double), lo (float)}, j = 0..64
-#define FM_ATANC_TABLE_INIT { \
-  {0x1.921fb54442d18p+0, 0x1.1a62640000000p-54f, 0}, \
-  {0x1.8e1fca98cb633p+0, 0x1.1299ee0000000p-56f, 0}, \
-  {0x1.8a205fd558740p+0, -0x1.30228c0000000p-54f, 0}, \
-  {0x1.8621f4822a647p+0, -0x1.26d1280000000p-57f, 0}, \
-  {0x1.82250768ac529p+0, -0x1.e78c960000000p-58f, 0}, \
-  {0x1.7e2a1635c67bep+0, 0x1.bf9d960000000p-54f, 0}, \
-  {0x1.7a319d1e3fe07p+0, 0x1.775dc80000000p-54f, 0}, \
-  {0x1.763c1685d3c9cp+0, 0x1.d736a00000000p-57f, 0}, \
-  {0x1.7249faa996a21p+0, 0x1.a8cc1e0000000p-54f, 0}, \
-  {0x1.6e5bbf4e3a633p+0, 0x1.a806900000000p-54f, 0}, \
-  {0x1.6a71d772b60cbp+0, -0x1.11d2120000000p-54f, 0}, \
-  {0x1.668cb307c54cbp+0, 0x1.55b8720000000p-57f, 0}, \
-  {0x1.62acbeaca61b8p+0, 0x1.c6aca00000000p-60f, 0}, \
-  {0x1.5ed2637169c54p+0, -0x1.f4189e0000000p-54f, 0}, \
-  {0x1.5afe069f1e104p+0, 0x1.8330120000000p-58f, 0}, \
-  {0x1.5730098602231p+0, 0x1.e1994a0000000p-54f, 0}, \
-  {0x1.5368c951e9cfdp+0, -0x1.96f47a0000000p-54f, 0}, \
-  {0x1.4fa89ee4e1440p+0, -0x1.3e56ba0000000p-54f, 0}, \
-  {0x1.4befdeb8130bap+0, 0x1.e892340000000p-55f, 0}, \
-  {0x1.483ed8c2e3147p+0, -0x1.477ccc0000000p-55f, 0}, \
-  {0x1.4495d86823225p+0, 0x1.4d29ae0000000p-54f, 0}, \
-  {0x1.40f5246938156p+0, -0x1.1c8c180000000p-55f, 0}, \
-  {0x1.3d5cfedefb9c6p+0, -0x1.81e1a80000000p-55f, 0}, \
-  {0x1.39cda5381b920p+0, -0x1.ef51020000000p-56f, 0}, \
-  {0x1.3647503caf55cp+0, 0x1.17e21e0000000p-55f, 0}, \
-  {0x1.32ca3416b401ap+0, 0x1.bff0420000000p-54f, 0}, \
-  {0x1.2f56805f1a64fp+0, -0x1.4d472e0000000p-56f, 0}, \
-  {0x1.2bec602f0d252p+0, 0x1.658e7a0000000p-55f, 0}, \
-  {0x1.288bfa3512419p+0, 0x1.8e684e0000000p-56f, 0}, \
-  {0x1.253570cda95fdp+0, 0x1.5db8880000000p-55f, 0}, \
-  {0x1.21e8e21f07a9cp+0, 0x1.8d699c0000000p-54f, 0}, \
-  {0x1.1ea6683792844p+0, 0x1.062c980000000p-55f, 0}, \
-  {0x1.1b6e192ebbe44p+0, 0x1.b1b4660000000p-54f, 0}, \
-  {0x1.18400747e568bp+0, 0x1.ad9ad80000000p-55f, 0}, \
-  {0x1.151c4116f2812p+0, 0x1.4ed5880000000p-54f, 0}, \
-  {0x1.1202d1a635b12p+0, 0x1.f3f8ae0000000p-54f, 0}, \
-  {0x1.0ef3c09d694b0p+0, 0x1.8fcf880000000p-54f, 0}, \
-  {0x1.0bef126968b2bp+0, 0x1.00ed6a0000000p-54f, 0}, \
-  {0x1.08f4c864643c4p+0, -0x1.a5bfdc0000000p-55f, 0}, \
-  {0x1.0604e0fe4ef0fp+0, -0x1.c8ae840000000p-54f, 0}, \
-  {0x1.031f57e54adbep+0, 0x1.338b420000000p-54f, 0}, \
-  {0x1.0044262dddde3p+0, 0x1.c3bc540000000p-55f, 0}, \
-  {0x1.fae684f57cc00p-1, -0x1.46479c0000000p-55f, 0}, \
-  {0x1.f559424818e66p-1, 0x1.bbbb720000000p-57f, 0}, \
-  {0x1.efe068bba2275p-1, 0x1.24a3b20000000p-55f, 0}, \
-  {0x1.ea7bd8bb44317p-1, -0x1.506e0c0000000p-56f, 0}, \
-  {0x1.e52b6efe9c33cp-1, 0x1.3e486c0000000p-55f, 0}, \
-  {0x1.dfef04d0efedbp-1, -0x1.9f09720000000p-56f, 0}, \
-  {0x1.dac670561bb4fp-1, 0x1.a2b7f20000000p-55f, 0}, \
-  {0x1.d5b184cd16e2cp-1, 0x1.d521d40000000p-56f, 0}, \
-  {0x1.d0b012cff5412p-1, -0x1.5f07de0000000p-56f, 0}, \
-  {0x1.cbc1e89152a76p-1, -0x1.1c0cea0000000p-55f, 0}, \
-  {0x1.c6e6d2171bf18p-1, 0x1.f4ba8e0000000p-55f, 0}, \
-  {0x1.c21e9972adea3p-1, -0x1.805d240000000p-55f, 0}, \
-  {0x1.bd6906f6479aap-1, -0x1.13e7ba0000000p-55f, 0}, \
-  {0x1.b8c5e167d1c98p-1, -0x1.19bd9c0000000p-58f, 0}, \
-  {0x1.b434ee31013fdp-1, -0x1.0520d00000000p-55f, 0}, \
-  {0x1.afb5f18cdcc22p-1, -0x1.e2ede00000000p-55f, 0}, \
-  {0x1.ab48aeb2b28d2p-1, 0x1.e8b57c0000000p-56f, 0}, \
-  {0x1.a6ece7fe8b99dp-1, 0x1.bd79480000000p-56f, 0}, \
-  {0x1.a2a25f172cfe4p-1, -0x1.d700500000000p-56f, 0}, \
-  {0x1.9e68d511b976bp-1, 0x1.d9eb0c0000000p-55f, 0}, \
-  {0x1.9a400a9306839p-1, -0x1.d6064e0000000p-57f, 0}, \
-  {0x1.9627bfeeb99d3p-1, -0x1.aa5e480000000p-56f, 0}, \
-  {0x1.921fb54442d18p-1, 0x1.1a62640000000p-55f, 0}, \
+  {0x0000000000000000ull, 0x6487ed5110b4611aull}, \
+  {0x00fffaaadddb94d6ull, 0x6387f2a632d8cc45ull}, \
+  {0x01ffd55bba97624bull, 0x628817f5561cfed0ull}, \
+  {0x02ff7030861b453full, 0x61887d208a991bdbull}, \
+  {0x03feab76e59fbd39ull, 0x608941da2b14a3e2ull}, \
+  {0x04fd67c39f15675bull, 0x5f8a858d719ef9c0ull}, \
+  {0x05fb860980bc43a3ull, 0x5e8c67478ff81d77ull}, \
+  {0x06f8e7af9bc1f0dfull, 0x5d8f05a174f2703bull}, \
+  {0x07f56ea6ab0bdb72ull, 0x5c927eaa65a885a9ull}, \
+  {0x08f0fd7d821b9372ull, 0x5b96efd38e98cda8ull}, \
+  {0x09eb77746331362cull, 0x5a9c75dcad832aeeull}, \
+  {0x0ae4c08f1f6134f0ull, 0x59a32cc1f1532c2bull}, \
+  {0x0bdcbda5e72d8113ull, 0x58ab2fab2986e007ull}, \
+  {0x0cd35474b643130eull, 0x57b498dc5a714e0cull}, \
+  {0x0dc86ba949305102ull, 0x56bf81a7c7841018ull}, \
+  {0x0ebbeaef902b9b39ull, 0x55cc02618088c5e2ull}, \
+  {0x0fadbafc96406eb1ull, 0x54da32547a73f269ull}, \
+  {0x109dc597d8636259ull, 0x53ea27b93850fec2ull}, \
+  {0x118bf5a30bf17826ull, 0x52fbf7ae04c2e8f4ull}, \
+  {0x1278372057ef45beull, 0x520fb630b8c51b5cull}, \
+  {0x1362773707ebcbcdull, 0x5125761a08c8954dull}, \
+  {0x144aa436c2af09a9ull, 0x503d491a4e055772ull}, \
+  {0x1530ad9951cd49dbull, 0x4f573fb7bee7173full}, \
+  {0x1614840309cfe196ull, 0x4e73694e06e47f84ull}, \
+  {0x16f61941e4def08eull, 0x4d91d40f2bd5708cull}, \
+  {0x17d5604b63b3f75aull, 0x4cb28d05ad0069c0ull}, \
+  {0x18b24d394a1b256eull, 0x4bd5a017c6993badull}, \
+  {0x198cd5454d6b1868ull, 0x4afb180bc34948b3ull}, \
+  {0x1a64eec3cc23fcb7ull, 0x4a22fe8d44906464ull}, \
+  {0x1b3a911da65c6c6cull, 0x494d5c336a57f4afull}, \
+  {0x1c0db4c94ec9ef8dull, 0x487a3887c1ea718dull}, \
+  {0x1cde53432c135097ull, 0x47a99a0de4a11083ull}, \
+  {0x1dac670561bb4f69ull, 0x46db864baef911b2ull}, \
+  {0x1e77eb7f175a3444ull, 0x461001d1f95a2cd7ull}, \
+  {0x1f40dd0b541417ccull, 0x45471045bca0494full}, \
+  {0x200738e783481726ull, 0x4480b4698d6c49f4ull}, \
+  {0x20cafd29b6619f8bull, 0x43bcf0275a52c190ull}, \
+  {0x218c28b6b687b419ull, 0x42fbc49a5a2cad01ull}, \
+  {0x224abb37f7a551edull, 0x423d3219190f0f2dull}, \
+  {0x2306b5117cf826e3ull, 0x4181383f93bc3a37ull}, \
+  {0x23c01757bdfd67e7ull, 0x40c7d5f952b6f934ull}, \
+  {0x2476e3c5993cd439ull, 0x4011098b77778ce2ull}, \
+  {0x252b1cb2611c61beull, 0x3f5cd09eaf97ff5dull}, \
+  {0x25dcc5080d9794e3ull, 0x3eab2849031ccc37ull}, \
+  {0x268be0399c6f7688ull, 0x3dfc0d177444ea92ull}, \
+  {0x27387239a82e336eull, 0x3d4f7b1768862dacull}, \
+  {0x27e27f713d2de87bull, 0x3ca56ddfd386789full}, \
+  {0x288a0cb6f2b6ab82ull, 0x3bfde09a1dfdb598ull}, \
+  {0x292f1f464d3dc249ull, 0x3b58ce0ac3769ed1ull}, \
+  {0x29d1bcb76dd808a5ull, 0x3ab63099a2dc5875ull}, \
+  {0x2a71eaf7120c3d72ull, 0x3a160259fea823a8ull}, \
+  {0x2b0fb03ee65f75a8ull, 0x39783d122a54eb72ull}, \
+  {0x2bab130e2d363020ull, 0x38dcda42e37e30faull}, \
+  {0x2c441a22baf71bdbull, 0x3843d32e55bd4540ull}, \
+  {0x2cdacc7247c10da4ull, 0x37ad20dec8f35376ull}, \
+  {0x2d6f3124167b312cull, 0x3718bc2cfa392feeull}, \
+  {0x2e014f8af08c679dull, 0x36869dc62027f97dull}, \
+  {0x2e912f1f751c1e0cull, 0x35f6be319b98430full}, \
+  {0x2f1ed77aba62bca0ull, 0x356915d65651a47aull}, \
+  {0x2faa50513f4126abull, 0x34dd9cffd1733a6full}, \
+  {0x3033a16e2b149990ull, 0x34544be2e59fc78aull}, \
+  {0x30bad2aed9858a2dull, 0x33cd1aa2372ed6edull}, \
+  {0x313febfeafe3ef55ull, 0x3348015260d071c5ull}, \
+  {0x31c2f5533980bb85ull, 0x32c4f7fdd733a595ull}, \
+  {0x3243f6a8885a308dull, 0x3243f6a8885a308dull}, \
 }
 
 #define FM_INV_L512_F 0x1.7154760000000p+9f

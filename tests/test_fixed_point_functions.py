@@ -1,9 +1,10 @@
-"""The fixed-point exp / exp10 / log of fastmath.cuh (host build of the
+"""The fixed-point exp / exp10 / log / atan of fastmath.cuh (host build of the
 kernels' source) where they can go wrong: at the edges of the reduction and of
 the table intervals, next to x = 1, in the last normal binades and across the
 gradual underflow, against 200-bit mpmath values.  The fixed-point error is
 below 2^-58 of the result, so the rounded results are within 0.55 ulp (1 ulp
-where the result is subnormal or the FP64 form next to x = 1 is used)."""
+where the result is subnormal or an FP64 form is used: log next to x = 1, atan
+below 2^-7)."""
 import ctypes
 import os
 import subprocess
@@ -67,12 +68,18 @@ CASES = {
     "log-at-one": (2, np.concatenate([1 + s * 2.0 ** RNG.uniform(-52, -8.001, 300) for s in (1, -1)]), 1.0),
     "log-binades": (2, 2.0 ** RNG.uniform(-1022, 1023.9, 500), 0.55),
     "log-subnormal": (2, 2.0 ** RNG.uniform(-1073, -1022, 200), 0.55),
+    "atan-table-steps": (4, around(np.concatenate([np.arange(1, 65) / 64, (np.arange(1, 65) - 0.5) / 64])), 0.55),
+    "atan-reciprocal-steps": (4, around(64 / np.concatenate([np.arange(1, 65), np.arange(1, 65) - 0.5])), 0.55),
+    "atan-at-one": (4, around([1.0, -1.0], 4), 0.55),
+    "atan-small-end": (4, around([2.0 ** -7, -2.0 ** -7], 4), 1.0),
+    "atan-range": (4, np.concatenate([s * 2.0 ** RNG.uniform(-6.9, 59.9, 400) for s in (1, -1)]), 0.55),
+    "atan-small": (4, np.concatenate([s * 2.0 ** RNG.uniform(-40, -7, 300) for s in (1, -1)]), 1.0),
 }
 
 
 @pytest.mark.parametrize("name", list(CASES))
 def test_within_bound(ev, name):
     fn, xs, bound = CASES[name]
-    exact = (mp.exp, lambda v: mp.power(10, v), mp.log)[fn]
+    exact = (mp.exp, lambda v: mp.power(10, v), mp.log, None, mp.atan)[fn]
     xs = xs[xs != 1.0] if fn == 2 else xs
     assert worst_ulp(ev(fn, xs), exact, xs) <= bound
