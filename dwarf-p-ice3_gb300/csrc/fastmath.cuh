@@ -51,9 +51,11 @@
 //   fatan  reduction to y in (0, 1] by atan(x) = pi/2 - atan(1/x), then
 //          atan(y) = atan(c) + atan(r), c = j/64 the nearest table point,
 //          r = (y - c)/(1 + y c) (|r| <= 1/128), atan(r) by its Taylor series
-//          to r^7; atan(c) and pi/2 - atan(c) tabulated; in 64-bit fixed point
-//          to 2^-60, rounded once, no FP64 operation.  Below 2^-7 the series
-//          in FP64.
+//          to r^7; atan(c) and pi/2 - atan(c) tabulated; in 64-bit fixed
+//          point, units of 2^-64 where the result is below 1 (table and shift
+//          each rounded to 2^-65, r within 2^-66: below 0.04 ulp of the
+//          smallest result, 2^-7) and 2^-62 above; rounded once, no FP64
+//          operation.  Below 2^-7 the series in FP64.
 //
 // Accuracy: within 2 ulp (tests compare the host build of this code with
 // 200-bit mpmath values).  Every FP64 and FP32 operation is an explicit fma or
@@ -87,7 +89,7 @@
 
 namespace fm {
 
-struct alignas(16) AtanEntry { uint64_t at, co; };   // atan(j/64), pi/2 - atan(j/64), 2^-62
+struct alignas(16) AtanEntry { uint64_t at, co; };   // atan(j/64), 2^-64; pi/2 - atan(j/64), 2^-62
 struct alignas(16) LogEntry { uint32_t c, n0, n1, n2; };
 
 #if defined(__CUDA_ARCH__)
@@ -594,13 +596,14 @@ FM_NI double fatan(double x)
   const uint32_t r46 = (uint32_t)(r2 >> 30);
   const uint32_t v = 858993459u - mulhi_(r46 >> 14, 613566757u); // (1/5 - r^2/7) 2^32
   const uint64_t w = 0x5555555555555555ull - (((uint64_t)r46 * v) >> 14);   // 2^-64
-  const uint64_t at = (r >> 7) - (mulhi64_(r << 1, mulhi64_(r2, w)) >> 20);   // 2^-62
+  const uint64_t ar = r - (mulhi64_(r << 1, mulhi64_(r2, w)) >> 13);        // 2^-69
+  const uint64_t at = comp ? (ar + 64u) >> 7 : (ar + 16u) >> 5;   // 2^-62, 2^-64
   const AtanEntry t = atan_entry(j);
-  const uint64_t res = (comp ? t.co : t.at) + ((comp != neg) ? 0u - at : at);   // (0, pi/2), 2^-62
+  const uint64_t res = (comp ? t.co : t.at) + ((comp != neg) ? 0u - at : at);   // (0, pi/2), 2^-62; (0, 1), 2^-64
   const uint32_t lz = (uint32_t)clz32_((uint32_t)(res >> 32));
   const uint64_t top = res << lz;
   const uint64_t m = (top >> 11) + ((uint32_t)(top >> 10) & 1u);
-  return from_bits_((int64_t)(m + ((uint64_t)(1023u - lz) << 52) + ((uint64_t)(h & 0x80000000u) << 32)));
+  return from_bits_((int64_t)(m + ((uint64_t)((comp ? 1023u : 1021u) - lz) << 52) + ((uint64_t)(h & 0x80000000u) << 32)));
 }
 
 // x^a = e^(a log x) for x > 0 (relative error ~|a log x| ulp).

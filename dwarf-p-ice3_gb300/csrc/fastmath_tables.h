@@ -1033,73 +1033,73 @@
   {1026u, 0xa467ea69u, 0xb33b13a3u, 0xfffd063au}, \
 }
 
-// {atan(j/64), pi/2 - atan(j/64)} 2^62, j = 0..64
+// {atan(j/64) 2^64, (pi/2 - atan(j/64)) 2^62}, j = 0..64
 #define FM_ATAN_TABLE_INIT { \
   {0x0000000000000000ull, 0x6487ed5110b4611aull}, \
-  {0x00fffaaadddb94d6ull, 0x6387f2a632d8cc45ull}, \
-  {0x01ffd55bba97624bull, 0x628817f5561cfed0ull}, \
-  {0x02ff7030861b453full, 0x61887d208a991bdbull}, \
-  {0x03feab76e59fbd39ull, 0x608941da2b14a3e2ull}, \
-  {0x04fd67c39f15675bull, 0x5f8a858d719ef9c0ull}, \
-  {0x05fb860980bc43a3ull, 0x5e8c67478ff81d77ull}, \
-  {0x06f8e7af9bc1f0dfull, 0x5d8f05a174f2703bull}, \
-  {0x07f56ea6ab0bdb72ull, 0x5c927eaa65a885a9ull}, \
-  {0x08f0fd7d821b9372ull, 0x5b96efd38e98cda8ull}, \
-  {0x09eb77746331362cull, 0x5a9c75dcad832aeeull}, \
-  {0x0ae4c08f1f6134f0ull, 0x59a32cc1f1532c2bull}, \
-  {0x0bdcbda5e72d8113ull, 0x58ab2fab2986e007ull}, \
-  {0x0cd35474b643130eull, 0x57b498dc5a714e0cull}, \
-  {0x0dc86ba949305102ull, 0x56bf81a7c7841018ull}, \
-  {0x0ebbeaef902b9b39ull, 0x55cc02618088c5e2ull}, \
-  {0x0fadbafc96406eb1ull, 0x54da32547a73f269ull}, \
-  {0x109dc597d8636259ull, 0x53ea27b93850fec2ull}, \
-  {0x118bf5a30bf17826ull, 0x52fbf7ae04c2e8f4ull}, \
-  {0x1278372057ef45beull, 0x520fb630b8c51b5cull}, \
-  {0x1362773707ebcbcdull, 0x5125761a08c8954dull}, \
-  {0x144aa436c2af09a9ull, 0x503d491a4e055772ull}, \
-  {0x1530ad9951cd49dbull, 0x4f573fb7bee7173full}, \
-  {0x1614840309cfe196ull, 0x4e73694e06e47f84ull}, \
-  {0x16f61941e4def08eull, 0x4d91d40f2bd5708cull}, \
-  {0x17d5604b63b3f75aull, 0x4cb28d05ad0069c0ull}, \
-  {0x18b24d394a1b256eull, 0x4bd5a017c6993badull}, \
-  {0x198cd5454d6b1868ull, 0x4afb180bc34948b3ull}, \
-  {0x1a64eec3cc23fcb7ull, 0x4a22fe8d44906464ull}, \
-  {0x1b3a911da65c6c6cull, 0x494d5c336a57f4afull}, \
-  {0x1c0db4c94ec9ef8dull, 0x487a3887c1ea718dull}, \
-  {0x1cde53432c135097ull, 0x47a99a0de4a11083ull}, \
-  {0x1dac670561bb4f69ull, 0x46db864baef911b2ull}, \
-  {0x1e77eb7f175a3444ull, 0x461001d1f95a2cd7ull}, \
-  {0x1f40dd0b541417ccull, 0x45471045bca0494full}, \
-  {0x200738e783481726ull, 0x4480b4698d6c49f4ull}, \
-  {0x20cafd29b6619f8bull, 0x43bcf0275a52c190ull}, \
-  {0x218c28b6b687b419ull, 0x42fbc49a5a2cad01ull}, \
-  {0x224abb37f7a551edull, 0x423d3219190f0f2dull}, \
-  {0x2306b5117cf826e3ull, 0x4181383f93bc3a37ull}, \
-  {0x23c01757bdfd67e7ull, 0x40c7d5f952b6f934ull}, \
-  {0x2476e3c5993cd439ull, 0x4011098b77778ce2ull}, \
-  {0x252b1cb2611c61beull, 0x3f5cd09eaf97ff5dull}, \
-  {0x25dcc5080d9794e3ull, 0x3eab2849031ccc37ull}, \
-  {0x268be0399c6f7688ull, 0x3dfc0d177444ea92ull}, \
-  {0x27387239a82e336eull, 0x3d4f7b1768862dacull}, \
-  {0x27e27f713d2de87bull, 0x3ca56ddfd386789full}, \
-  {0x288a0cb6f2b6ab82ull, 0x3bfde09a1dfdb598ull}, \
-  {0x292f1f464d3dc249ull, 0x3b58ce0ac3769ed1ull}, \
-  {0x29d1bcb76dd808a5ull, 0x3ab63099a2dc5875ull}, \
-  {0x2a71eaf7120c3d72ull, 0x3a160259fea823a8ull}, \
-  {0x2b0fb03ee65f75a8ull, 0x39783d122a54eb72ull}, \
-  {0x2bab130e2d363020ull, 0x38dcda42e37e30faull}, \
-  {0x2c441a22baf71bdbull, 0x3843d32e55bd4540ull}, \
-  {0x2cdacc7247c10da4ull, 0x37ad20dec8f35376ull}, \
-  {0x2d6f3124167b312cull, 0x3718bc2cfa392feeull}, \
-  {0x2e014f8af08c679dull, 0x36869dc62027f97dull}, \
-  {0x2e912f1f751c1e0cull, 0x35f6be319b98430full}, \
-  {0x2f1ed77aba62bca0ull, 0x356915d65651a47aull}, \
-  {0x2faa50513f4126abull, 0x34dd9cffd1733a6full}, \
-  {0x3033a16e2b149990ull, 0x34544be2e59fc78aull}, \
-  {0x30bad2aed9858a2dull, 0x33cd1aa2372ed6edull}, \
-  {0x313febfeafe3ef55ull, 0x3348015260d071c5ull}, \
-  {0x31c2f5533980bb85ull, 0x32c4f7fdd733a595ull}, \
-  {0x3243f6a8885a308dull, 0x3243f6a8885a308dull}, \
+  {0x03ffeaab776e5357ull, 0x6387f2a632d8cc45ull}, \
+  {0x07ff556eea5d892aull, 0x628817f5561cfed0ull}, \
+  {0x0bfdc0c2186d14fdull, 0x61887d208a991bdbull}, \
+  {0x0ffaaddb967ef4e3ull, 0x608941da2b14a3e2ull}, \
+  {0x13f59f0e7c559d6bull, 0x5f8a858d719ef9c0ull}, \
+  {0x17ee182602f10e8cull, 0x5e8c67478ff81d77ull}, \
+  {0x1be39ebe6f07c37eull, 0x5d8f05a174f2703bull}, \
+  {0x1fd5ba9aac2f6dc6ull, 0x5c927eaa65a885a9ull}, \
+  {0x23c3f5f6086e4dc9ull, 0x5b96efd38e98cda8ull}, \
+  {0x27adddd18cc4d8b1ull, 0x5a9c75dcad832aeeull}, \
+  {0x2b93023c7d84d3bfull, 0x59a32cc1f1532c2bull}, \
+  {0x2f72f6979cb6044dull, 0x58ab2fab2986e007ull}, \
+  {0x334d51d2d90c4c3aull, 0x57b498dc5a714e0cull}, \
+  {0x3721aea524c14409ull, 0x56bf81a7c7841018ull}, \
+  {0x3aefabbe40ae6ce3ull, 0x55cc02618088c5e2ull}, \
+  {0x3eb6ebf25901bac5ull, 0x54da32547a73f269ull}, \
+  {0x4277165f618d8963ull, 0x53ea27b93850fec2ull}, \
+  {0x462fd68c2fc5e098ull, 0x52fbf7ae04c2e8f4ull}, \
+  {0x49e0dc815fbd16f9ull, 0x520fb630b8c51b5cull}, \
+  {0x4d89dcdc1faf2f35ull, 0x5125761a08c8954dull}, \
+  {0x512a90db0abc26a3ull, 0x503d491a4e055772ull}, \
+  {0x54c2b6654735276dull, 0x4f573fb7bee7173full}, \
+  {0x5852100c273f8659ull, 0x4e73694e06e47f84ull}, \
+  {0x5bd86507937bc23aull, 0x4d91d40f2bd5708cull}, \
+  {0x5f55812d8ecfdd6aull, 0x4cb28d05ad0069c0ull}, \
+  {0x62c934e5286c95b7ull, 0x4bd5a017c6993badull}, \
+  {0x6633551535ac619eull, 0x4afb180bc34948b3ull}, \
+  {0x6993bb0f308ff2dbull, 0x4a22fe8d44906464ull}, \
+  {0x6cea44769971b1aeull, 0x494d5c336a57f4afull}, \
+  {0x7036d3253b27be34ull, 0x487a3887c1ea718dull}, \
+  {0x73794d0cb04d425dull, 0x47a99a0de4a11083ull}, \
+  {0x76b19c1586ed3da3ull, 0x46db864baef911b2ull}, \
+  {0x79dfadfc5d68d10eull, 0x461001d1f95a2cd7ull}, \
+  {0x7d03742d50505f2eull, 0x45471045bca0494full}, \
+  {0x801ce39e0d205c9aull, 0x4480b4698d6c49f4ull}, \
+  {0x832bf4a6d9867e2aull, 0x43bcf0275a52c190ull}, \
+  {0x8630a2dada1ed066ull, 0x42fbc49a5a2cad01ull}, \
+  {0x892aecdfde9547b5ull, 0x423d3219190f0f2dull}, \
+  {0x8c1ad445f3e09b8cull, 0x4181383f93bc3a37ull}, \
+  {0x8f005d5ef7f59f9bull, 0x40c7d5f952b6f934ull}, \
+  {0x91db8f1664f350e2ull, 0x4011098b77778ce2ull}, \
+  {0x94ac72c9847186f6ull, 0x3f5cd09eaf97ff5dull}, \
+  {0x97731420365e538cull, 0x3eab2849031ccc37ull}, \
+  {0x9a2f80e671bdda20ull, 0x3dfc0d177444ea92ull}, \
+  {0x9ce1c8e6a0b8cdbaull, 0x3d4f7b1768862dacull}, \
+  {0x9f89fdc4f4b7a1edull, 0x3ca56ddfd386789full}, \
+  {0xa22832dbcadaae09ull, 0x3bfde09a1dfdb598ull}, \
+  {0xa4bc7d1934f70924ull, 0x3b58ce0ac3769ed1ull}, \
+  {0xa746f2ddb7602294ull, 0x3ab63099a2dc5875ull}, \
+  {0xa9c7abdc4830f5c9ull, 0x3a160259fea823a8ull}, \
+  {0xac3ec0fb997dd6a2ull, 0x39783d122a54eb72ull}, \
+  {0xaeac4c38b4d8c080ull, 0x38dcda42e37e30faull}, \
+  {0xb110688aebdc6f6aull, 0x3843d32e55bd4540ull}, \
+  {0xb36b31c91f043691ull, 0x37ad20dec8f35376ull}, \
+  {0xb5bcc49059ecc4b0ull, 0x3718bc2cfa392feeull}, \
+  {0xb8053e2bc2319e74ull, 0x36869dc62027f97dull}, \
+  {0xba44bc7dd470782full, 0x35f6be319b98430full}, \
+  {0xbc7b5deae98af281ull, 0x356915d65651a47aull}, \
+  {0xbea94144fd049aacull, 0x34dd9cffd1733a6full}, \
+  {0xc0ce85b8ac526641ull, 0x34544be2e59fc78aull}, \
+  {0xc2eb4abb661628b6ull, 0x33cd1aa2372ed6edull}, \
+  {0xc4ffaffabf8fbd55ull, 0x3348015260d071c5ull}, \
+  {0xc70bd54ce602ee14ull, 0x32c4f7fdd733a595ull}, \
+  {0xc90fdaa22168c235ull, 0x3243f6a8885a308dull}, \
 }
 
 #define FM_INV_L512_F 0x1.7154760000000p+9f

@@ -10,7 +10,7 @@ times 2^-70 and 32 further bits, and 2^20 times each modulo 2^-6 (the bias
 that keeps the multiple positive).
 
 atan (table-driven reduction in the manner of Tang's methods): atan(j/64) and
-pi/2 - atan(j/64), j = 0..64, as 64-bit integers times 2^-62.
+pi/2 - atan(j/64), j = 0..64, as 64-bit integers times 2^-64 and 2^-62.
 
 log (after Tang, ACM TOMS 16(4), 1990, in fixed point): the significand z in
 [1, 2) is split into 512 intervals by its 9 leading fraction bits; per
@@ -67,11 +67,11 @@ def main() -> None:
         w = words(fix(-mp.log(mp.mpf(c) / 2048) - 1100 * mp.log(2), 72), 3)
         lines.append(f"  {{{c}u, {w[0]:#010x}u, {w[1]:#010x}u, {w[2]:#010x}u}}, \\")
     lines += ["}", "",
-              "// {atan(j/64), pi/2 - atan(j/64)} 2^62, j = 0..64",
+              "// {atan(j/64) 2^64, (pi/2 - atan(j/64)) 2^62}, j = 0..64",
               "#define FM_ATAN_TABLE_INIT { \\"]
     for j in range(65):
         t = mp.atan(mp.mpf(j) / 64)
-        lines.append(f"  {{{fix(t, 62):#018x}ull, {fix(mp.pi / 2 - t, 62):#018x}ull}}, \\")
+        lines.append(f"  {{{fix(t, 64):#018x}ull, {fix(mp.pi / 2 - t, 62):#018x}ull}}, \\")
     lines += ["}", ""]
     l512 = mp.log(2) / 512
     lg512 = mp.log10(2) / 512
