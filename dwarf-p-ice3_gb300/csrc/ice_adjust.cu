@@ -17,11 +17,13 @@ using namespace ice3ia;
 // physics step) instead of th/rv/.../rg, which are then not read; rrs/rss/rgs
 // are read instead.  Output pointers may be NULL in the internal chained use
 // (store skipped).
-// Bound: the FP64 pipe (about 115 operations per point; 1.4 TB/s of HBM).
-// 126 registers, two blocks per SM; two points per thread with 128-bit
-// accesses (152 registers, one block) took 22.45 against 19.26 ms per launch
-// at 1024x1024x90, and with the registers capped for two / three / four
-// blocks either form stays within 19.2-19.5 ms.
+// Bound: the FP64 pipe.  At 1024x1024x90 a launch takes 15.4 ms (1.7 TB/s of
+// HBM); 16.8 ms before the ice fraction was decided on the high words, the
+// products of sbar shared and sigma formed only where there is a condensate,
+// 19.3 ms with the arc tangent in FP64 as well.  One point per thread: two
+// with 128-bit accesses took 22.45 ms when this form took 19.26, and with the
+// registers capped for two / three / four blocks either stayed within
+// 19.2-19.5 ms.
 template <bool ADV, bool SRC>
 __global__ void __launch_bounds__(256) ice_adjust_kernel(const __grid_constant__ Cst c,
                                                             const __grid_constant__ IaKernelFields kf,

@@ -143,12 +143,14 @@ struct IaDerived {
   double cpv_cl, cpv_ci;    // CPV - CL, CPV - CI
   int nrr, fmode, mfpdf, lambda3;
   int subg, sig_full;       // LSUBG_COND; LSIGMAS and not LSTATNW
+  int mix_up;               // 0 < TMINMIX < TMAXMIX
 };
 ICE3_HD IaDerived ia_derived(const Cst &c)
 {
   return {c.RD / c.RV, c.RV / c.RD, 1.0 / c.RV, fm::frcp(c.TMAXMIX - c.TMINMIX), c.CPV - c.CL, c.CPV - c.CI,
           (int)c.NRR, (int)c.FRAC_ICE_ADJUST, (int)c.SUBG_MF_PDF, (int)c.LAMBDA3,
-          c.LSUBG_COND != 0.0, c.LSIGMAS != 0.0 && c.LSTATNW == 0.0};
+          c.LSUBG_COND != 0.0, c.LSIGMAS != 0.0 && c.LSTATNW == 0.0,
+          0.0 < c.TMINMIX && c.TMINMIX < c.TMAXMIX};
 }
 
 // min(e, 0.99 p): the product only where a lane of the warp has e above p / 4
@@ -186,7 +188,7 @@ ICE3_HD void ia_point(const Cst &c, const IaDerived &d, double dt, double inv_dt
   double hlc_hrc = 0.0, hlc_hcf = 0.0, hli_hri = 0.0, hli_hcf = 0.0;
   if (d.subg) {
     // OCND2: ZPRIFACT = 0, the ice is kept out of the total water (condensation.F90:265-273)
-    const double rt = OCND2 ? x.rv + x.rc : x.rv + x.rc + x.ri;
+    const double rci = OCND2 ? x.rc : x.rc + x.ri, rt = x.rv + rci;
     const double it = fm::frcp(t);
     double pv, piv, frac, esw = 0.0;
     if (!OCND2) {
@@ -197,9 +199,17 @@ ICE3_HD void ia_point(const Cst &c, const IaDerived &d, double dt, double inv_dt
       // of the condensate
       const int fmode = d.fmode;
       if (fmode == 0) {
-        frac = nclip01(fm::mul_(c.TMAXMIX - t, d.imix));
+        // (0 above TMAXMIX and 1 below TMINMIX decided on the high words of a
+        // finite t; a NaN has to reach the clip, which keeps it)
+        const int32_t ht = (int32_t)fm::hi_(t);
+        const bool words = d.mix_up && (ht & 0x7fffffff) < 0x7ff00000;
+        const bool above = words && ht > (int32_t)fm::hi_(c.TMAXMIX);
+        const bool below = words && ht < (int32_t)fm::hi_(c.TMINMIX);
+        frac = below ? 1.0 : 0.0;
+        if (warp_any(!above && !below) && !above && !below) frac = nclip01(fm::mul_(c.TMAXMIX - t, d.imix));
       } else {
-        frac = fgt(x.rc + x.ri, 1e-20) ? fm::fdiv(x.rc, x.rc + x.ri) : 0.0;
+        const double s = x.rc + x.ri;
+        frac = fgt(s, 1e-20) ? fm::fdiv(x.rc, s) : 0.0;
         if (fmode == 3) frac = nclip01(frac);
       }
       // saturation over water and over ice, each only where the fraction
@@ -234,25 +244,22 @@ ICE3_HD void ia_point(const Cst &c, const IaDerived &d, double dt, double inv_dt
       qsl = qsi;
     }
     const double ah = lvs * qsl * (it * it * d.irv) * (1.0 + qsl * d.rvrd);
-    const double a = fm::frcp(1.0 + lvs * inv_cph * ah);
-    const double sbar = a * (rt - qsl + ah * lvs * (OCND2 ? x.rc : x.rc + x.ri) * inv_cph);
-    // sigma = sqrt(S) as S * S^(-1/2), the reciprocal reused for q1 when the
-    // 1e-10 floor leaves sigma alone
-    double sigma, isig = 0.0;
-    if (d.sig_full && !(fge(x.sigqsat, 0.0) && fge(0.0, x.sigqsat))) {
-      const double s2 = sq(2.0 * x.sigs) + sq(x.sigqsat * qsl * a);
-      if (fm::frsqrt_ok(s2)) {
-        isig = fm::frsqrt(s2);
-        sigma = s2 * isig;
-      } else {
-        sigma = sqrt(s2);
-      }
+    const double lah = lvs * inv_cph * ah;
+    const double a = fm::frcp(1.0 + lah);
+    const double sbar = a * (rt - qsl + lah * rci);
+    // q1 = sbar / sigma with sigma = sqrt(S) as S^(-1/2), sigma itself formed
+    // where there is a condensate; the 1e-10 floor of sigma is S <= 1e-20
+    double s2 = 0.0, isig = 0.0, sigma = 0.0, q1;
+    const bool full = d.sig_full && !(fge(x.sigqsat, 0.0) && fge(0.0, x.sigqsat));
+    if (full) s2 = sq(2.0 * x.sigs) + sq(x.sigqsat * qsl * a);
+    const bool fast = full && gtp(s2, 1.0000001e-20) && fm::frsqrt_ok(s2);
+    if (fast) {
+      isig = fm::frsqrt(s2);
+      q1 = sbar * isig;
     } else {
-      sigma = 2.0 * x.sigs;
+      sigma = nmax(1e-10, full ? fm::fsqrt_rn(s2) : 2.0 * x.sigs);
+      q1 = fm::fdiv(sbar, sigma);
     }
-    const double sig = nmax(1e-10, sigma);
-    const double q1 = (nz(isig) && fm::bits_(sig) == fm::bits_(sigma)) ? sbar * isig : fm::fdiv(sbar, sig);
-    sigma = sig;
     if (srcs) *srcs = sigrc_cb(d.lambda3, q1);
     // where the clipped cloud fraction is 0 the condensate is 0 too: below
     // -ICE3_Q1_CLIP neither the exponential nor the arc tangent is formed,
@@ -261,6 +268,7 @@ ICE3_HD void ia_point(const Cst &c, const IaDerived &d, double dt, double inv_dt
     if (!fge(-ICE3_Q1_CLIP, q1)) {
       if (fgt(q1, 0.0)) cond = fge(2.0, q1) ? nmin(0.36787944117144233 + 0.66 * q1 + 0.086 * q1 * q1, 2.0) : q1;
       else cond = fm::fexp(1.2 * q1 - 1.0);
+      if (fast) sigma = s2 * isig;
       cond *= sigma;
       if (fge(cond, 1e-12)) cldfr = fge(q1, ICE3_Q1_CLIP) ? 1.0 : nclip01(0.5 + 0.36 * fm::fatan(1.55 * q1));
       if (fge(cldfr, 0.0) && fge(0.0, cldfr)) cond = 0.0;
@@ -268,12 +276,12 @@ ICE3_HD void ia_point(const Cst &c, const IaDerived &d, double dt, double inv_dt
     if (!OCND2) {
       rc_out = all_i ? 0.0 : cond;
       ri_out = all_i ? cond : 0.0;
-      if (mixed) {
+      if (mixed || warp_any(isnan_(cond))) {           // (a NaN condensate goes to both)
         rc_out = (1.0 - frac) * cond;
         ri_out = frac * cond;
       }
       t = t + ((rc_out - x.rc) * lv + (ri_out - x.ri) * ls) * inv_cph;
-      rv_out = rt - rc_out - ri_out;
+      rv_out = mixed ? rt - rc_out - ri_out : rt - cond;
     } else {
       // condensation.F90:588-637.  ZRSW = -9999 (:263) keeps the noise
       // check's sub-saturation branch closed (ZRSDIF = 0): the liquid content
@@ -302,11 +310,10 @@ ICE3_HD void ia_point(const Cst &c, const IaDerived &d, double dt, double inv_dt
   w1 = fgt(0.0, w1) ? nmax(w1, -rcs) : nmin(w1, rvs);
   rvs = rvs - w1;
   rcs = rcs + w1;
-  ths = ths + w1 * lv * inv_cphex;
   w2 = fgt(0.0, w2) ? nmax(w2, -ris) : nmin(w2, rvs);
   rvs = rvs - w2;
   ris = ris + w2;
-  ths = ths + w2 * ls * inv_cphex;
+  ths = ths + (w1 * lv + w2 * ls) * inv_cphex;
   if (!d.subg) {
     cldfr = fgt((rcs + ris) * dt, 1e-12) ? 1.0 : 0.0;
     if (srcs) *srcs = cldfr;
