@@ -271,10 +271,10 @@ __global__ void __launch_bounds__(G_THREADS) tc_gemm_kernel(const TcGemmArgs a)
 //   21     one thread issues the weight copies
 // so that the MMAs of one slot run while the other slot's GELU does.
 // Bound: the GELU warps (32,768 hardware tanh per layer and tile at 16 per
-// clock, and the FP32 operations around them, 1.2 us) - the MMAs (1.4 us per
-// hidden layer and tile) are behind them.  2 M rows take 0.84 ms (684
-// TFLOP/s); with one tile in flight and all warps in step, MMAs and GELU
-// largely in turn, they took 1.21 ms.
+// clock and the FP32 operations around them, which take two values per
+// instruction) and their reads of TMEM.  2 M rows take 0.745 ms (775
+// TFLOP/s); 0.844 ms with one value per instruction; 1.21 ms with one tile in
+// flight and all warps in step, MMAs and GELU largely in turn.
 constexpr int FZ_NST = 4;                               // weight ring stages
 constexpr int FZ_KC = 32;                               // K of a weight chunk
 constexpr int FZ_GELU_WARPS = 16, FZ_IO_WARP = 16, FZ_MMA_WARP = 20, FZ_COPY_WARP = 21, FZ_THREADS = 32 * 22;
@@ -284,23 +284,61 @@ constexpr int FZ_OFF_H = 0, FZ_OFF_STAGE = 2 * 65536, FZ_OFF_W1 = FZ_OFF_STAGE +
 constexpr int FZ_OFF_W4 = FZ_OFF_W1 + 8192, FZ_OFF_X = FZ_OFF_W4 + 8192, FZ_OFF_B = FZ_OFF_X + 2 * 4096;
 constexpr int FZ_SMEM = FZ_OFF_B + (3 * 256 + 16) * 4;
 
+// Two FP32 operations per instruction (sm_100 and later), each rounded as the
+// scalar one.
+__device__ __forceinline__ uint64_t f32x2(float a, float b)
+{
+  uint64_t d;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(a), "f"(b));
+  return d;
+}
+__device__ __forceinline__ uint64_t add_f32x2(uint64_t a, uint64_t b)
+{
+  uint64_t d;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+__device__ __forceinline__ uint64_t mul_f32x2(uint64_t a, uint64_t b)
+{
+  uint64_t d;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+__device__ __forceinline__ uint64_t fma_f32x2(uint64_t a, uint64_t b, uint64_t c)
+{
+  uint64_t d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+  return d;
+}
+
+// gelu() of the two values r + b, packed to BF16: the same operations in the
+// same order, two at a time.
+__device__ __forceinline__ uint32_t fz_gelu2(uint32_t r0, uint32_t r1, uint64_t b)
+{
+  const uint64_t z = add_f32x2(f32x2(__uint_as_float(r0), __uint_as_float(r1)), b);
+  const uint64_t k1 = f32x2(0.035677408136300125f, 0.035677408136300125f), k0 = f32x2(0.7978845608028654f, 0.7978845608028654f);
+  const uint64_t u = mul_f32x2(z, fma_f32x2(k1, mul_f32x2(z, z), k0)), h = mul_f32x2(f32x2(0.5f, 0.5f), z);
+  float ux, uy, gx, gy;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(ux), "=f"(uy) : "l"(u));
+  const uint64_t g = fma_f32x2(h, f32x2(tanh_hw(ux), tanh_hw(uy)), h);
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(gx), "=f"(gy) : "l"(g));
+  return bf16x2_bits(gx, gy);
+}
+
 // Bias + GELU of 32 accumulator columns (from cb0) of one row into the
-// activation tile (the MUFU tanh is the epilogue's bound); the biases are read
-// four at a time (the same address for the whole warp).
+// activation tile; the biases are read four at a time (the same address for
+// the whole warp).
 __device__ __forceinline__ void fz_gelu32(const uint32_t r[32], const float *bias, int cb0, int row, __nv_bfloat16 *sH)
 {
 #pragma unroll
   for (int g = 0; g < 4; ++g) {
     const int cb = cb0 + 8 * g;
-    const float4 b0 = *reinterpret_cast<const float4 *>(bias + cb);
-    const float4 b1 = *reinterpret_cast<const float4 *>(bias + cb + 4);
-    const float bb[8] = {b0.x, b0.y, b0.z, b0.w, b1.x, b1.y, b1.z, b1.w};
-    uint32_t w[4];
-#pragma unroll
-    for (int j = 0; j < 4; ++j)
-      w[j] = bf16x2_bits(gelu(__uint_as_float(r[8 * g + 2 * j]) + bb[2 * j]),
-                         gelu(__uint_as_float(r[8 * g + 2 * j + 1]) + bb[2 * j + 1]));
-    *reinterpret_cast<uint4 *>(sH + tc::core_off(row, cb, 256)) = make_uint4(w[0], w[1], w[2], w[3]);
+    const ulonglong2 b0 = *reinterpret_cast<const ulonglong2 *>(bias + cb);
+    const ulonglong2 b1 = *reinterpret_cast<const ulonglong2 *>(bias + cb + 4);
+    const uint32_t *q = r + 8 * g;
+    *reinterpret_cast<uint4 *>(sH + tc::core_off(row, cb, 256)) =
+        make_uint4(fz_gelu2(q[0], q[1], b0.x), fz_gelu2(q[2], q[3], b0.y), fz_gelu2(q[4], q[5], b1.x),
+                   fz_gelu2(q[6], q[7], b1.y));
   }
 }
 
