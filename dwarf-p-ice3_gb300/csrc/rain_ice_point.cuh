@@ -349,9 +349,10 @@ ICE3_HD double compute_pdf(const Cst &c, const Derived &d, double rcrautc, doubl
   if (soft && aucv_ri == 0) {
     // a soft pass reads only rit > MIN(CRIAUTI, 10**x) = rit > CRIAUTI or
     // rit > 10**x, decided from an FP32 estimate of 10**x (within 2^-16)
-    // unless rit is within 2^-12 of it
+    // unless rit is within 2^-12 of it; a NaN or infinite t (which to_f32 does
+    // not keep) leaves rit > CRIAUTI
     ice_high = gtd(rit, c.CRIAUTI);
-    const bool open = !ice_high && gtp(rit, c.I_RTMIN);
+    const bool open = !ice_high && gtp(rit, c.I_RTMIN) && finite_(t);
     bool near = false;
     if (warp_any(open)) {
       const float x = fm::fmaf_(d.acriauti_f, fm::to_f32(t) - d.tt_f, d.bcriauti_f);
@@ -1294,6 +1295,13 @@ ICE3_HD void tendencies(const Cst &c, const Derived &d, const double *__restrict
   aggregate<H, O>(c, d, t, v, lvfact, lsfact, R, A, soft, hr, B, orr, ext);
 }
 
+// (a - z) (b - z) < 0: a and b on different sides of z.  The integer compares
+// rank a NaN as a number; a product with one is not < 0.
+ICE3_HD bool crosses(double a, double b, double z)
+{
+  return ((gtd(a, z) && ltd(b, z)) || (ltd(a, z) && gtd(b, z))) && !isnan_(a) && !isnan_(b) && !isnan_(z);
+}
+
 // ICE4_STEPPING for one micro point (mode_ice4_stepping.F90:139-518).
 // Returns the pass key (outer << 16 | inner-of-last-outer), 0 if capped.
 // t_0, ls_0, lv_0, zdev_0: temperature, latent heats and cph of the state at
@@ -1379,11 +1387,9 @@ ICE3_HD unsigned int stepping(const Cst &c, const Derived &d, const double *__re
       // B (the instantaneous changes) is zero on soft passes: no theta jump
       // across TT/exn, no B in the depletion limits and the state update
       if (d.lfeedbackt) {
-        // (th - zx) (th + B - zx) < 0: the two on different sides of zx
         double num = zx;
         if (!soft) {
-          const double tb = vart[ITH] + B[ITH];
-          if ((gtd(vart[ITH], zx) && ltd(tb, zx)) || (ltd(vart[ITH], zx) && gtd(tb, zx))) maxtime = 0.;
+          if (crosses(vart[ITH], vart[ITH] + B[ITH], zx)) maxtime = 0.;
           num = zx - B[ITH];
         }
         if (abs_gtp(A[ITH], 1.e-20)) {
