@@ -17,7 +17,7 @@ using namespace ice3ia;
 // physics step) instead of th/rv/.../rg, which are then not read; rrs/rss/rgs
 // are read instead.  Output pointers may be NULL in the internal chained use
 // (store skipped).
-// Bound: the FP64 pipe.  At 1024x1024x90 a launch takes 15.4 ms (1.7 TB/s of
+// Bound: the FP64 pipe.  At 1024x1024x90 a launch takes 15.9 ms (1.7 TB/s of
 // HBM); 16.8 ms before the ice fraction was decided on the high words, the
 // products of sbar shared and sigma formed only where there is a condensate,
 // 19.3 ms with the arc tangent in FP64 as well.  One point per thread: two

@@ -276,12 +276,13 @@ ICE3_HD void ia_point(const Cst &c, const IaDerived &d, double dt, double inv_dt
     if (!OCND2) {
       rc_out = all_i ? 0.0 : cond;
       ri_out = all_i ? cond : 0.0;
-      if (mixed || warp_any(isnan_(cond))) {           // (a NaN condensate goes to both)
+      const bool split = warp_any(mixed || !finite_(cond));   // (0 of an infinite or NaN condensate is NaN)
+      if (split) {
         rc_out = (1.0 - frac) * cond;
         ri_out = frac * cond;
       }
       t = t + ((rc_out - x.rc) * lv + (ri_out - x.ri) * ls) * inv_cph;
-      rv_out = mixed ? rt - rc_out - ri_out : rt - cond;
+      rv_out = split ? rt - rc_out - ri_out : rt - cond;
     } else {
       // condensation.F90:588-637.  ZRSW = -9999 (:263) keeps the noise
       // check's sub-saturation branch closed (ZRSDIF = 0): the liquid content
@@ -310,10 +311,11 @@ ICE3_HD void ia_point(const Cst &c, const IaDerived &d, double dt, double inv_dt
   w1 = fgt(0.0, w1) ? nmax(w1, -rcs) : nmin(w1, rvs);
   rvs = rvs - w1;
   rcs = rcs + w1;
+  ths = ths + w1 * lv * inv_cphex;
   w2 = fgt(0.0, w2) ? nmax(w2, -ris) : nmin(w2, rvs);
   rvs = rvs - w2;
   ris = ris + w2;
-  ths = ths + (w1 * lv + w2 * ls) * inv_cphex;
+  ths = ths + w2 * ls * inv_cphex;
   if (!d.subg) {
     cldfr = fgt((rcs + ris) * dt, 1e-12) ? 1.0 : 0.0;
     if (srcs) *srcs = cldfr;
@@ -457,13 +459,15 @@ ICE3_HD void ia_point_vjp(const Cst &c, const IaDerived &d, double dt, double in
       frac_pass = true;
     }
     // the saturation over water / ice where it has a weight, or where the
-    // weight's own derivative reads it (FRAC_ICE_ADJUST 0 within its range)
-    if (fmode != 0 || frac_pass || fm::bits_(frac) != fm::bits_(1.0)) {
+    // weight's own derivative reads it (FRAC_ICE_ADJUST 0 within its range),
+    // both at a temperature that is not finite
+    const bool both = fmode != 0 || frac_pass || !finite_(t0);
+    if (both || fm::bits_(frac) != fm::bits_(1.0)) {
       ew = fm::fexp(c.ALPW - c.BETAW * it - c.GAMW * lt);
       pv = nmin_sel(ew, 0.99 * x.pabs, pv_first);
       qsl0 = fm::fdiv(d.rdrv * pv, x.pabs - pv);
     }
-    if (fmode != 0 || frac_pass || !zerod_(frac)) {
+    if (both || !zerod_(frac)) {
       ei = fm::fexp(c.ALPI - c.BETAI * it - c.GAMI * lt);
       piv = nmin_sel(ei, 0.99 * x.pabs, piv_first);
       qsi = fm::fdiv(d.rdrv * piv, x.pabs - piv);
@@ -536,8 +540,9 @@ ICE3_HD void ia_point_vjp(const Cst &c, const IaDerived &d, double dt, double in
     double b_w1m = 0.0, b_w2m = 0.0, b_cf = 0.0;
     const int mfpdf = d.mfpdf;
     // (a warp without mass-flux clouds has zero contents on the flat part of
-    // the PDF: nothing flows back)
-    if ((mfpdf == 0 || mfpdf == 1) && warp_any(nz(x.cf_mf) || nz(w1m) || nz(w2m))) {
+    // the PDF: nothing flows back where the thresholds are finite)
+    if ((mfpdf == 0 || mfpdf == 1) &&
+        warp_any(nz(x.cf_mf) || nz(w1m) || nz(w2m) || !finite_(x.rho) || !finite_(t))) {
       const double criaut = fm::fdiv(c.CRIAUTC, x.rho);
       const double p10 = fm::fexp10(c.ACRIAUTI * (t - c.TT) + c.BCRIAUTI);
       bool ci_const;
