@@ -2,7 +2,7 @@
 // per-point MLP of the slow-process surrogate built on it (forward,
 // hand-written backward, Adam).
 //
-// tc_gemm_kernel: one CTA (8 warps) computes a 128 x N tile (N <= 256) of
+// tc_gemm_kernel: one CTA (8 warps) computes a 128 x 128 tile (N <= 256) of
 //   C[m][n] = sum_k A(m, k) B(n, k),  A(m, k) = A[m*sam + k*sak],  B(n, k) = B[n*sbn + k*sbk]
 // in FP32 in TMEM.  K is walked in chunks of 64 through a ring of G_NST
 // shared-memory stages in the K-major core-matrix layout, filled with 16-byte
@@ -22,7 +22,8 @@
 // Bound: at the training batch (16,384 rows) the latency of filling the ring
 // and the epilogue's stores; four warps, one stage and element-wise transposing
 // took 122 us per hidden layer forward, 299 us backward and 776 us per weight
-// gradient.
+// gradient.  Tiles of 128 columns with three stages put two CTAs on an SM: a
+// gradient of 16,384 rows 407 -> 387 us against tiles of 256 with four.
 // On a barrier timeout the kernel sets *err, stops issuing and frees its
 // TMEM after a second bounded wait.
 #include <cuda_bf16.h>
@@ -60,8 +61,8 @@ __device__ __forceinline__ float dgelu(float z)
   return 0.5f * (1.0f + th) + 0.5f * z * (1.0f - th * th) * du;
 }
 
-constexpr int G_THREADS = 256, G_NST = 4;
-constexpr int G_A = 128 * KC, G_STAGE = (128 + 256) * KC;         // elements of a stage (A, then B)
+constexpr int G_THREADS = 256, G_NST = 3, G_NT = 128;             // G_NT: columns of a CTA's tile
+constexpr int G_A = 128 * KC, G_STAGE = (128 + G_NT) * KC;        // elements of a stage (A, then B)
 
 // 16 bytes global -> shared, or zeros
 __device__ __forceinline__ void copy16(__nv_bfloat16 *dst, const __nv_bfloat16 *src, bool in)
@@ -109,8 +110,8 @@ __global__ void __launch_bounds__(G_THREADS) tc_gemm_kernel(const TcGemmArgs a)
   __shared__ __align__(8) uint64_t mbar[G_NST];
   __shared__ uint32_t tmem_base;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int np = (a.N + 15) & ~15;
-  const uint32_t ncols = np <= 32 ? 32u : np <= 64 ? 64u : np <= 128 ? 128u : 256u;
+  const int n0 = blockIdx.z * G_NT, nt = min(a.N - n0, G_NT), np = (nt + 15) & ~15;
+  const uint32_t ncols = np <= 32 ? 32u : np <= 64 ? 64u : 128u;
   const long m0 = (long)blockIdx.x * 128;
   // K range of this split
   const int kpad = (a.K + 15) & ~15;
@@ -137,7 +138,7 @@ __global__ void __launch_bounds__(G_THREADS) tc_gemm_kernel(const TcGemmArgs a)
     // (nothing past this split's range is read: its chunk count ends there)
     const int k0 = kbeg + ch * KC, K = min(a.K, kend);
     stage_tile(sA, a.A, a.sam, a.sak, m0, 128, a.M, k0, K, a_vec, tid);
-    stage_tile(sA + G_A, a.B, a.sbn, a.sbk, 0, np, a.N, k0, K, b_vec, tid);
+    stage_tile(sA + G_A, a.B, a.sbn, a.sbk, n0, np, a.N, k0, K, b_vec, tid);
   };
   for (int ch = 0; ch < G_NST - 1; ++ch) {
     if (ch < nch) fill(ch);
@@ -186,38 +187,39 @@ __global__ void __launch_bounds__(G_THREADS) tc_gemm_kernel(const TcGemmArgs a)
     const bool c4 = aligned_rows(a.C, a.ldc, 4), z4 = aligned_rows(a.Zout ? a.Zout : a.Zin, a.ldz, 4);
     const bool h8 = aligned_rows(a.H, a.ldh, 2);
     for (int c0 = 16 * (warp >> 2); c0 < np; c0 += 32) {
+      const int gc = n0 + c0;                          // the column of C
       float v[16];
       if (issued) tc::tmem_ld16(tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)c0, v);
       else
         for (int j = 0; j < 16; ++j) v[j] = 0.0f;
-      const bool full = c0 + 16 <= a.N;
+      const bool full = c0 + 16 <= nt;
       float h[16];                                     // what H takes
       if (a.epi == EPI_DGELU) {
         float z[16];
         if (in && full && z4) {
 #pragma unroll
           for (int q = 0; q < 4; ++q) {
-            const float4 t = __ldg(reinterpret_cast<const float4 *>(a.Zin + m * a.ldz + c0) + q);
+            const float4 t = __ldg(reinterpret_cast<const float4 *>(a.Zin + m * a.ldz + gc) + q);
             z[4 * q] = t.x; z[4 * q + 1] = t.y; z[4 * q + 2] = t.z; z[4 * q + 3] = t.w;
           }
         } else {
 #pragma unroll
-          for (int j = 0; j < 16; ++j) z[j] = (in && c0 + j < a.N) ? a.Zin[m * a.ldz + c0 + j] : 0.0f;
+          for (int j = 0; j < 16; ++j) z[j] = (in && c0 + j < nt) ? a.Zin[m * a.ldz + gc + j] : 0.0f;
         }
 #pragma unroll
         for (int j = 0; j < 16; ++j) h[j] = v[j] *= dgelu(z[j]);
       } else if (a.epi != EPI_STORE) {
 #pragma unroll
         for (int j = 0; j < 16; ++j) {
-          if (c0 + j < a.N) v[j] += a.bias[c0 + j];
+          if (c0 + j < nt) v[j] += a.bias[gc + j];
           h[j] = a.epi == EPI_BIAS_GELU ? gelu(v[j]) : 0.0f;
         }
       }
       // FP32 result: Z of the forward, C of the others
       float *const o = a.epi == EPI_BIAS_GELU ? a.Zout : a.C;
       if (o && in) {
-        float *const d = a.epi == EPI_BIAS_GELU ? o + m * a.ldz + c0
-                                                : o + (a.epi == EPI_STORE ? (long)blockIdx.y * a.M * a.ldc : 0L) + m * a.ldc + c0;
+        float *const d = a.epi == EPI_BIAS_GELU ? o + m * a.ldz + gc
+                                                : o + (a.epi == EPI_STORE ? (long)blockIdx.y * a.M * a.ldc : 0L) + m * a.ldc + gc;
         if (full && (a.epi == EPI_BIAS_GELU ? z4 : (c4 && (a.epi != EPI_STORE || ((a.M * a.ldc) & 3) == 0)))) {
 #pragma unroll
           for (int q = 0; q < 4; ++q)
@@ -225,12 +227,12 @@ __global__ void __launch_bounds__(G_THREADS) tc_gemm_kernel(const TcGemmArgs a)
         } else {
 #pragma unroll
           for (int j = 0; j < 16; ++j)
-            if (c0 + j < a.N) d[j] = v[j];
+            if (c0 + j < nt) d[j] = v[j];
         }
       }
       if (a.epi != EPI_BIAS_GELU && a.epi != EPI_DGELU) continue;
       if (in) {
-        __nv_bfloat16 *const d = a.H + m * a.ldh + c0;
+        __nv_bfloat16 *const d = a.H + m * a.ldh + gc;
         if (full && h8) {
 #pragma unroll
           for (int q = 0; q < 2; ++q)
@@ -240,13 +242,13 @@ __global__ void __launch_bounds__(G_THREADS) tc_gemm_kernel(const TcGemmArgs a)
         } else {
 #pragma unroll
           for (int j = 0; j < 16; ++j)
-            if (c0 + j < a.N) d[j] = __float2bfloat16(h[j]);
+            if (c0 + j < nt) d[j] = __float2bfloat16(h[j]);
         }
       }
       if (a.HT) {
 #pragma unroll
         for (int j = 0; j < 16; ++j)
-          if (c0 + j < a.N) a.HT[(long)(c0 + j) * a.ldht + m] = __float2bfloat16(in ? h[j] : 0.0f);
+          if (c0 + j < nt) a.HT[(long)(gc + j) * a.ldht + m] = __float2bfloat16(in ? h[j] : 0.0f);
       }
     }
   }
@@ -690,7 +692,7 @@ cudaError_t launch_tc_gemm(const TcGemmArgs &a, cudaStream_t s)
   cudaError_t e = cudaFuncSetAttribute(tc_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        (int)tc_gemm_smem_bytes());
   if (e != cudaSuccess) return e;
-  dim3 grid((unsigned)((a.M + 127) / 128), (unsigned)a.k_split);
+  dim3 grid((unsigned)((a.M + 127) / 128), (unsigned)a.k_split, (unsigned)((a.N + G_NT - 1) / G_NT));
   tc_gemm_kernel<<<grid, G_THREADS, tc_gemm_smem_bytes(), s>>>(a);
   return cudaGetLastError();
 }

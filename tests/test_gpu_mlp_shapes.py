@@ -48,3 +48,11 @@ def test_transposed_weights_follow_training_steps():
     other, _, _ = _case(300, 256, 3, 10, seed=4)
     other.set_params(net.get_params())
     assert torch.equal(net.loss_grad(x, t)[1], other.loss_grad(x, t)[1])
+
+
+@pytest.mark.parametrize("n,hidden,layers,n_out", [(129, 128, 2, 10), (200, 132, 2, 10), (257, 144, 3, 16), (130, 200, 2, 6),
+                                                   (64, 252, 2, 2)])
+def test_gradients_at_column_tile_edges(n, hidden, layers, n_out):
+    """Hidden widths around the 128 columns of a CTA's tile, with a second tile
+    from 4 columns to almost full; the bounds above."""
+    test_gradients_at_tile_edges(n, hidden, layers, n_out)
