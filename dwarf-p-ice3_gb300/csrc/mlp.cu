@@ -24,6 +24,8 @@
 // took 122 us per hidden layer forward, 299 us backward and 776 us per weight
 // gradient.  Tiles of 128 columns with three stages put two CTAs on an SM: a
 // gradient of 16,384 rows 407 -> 387 us against tiles of 256 with four.
+// The epilogue's rows go through the ring's shared memory, four lanes to a
+// row: 387 -> 359 us against a lane to a row, whose accesses touch 32 lines.
 // On a barrier timeout the kernel sets *err, stops issuing and frees its
 // TMEM after a second bounded wait.
 #include <cuda_bf16.h>
@@ -101,6 +103,56 @@ __device__ __forceinline__ uint32_t bf16x2_bits(float a, float b)
 __device__ __forceinline__ bool aligned_rows(const void *p, long ld, int elem)
 {
   return (((uintptr_t)p | (uintptr_t)(ld * elem)) & 15) == 0;
+}
+
+// A warp's 32 rows x 16 values (row = lane, in v) to rows of x, and back,
+// through its part of shared memory: four lanes take a row's 64 bytes (two a
+// row's 32 for BF16), so that an access touches 8 (16) lines instead of 32.
+// rows: how many of the 32 there are.  All lanes call.
+constexpr int G_LINE = 20;                                        // words per row in the buffer (16 bytes apart)
+__device__ __forceinline__ void store_rows(float *x, long ld, int rows, const float v[16], float *buf, int lane)
+{
+#pragma unroll
+  for (int q = 0; q < 4; ++q)
+    *reinterpret_cast<float4 *>(buf + lane * G_LINE + 4 * q) = make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
+  __syncwarp();
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const int r = 8 * i + (lane >> 2), q = lane & 3;
+    if (r < rows) *reinterpret_cast<float4 *>(x + r * ld + 4 * q) = *reinterpret_cast<const float4 *>(buf + r * G_LINE + 4 * q);
+  }
+  __syncwarp();
+}
+__device__ __forceinline__ void load_rows(const float *x, long ld, int rows, float v[16], float *buf, int lane)
+{
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const int r = 8 * i + (lane >> 2), q = lane & 3;
+    *reinterpret_cast<float4 *>(buf + r * G_LINE + 4 * q) =
+        r < rows ? __ldg(reinterpret_cast<const float4 *>(x + r * ld + 4 * q)) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+  }
+  __syncwarp();
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    const float4 t = *reinterpret_cast<const float4 *>(buf + lane * G_LINE + 4 * q);
+    v[4 * q] = t.x; v[4 * q + 1] = t.y; v[4 * q + 2] = t.z; v[4 * q + 3] = t.w;
+  }
+  __syncwarp();
+}
+__device__ __forceinline__ void store_rows(__nv_bfloat16 *x, long ld, int rows, const float h[16], float *buf, int lane)
+{
+#pragma unroll
+  for (int q = 0; q < 2; ++q)
+    *reinterpret_cast<uint4 *>(buf + lane * G_LINE + 4 * q) =
+        make_uint4(bf16x2_bits(h[8 * q], h[8 * q + 1]), bf16x2_bits(h[8 * q + 2], h[8 * q + 3]),
+                   bf16x2_bits(h[8 * q + 4], h[8 * q + 5]), bf16x2_bits(h[8 * q + 6], h[8 * q + 7]));
+  __syncwarp();
+#pragma unroll
+  for (int i = 0; i < 2; ++i) {
+    const int r = 16 * i + (lane >> 1), q = lane & 1;
+    if (r < rows) *reinterpret_cast<uint4 *>(x + r * ld + 8 * q) = *reinterpret_cast<const uint4 *>(buf + r * G_LINE + 4 * q);
+  }
+  __syncwarp();
 }
 
 __global__ void __launch_bounds__(G_THREADS) tc_gemm_kernel(const TcGemmArgs a)
@@ -182,8 +234,10 @@ __global__ void __launch_bounds__(G_THREADS) tc_gemm_kernel(const TcGemmArgs a)
   // ---- epilogue
   if (ok) {
     const int row = (warp & 3) * 32 + lane;
-    const long m = m0 + row;
+    const long m = m0 + row, mw = m - lane;            // the lane's row, the warp's first
     const bool in = m < a.M;
+    const int rows = (int)min(32L, (long)a.M - mw);
+    float *const buf = reinterpret_cast<float *>(smem_raw) + warp * 32 * G_LINE;   // (the ring: its MMAs are done)
     const bool c4 = aligned_rows(a.C, a.ldc, 4), z4 = aligned_rows(a.Zout ? a.Zout : a.Zin, a.ldz, 4);
     const bool h8 = aligned_rows(a.H, a.ldh, 2);
     for (int c0 = 16 * (warp >> 2); c0 < np; c0 += 32) {
@@ -196,12 +250,8 @@ __global__ void __launch_bounds__(G_THREADS) tc_gemm_kernel(const TcGemmArgs a)
       float h[16];                                     // what H takes
       if (a.epi == EPI_DGELU) {
         float z[16];
-        if (in && full && z4) {
-#pragma unroll
-          for (int q = 0; q < 4; ++q) {
-            const float4 t = __ldg(reinterpret_cast<const float4 *>(a.Zin + m * a.ldz + gc) + q);
-            z[4 * q] = t.x; z[4 * q + 1] = t.y; z[4 * q + 2] = t.z; z[4 * q + 3] = t.w;
-          }
+        if (full && z4) {
+          load_rows(a.Zin + mw * a.ldz + gc, a.ldz, rows, z, buf, lane);
         } else {
 #pragma unroll
           for (int j = 0; j < 16; ++j) z[j] = (in && c0 + j < nt) ? a.Zin[m * a.ldz + gc + j] : 0.0f;
@@ -217,33 +267,25 @@ __global__ void __launch_bounds__(G_THREADS) tc_gemm_kernel(const TcGemmArgs a)
       }
       // FP32 result: Z of the forward, C of the others
       float *const o = a.epi == EPI_BIAS_GELU ? a.Zout : a.C;
-      if (o && in) {
-        float *const d = a.epi == EPI_BIAS_GELU ? o + m * a.ldz + gc
-                                                : o + (a.epi == EPI_STORE ? (long)blockIdx.y * a.M * a.ldc : 0L) + m * a.ldc + gc;
+      if (o) {
+        const long ld = a.epi == EPI_BIAS_GELU ? a.ldz : a.ldc;
+        float *const d = o + (a.epi == EPI_STORE ? (long)blockIdx.y * a.M * a.ldc : 0L) + mw * ld + gc;
         if (full && (a.epi == EPI_BIAS_GELU ? z4 : (c4 && (a.epi != EPI_STORE || ((a.M * a.ldc) & 3) == 0)))) {
-#pragma unroll
-          for (int q = 0; q < 4; ++q)
-            reinterpret_cast<float4 *>(d)[q] = make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
-        } else {
+          store_rows(d, ld, rows, v, buf, lane);
+        } else if (in) {
 #pragma unroll
           for (int j = 0; j < 16; ++j)
-            if (c0 + j < nt) d[j] = v[j];
+            if (c0 + j < nt) d[lane * ld + j] = v[j];
         }
       }
       if (a.epi != EPI_BIAS_GELU && a.epi != EPI_DGELU) continue;
-      if (in) {
-        __nv_bfloat16 *const d = a.H + m * a.ldh + gc;
-        if (full && h8) {
+      __nv_bfloat16 *const d = a.H + mw * a.ldh + gc;
+      if (full && h8) {
+        store_rows(d, a.ldh, rows, h, buf, lane);
+      } else if (in) {
 #pragma unroll
-          for (int q = 0; q < 2; ++q)
-            reinterpret_cast<uint4 *>(d)[q] =
-                make_uint4(bf16x2_bits(h[8 * q], h[8 * q + 1]), bf16x2_bits(h[8 * q + 2], h[8 * q + 3]),
-                           bf16x2_bits(h[8 * q + 4], h[8 * q + 5]), bf16x2_bits(h[8 * q + 6], h[8 * q + 7]));
-        } else {
-#pragma unroll
-          for (int j = 0; j < 16; ++j)
-            if (c0 + j < nt) d[j] = __float2bfloat16(h[j]);
-        }
+        for (int j = 0; j < 16; ++j)
+          if (c0 + j < nt) d[lane * a.ldh + j] = __float2bfloat16(h[j]);
       }
       if (a.HT) {
 #pragma unroll
@@ -684,6 +726,7 @@ __global__ void to_bf16_t_kernel(const float *__restrict__ x, __nv_bfloat16 *__r
 
 // The stage ring takes 192 KB, so one CTA is resident per SM and no
 // tcgen05.alloc has to wait for columns.
+static_assert(G_NST * G_STAGE * 2 >= G_THREADS * G_LINE * 4, "the epilogue's buffers fit in the ring");
 size_t tc_gemm_smem_bytes() { return (size_t)G_NST * G_STAGE * sizeof(__nv_bfloat16); }
 
 cudaError_t launch_tc_gemm(const TcGemmArgs &a, cudaStream_t s)
