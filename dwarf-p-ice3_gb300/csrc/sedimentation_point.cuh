@@ -321,6 +321,20 @@ ICE3_HD double sed_vjp_species(const Cst &c, int s, bool fortran, const CloudPar
   return b_fa;
 }
 
+// The gradients of the pressure and of theta at a level from the cotangent of
+// wlbda (proportional to theta / pressure): formed wherever a cloud speed was,
+// also where its cotangent is 0, so that a NaN input gives a NaN gradient;
+// 0 at a level without falling cloud.
+ICE3_HD void sed_cloud_gradients(bool cloud, double wlbda, double pabs, double tht, double b_wlbda, double &g_pabs,
+                                 double &g_tht)
+{
+  g_pabs = g_tht = 0.0;
+  if (cloud) {
+    g_pabs = -fm::fdiv(wlbda, pabs) * b_wlbda;
+    g_tht = fm::fdiv(wlbda, tht) * b_wlbda;
+  }
+}
+
 // Reverse sweep of one column (hand-written adjoint of sed_column_forward):
 // bottom-up, carrying the cotangent of the flux entering each level from
 // above.  `flux` holds the forward fluxes F_k of the column (io.fpr layout),
@@ -346,6 +360,7 @@ ICE3_HD void sed_column_vjp(const Cst &c, bool fortran, bool skip_c, const Cloud
     const double pabs = sed_load(io.pabs, p), tht = sed_load(io.tht, p);
     l.wlbda = 6.6e-8 * fm::fdiv(101325.0, pabs) * (tht * (1.0 / 293.15));
     SedLevelCot b = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+    bool cloud = false;
     for (int s = 0; s < 5; ++s) {
       const double gS = g.src[s] ? g.src[s][p] : 0.0;
       if (s == 0 && skip_c) {                       // sources passed through unchanged
@@ -354,6 +369,7 @@ ICE3_HD void sed_column_vjp(const Cst &c, bool fortran, bool skip_c, const Cloud
       }
       if (g.fpr[s]) bF[s] += g.fpr[s][p];
       const double fa = (k + 1 < io.nk) ? flux[s][p + io.nij] : 0.0;
+      if (s == 0) cloud = gtp(io.src_in[s][p] * dt, rtmin[s]) || gtp(fa * l.tso, rtmin[s]);
       double b_src;
       bF[s] = sed_vjp_species(c, s, fortran, cp, dt, inv_dt, l, io.src_in[s][p], rtmin[s], fa, flux[s][p], gS, bF[s],
                               b_src, b);
@@ -363,8 +379,10 @@ ICE3_HD void sed_column_vjp(const Cst &c, bool fortran, bool skip_c, const Cloud
     b.rhodz += -fm::fdiv(l.tso, l.rhodz) * b.tso;
     if (gx.rhodref) gx.rhodref[p] = b.rho + l.dz * b.rhodz + fm::fdiv(b.lrho, l.rho);
     if (gx.dzz) gx.dzz[p] = b.dz + l.rho * b.rhodz;
-    if (gx.pabs) gx.pabs[p] = -fm::fdiv(l.wlbda, pabs) * b.wlbda;
-    if (gx.tht) gx.tht[p] = fm::fdiv(l.wlbda, tht) * b.wlbda;
+    double g_pabs, g_tht;
+    sed_cloud_gradients(cloud, l.wlbda, pabs, tht, b.wlbda, g_pabs, g_tht);
+    if (gx.pabs) gx.pabs[p] = g_pabs;
+    if (gx.tht) gx.tht[p] = g_tht;
   }
 }
 

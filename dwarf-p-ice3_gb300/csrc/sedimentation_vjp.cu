@@ -89,17 +89,15 @@ __global__ void __launch_bounds__(32 * 5) sedimentation_vjp_kernel(const __grid_
           const double fa = (k + 1 < a.nk) ? flux[p + nij] : 0.0;
           SedLevelCot b = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
           double b_src;
-          bF = sed_vjp_species(c, s, fortran, cp, dt, inv_dt, l, ld1(src, p), rtmin, fa, flux[p], gS, bF, b_src, b);
+          const double sr = ld1(src, p);
+          bF = sed_vjp_species(c, s, fortran, cp, dt, inv_dt, l, sr, rtmin, fa, flux[p], gS, bF, b_src, b);
           if (gx_src) gx_src[p] = b_src;
           b.rhodz -= lv[LV_TSOR][lane] * b.tso;
           c_rho = b.rho + l.dz * b.rhodz + b.lrho * lv[LV_IRHO][lane];
           c_dz = b.dz + l.rho * b.rhodz;
           if (s == 0) {
-            double gp = 0.0, gt = 0.0;
-            if (nz(b.wlbda)) {
-              gp = -fm::fdiv(l.wlbda, pabs) * b.wlbda;
-              gt = fm::fdiv(l.wlbda, tht) * b.wlbda;
-            }
+            double gp, gt;
+            sed_cloud_gradients(gtp(sr * dt, rtmin) || gtp(fa * l.tso, rtmin), l.wlbda, pabs, tht, b.wlbda, gp, gt);
             if (a.gx.pabs) a.gx.pabs[p] = gp;
             if (a.gx.tht) a.gx.tht[p] = gt;
           }
