@@ -161,7 +161,11 @@ inline int clz32_(uint32_t v) { return v ? __builtin_clz(v) : 32; }
 inline uint32_t hi_(double x) { return (uint32_t)((uint64_t)bits_(x) >> 32); }
 inline uint32_t lo_(double x) { return (uint32_t)bits_(x); }
 inline uint32_t mulhi_(uint32_t a, uint32_t b) { return (uint32_t)(((uint64_t)a * b) >> 32); }
-inline float rcp_seed_(float x) { return rcpf_(x); }
+// (FM_HOST_SEED_ULPS: the tests move the seed by what the device's may be off)
+#ifndef FM_HOST_SEED_ULPS
+#define FM_HOST_SEED_ULPS 0
+#endif
+inline float rcp_seed_(float x) { return ffrom_bits_(fbits_(rcpf_(x)) + FM_HOST_SEED_ULPS); }
 #endif
 
 // double -> float by truncation of the significand, with integer operations
@@ -411,9 +415,10 @@ FM_HD uint64_t rcp_fixed60_(uint64_t X)
 {
   const uint32_t xh = (uint32_t)(X >> 32), xl = (uint32_t)X;
   const float xf = ffrom_bits_((int32_t)(0x3f800000u | ((uint32_t)(X >> 37) & 0x7fffffu)));   // x truncated
-  // y0 2^24, below 2^24 (y0 = 1 is taken one unit lower)
-  const uint32_t yb = (uint32_t)fbits_(rcp_seed_(xf));
-  const uint32_t y0 = ((yb < 0x3f7fffffu ? yb : 0x3f7fffffu) & 0x7fffffu) | 0x800000u;
+  // y0 2^24 in [2^23, 2^24): y0 = 1 is taken one unit lower, and a seed that
+  // the approximation's last unit puts below 1/2 (x next to 2) as 1/2
+  const uint32_t yb = (uint32_t)fbits_(rcp_seed_(xf)), yc = yb < 0x3f7fffffu ? yb : 0x3f7fffffu;
+  const uint32_t y0 = ((yc > 0x3f000000u ? yc : 0x3f000000u) & 0x7fffffu) | 0x800000u;
   // eps 2^84 = 2^84 - (x 2^60) (y0 2^24), modulo 2^64 (|eps| < 2^-21)
   const uint64_t p = (uint64_t)xl * y0 + ((uint64_t)(xh * y0) << 32);
   const int64_t e = (int64_t)(0u - p);
