@@ -59,10 +59,12 @@
 //
 // Accuracy: within 2 ulp (tests compare the host build of this code with
 // 200-bit mpmath values).  Every FP64 and FP32 operation is an explicit fma or
-// a separately rounded add/multiply, so host and device builds agree exactly.  Special
-// inputs (NaN, infinities, zero, negative, subnormal, overflow and underflow
-// ranges) leave the fast path through one integer test and get the IEEE
-// results of exp/log.
+// a separately rounded add/multiply, and the tests find the device build equal
+// to the host build bit for bit, but for the last bit of fatan: its quotient is
+// not settled, and the device's seed of it is the hardware's approximation (the
+// host's the rounded reciprocal).  Special inputs (NaN, infinities, zero,
+// negative, subnormal, overflow and underflow ranges) leave the fast path
+// through one integer test and get the IEEE results of exp/log.
 #pragma once
 
 #include <stdint.h>
