@@ -31,9 +31,9 @@ struct Mlp {
   float *p = nullptr, *g = nullptr, *m1 = nullptr, *m2 = nullptr;  // [nparam]
   std::vector<__nv_bfloat16 *> w16;   // BF16 copies of W
   // the transposes [din][ldt(l)], zero from dout to ldt, of the layers the
-  // backward pass contracts with (1 ..), valid for version t_version
+  // backward pass contracts with (1 ..): written wherever w16 is, so that a
+  // gradient (a captured one too) only reads them
   std::vector<__nv_bfloat16 *> w16t;
-  long t_version = -1;
   long ldt(int l) const { return (dout[l] + 15) / 16 * 16; }
   int *err = nullptr;
   float *loss = nullptr;
@@ -64,6 +64,19 @@ Mlp *as_mlp(void *p)
 {
   Mlp *m = static_cast<Mlp *>(p);
   return (m && m->magic == kMlpMagic) ? m : nullptr;
+}
+
+// The BF16 copies of the master weights and their transposes, on the default
+// stream (the caller synchronises).
+cudaError_t weights_to_bf16(Mlp *m)
+{
+  cudaError_t e = cudaSuccess;
+  for (int l = 0; l < m->nl && e == cudaSuccess; ++l) {
+    const float *w = m->p + m->woff[l];
+    if (l == 0) e = launch_to_bf16(w, m->w16[l], (long)m->din[l] * m->dout[l], nullptr);
+    else e = launch_to_bf16_t(w, m->w16[l], m->w16t[l], m->dout[l], m->din[l], m->ldt(l), m->ldt(l), nullptr);
+  }
+  return e;
 }
 
 void free_acts(Mlp *m)
@@ -248,27 +261,10 @@ cudaError_t weight_grad(Mlp *m, const __nv_bfloat16 *dzt, const __nv_bfloat16 *x
   return e;
 }
 
-// The transposed BF16 weights, refreshed when the parameters were set from
-// outside (a training step keeps them in step itself).
-cudaError_t ensure_transposes(Mlp *m, cudaStream_t s)
-{
-  if (m->t_version == m->version) return cudaSuccess;
-  cudaError_t e = cudaSuccess;
-  m->w16t.resize(m->nl, nullptr);
-  for (int l = 1; l < m->nl && e == cudaSuccess; ++l) {
-    if (!m->w16t[l]) e = cudaMalloc(&m->w16t[l], sizeof(__nv_bfloat16) * (size_t)m->din[l] * m->ldt(l));
-    if (e == cudaSuccess)
-      e = launch_to_bf16_t(m->p + m->woff[l], nullptr, m->w16t[l], m->dout[l], m->din[l], m->ldt(l), m->ldt(l), s);
-  }
-  if (e == cudaSuccess) m->t_version = m->version;
-  return e;
-}
-
 // Loss and gradient (into m->g) of n rows: x (device f32 [n][n_in]), tgt [n][16].
 cudaError_t mlp_loss_grad(Mlp *m, int n, const float *x, const float *tgt, cudaStream_t s)
 {
   cudaError_t e = ensure_acts(m, n);
-  if (e == cudaSuccess) e = ensure_transposes(m, s);
   const int n_max = m->n_hid > m->n_in ? m->n_hid : m->n_in;
   if (e == cudaSuccess) e = ensure_part(m, (long)(split_for(n) * n_max > COL_SUM_BLOCKS ? split_for(n) * n_max : COL_SUM_BLOCKS) * m->n_hid);
   const long pad = ((long)n + 127) / 128 * 128;
@@ -382,15 +378,18 @@ int ice3gb_mlp_create(const Ice3gbMlpShape *shape, uint64_t seed, void **out)
   if (e == cudaSuccess) e = cudaMemset(m->m2, 0, sizeof(float) * off);
   if (e == cudaSuccess) e = cudaMemset(m->err, 0, sizeof(int));
   m->w16.assign(m->nl, nullptr);
+  m->w16t.assign(m->nl, nullptr);
   for (int l = 0; l < m->nl && e == cudaSuccess; ++l) {
     e = cudaMalloc(&m->w16[l], sizeof(__nv_bfloat16) * (size_t)m->din[l] * m->dout[l]);
-    if (e == cudaSuccess) e = launch_to_bf16(m->p + m->woff[l], m->w16[l], (long)m->din[l] * m->dout[l], nullptr);
+    if (e == cudaSuccess && l > 0) e = cudaMalloc(&m->w16t[l], sizeof(__nv_bfloat16) * (size_t)m->din[l] * m->ldt(l));
   }
+  if (e == cudaSuccess) e = weights_to_bf16(m);
   if (e == cudaSuccess) e = cudaDeviceSynchronize();
   if (e != cudaSuccess) {
     free_acts(m);
     cudaFree(m->p); cudaFree(m->g); cudaFree(m->m1); cudaFree(m->m2); cudaFree(m->err); cudaFree(m->loss);
     for (auto *w : m->w16) cudaFree(w);
+    for (auto *w : m->w16t) cudaFree(w);
     delete m;
     return ICE3GB_ERR_CUDA;
   }
@@ -435,8 +434,7 @@ int ice3gb_mlp_set_params(void *mlp, const float *host)
   if (!m) return ICE3GB_ERR_HANDLE;
   if (!host) return ICE3GB_ERR_NULL;
   cudaError_t e = cudaMemcpy(m->p, host, sizeof(float) * m->nparam, cudaMemcpyHostToDevice);
-  for (int l = 0; l < m->nl && e == cudaSuccess; ++l)
-    e = launch_to_bf16(m->p + m->woff[l], m->w16[l], (long)m->din[l] * m->dout[l], nullptr);
+  if (e == cudaSuccess) e = weights_to_bf16(m);
   if (e == cudaSuccess) e = cudaMemset(m->m1, 0, sizeof(float) * m->nparam);
   if (e == cudaSuccess) e = cudaMemset(m->m2, 0, sizeof(float) * m->nparam);
   m->step = 0;
@@ -491,7 +489,6 @@ int ice3gb_mlp_train_step(void *mlp, int n, const float *x, const float *tgt, fl
   cudaError_t e = mlp_loss_grad(m, n, x, tgt, s);
   m->step += 1;
   m->version += 1;
-  if (e == cudaSuccess) m->t_version = m->version;     // adam_kernel writes the transposes too
   for (int l = 0; l < m->nl && e == cudaSuccess; ++l) {
     const long nw = (long)m->din[l] * m->dout[l];
     e = launch_adam(m->p + m->woff[l], m->g + m->woff[l], m->m1 + m->woff[l], m->m2 + m->woff[l], m->w16[l],

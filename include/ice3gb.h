@@ -384,7 +384,9 @@ int     ice3gb_mlp_forward(void *mlp, int n, const float *x, float *y, void *str
 int     ice3gb_mlp_forward_layered(void *mlp, int n, const float *x, float *y, void *stream);
 /* Loss (binary cross-entropy of the activity logits + squared error of the
  * values where active, mean over the n rows) and its gradient (device
- * [param_count] or NULL) for one batch. */
+ * [param_count] or NULL) for one batch.  The gradients and training steps of
+ * one network share its workspaces: the caller orders them, by one stream or by
+ * events between streams. */
 int     ice3gb_mlp_loss_grad(void *mlp, int n, const float *x, const float *targets, float *grad, float *loss,
                              void *stream);
 /* One Adam step (lr, beta 0.9 / 0.999) on one batch; loss: device float or NULL. */
