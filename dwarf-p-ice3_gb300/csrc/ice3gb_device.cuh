@@ -127,12 +127,14 @@ ICE3_HD float quot_est(double num, double den)
   return fm::mulf_(fm::to_f32(num), fm::rcp_seed_(fm::to_f32(den)));
 }
 // True only if the quotient that est estimates (quot_est) is above bound
-// for certain: above the truncated bound by 2^-17.
+// for certain: above the truncated bound by 2^-17, the bound positive and within
+// 2^-126 .. 2^126 (a smaller one truncates to 0, and the 0 that stands for no
+// estimate is above a negative one; a caller then forms the quotient).
 ICE3_HD bool est_above(float est, double bound)
 {
-  if (((fm::hi_(bound) >> 20) & 0x7ffu) >= 1149u) return false;
+  if ((fm::hi_(bound) >> 20) - 897u >= 252u) return false;
   const float b = fm::to_f32(bound);
-  return est > fm::fmaf_(fabsf(b), 0x1p-17f, b);
+  return est > fm::fmaf_(b, 0x1p-17f, b);
 }
 ICE3_HD bool quot_above(double num, double den, double bound) { return est_above(quot_est(num, den), bound); }
 
