@@ -32,23 +32,6 @@ using namespace ice3sed;
 // Levels a block forms the shared quantities of at a time, one per species
 // warp (a hail warp forms none).
 constexpr int SED_CH = 5;
-// The shared quantities of a level: LV_IDIV is dt / (rho dz) / dt (Fortran
-// scaling) or rho dz dt (the divisor of the JAX form).
-enum { LV_RHO = 0, LV_LRHO, LV_RHODZ_IDT, LV_TSO, LV_IDIV, LV_DZ_IDT, LV_N };
-
-// What a warp's species needs of the constants: its threshold and the power
-// law F exp(a log r + b log rho) (rain, snow, graupel, hail), the sum fused as
-// in power_speed.
-struct SpeciesPar {
-  double rtmin, f, a, b;
-};
-
-__device__ __forceinline__ SpeciesPar species_par(const Cst &c, int s)
-{
-  const double ex = s == 1 ? c.EXSEDR : s == 3 ? c.EXSEDS : s == 4 ? c.EXSEDG : c.EXSEDH;
-  return {sed_rtmin(c, s), s == 1 ? c.FSEDR : s == 3 ? c.FSEDS : s == 4 ? c.FSEDG : c.FSEDH, ex - 1.0,
-          ex - c.CEXVT - 1.0};
-}
 
 // FLUX_ONLY: the fluxes alone (the adjoint's recomputed forward sweep); the
 // sources and the surface precipitation are not written.
@@ -88,15 +71,7 @@ __global__ void __launch_bounds__(32 * 6) sedimentation_kernel(const __grid_cons
   int buf = 0;
   for (int top = a.nk - 1; top >= 0; top -= SED_CH, buf ^= 1) {
     if (s < SED_CH && top - s >= 0) {
-      const double rho = next_rho, dz = next_dz, rhodz = rho * dz;
-      const double tso = fm::fdiv(dt, rhodz);
-      double (*l)[32] = lev[buf][s];
-      l[LV_RHO][lane] = rho;
-      l[LV_LRHO][lane] = fm::flog(rho);
-      l[LV_RHODZ_IDT][lane] = rhodz * inv_dt;
-      l[LV_TSO][lane] = tso;
-      l[LV_IDIV][lane] = a.fortran ? tso * inv_dt : rhodz * dt;
-      l[LV_DZ_IDT][lane] = dz * inv_dt;
+      sed_shared(a.fortran, dt, inv_dt, next_rho, next_dz, LaneLev{lev[buf][s], lane});
     }
     __syncthreads();
     fetch_level(top - SED_CH - s);
@@ -107,49 +82,17 @@ __global__ void __launch_bounds__(32 * 6) sedimentation_kernel(const __grid_cons
       const long p = (long)(top - j) * nij + col;
       const double sr = next_src;
       if (valid && top - j > 0) next_src = src[p - nij];
-      const double (*l)[32] = lev[buf][j];
-      const double tso = l[LV_TSO][lane];
-      const double rt = sr * dt, qp = fabove * tso;
+      const LaneLev l = {lev[buf][j], lane};
+      const double rt = sr * dt, qp = fabove * l[LV_TSO];
       const bool c1 = valid && gtp(rt, par.rtmin), c2 = valid && gtp(qp, par.rtmin);
-      // no lane moves the species here (content at or below its threshold and
-      // not negative, nothing falling in): a zero flux, the source kept
-      if (__all_sync(0xffffffffu, !c1 && !c2 && !negd(rt) && zerod_(fabove))) {
+      if (__all_sync(0xffffffffu, sed_idle(c1, c2, rt, fabove))) {   // no lane moves the species here
         if (valid && fpr) fpr[p] = 0.0;
         fabove = 0.0;
         continue;
       }
-      const double lrho = l[LV_LRHO][lane];
-      // the fall speeds of the content (w1) and of the incoming flux (w2) as
-      // pairs; lanes without one carry 1/2 through
-      fm::Pair w;
-      {
-        const fm::Pair lr = fm::flog2(c1 ? rt : 0.5, c2 ? qp : 0.5);
-        if (s == 0) {          // as fall_speed's cloud droplets
-          double wlbda = 0.0;
-          if (c1 || c2) wlbda = 6.6e-8 * fm::fdiv(101325.0, ld1(a.pabs, p)) * (ld1(a.tht, p) * (1.0 / 293.15));
-          const double lc = cp.log_lbc_conc - lrho, lx = -c.CEXVT * lrho;
-          const fm::Pair lw = {c.LBEXC * (lc - lr.a), c.LBEXC * (lc - lr.b)};
-          const fm::Pair e2 = fm::fexp2(lw.a, lw.b), e1 = fm::fexp2(lx - c.DC * lw.a, lx - c.DC * lw.b);
-          const double k = 1.26 * wlbda * cp.ray_inv;
-          w = {e1.a * (c.CC * (1.0 + k * e2.a)) * cp.fsedc, e1.b * (c.CC * (1.0 + k * e2.b)) * cp.fsedc};
-        } else if (s == 2) {   // as fall_speed's pristine ice
-          const fm::Pair ld = fm::flog2(dmax(0.05e6, -0.15319e6 - 0.021454e6 * (lrho + lr.a)),
-                                        dmax(0.05e6, -0.15319e6 - 0.021454e6 * (lrho + lr.b)));
-          const double lx = -c.CEXVT * lrho;
-          const fm::Pair e = fm::fexp2(lx + c.EXCSEDI * ld.a, lx + c.EXCSEDI * ld.b);
-          w = {c.FSEDI * e.a, c.FSEDI * e.b};
-        } else {
-          const double blr = par.b * lrho;
-          const fm::Pair e = fm::fexp2(fm::fma_(par.a, lr.a, blr), fm::fma_(par.a, lr.b, blr));
-          w = {par.f * e.a, par.f * e.b};
-        }
-      }
-      const double w1 = c1 ? w.a : 0.0, w2 = c2 ? w.b : 0.0;
-      double flux = dmin(l[LV_RHODZ_IDT][lane] * rt, w1 * l[LV_RHO][lane] * rt);
-      if (!zerod_(w2)) flux += pmax0(1.0 - l[LV_DZ_IDT][lane] * fm::frcp(w2)) * fabove;
+      const double flux = sed_species_flux(c, s, par, cp, l, rt, qp, c1, c2, fabove, a.pabs, a.tht, p);
       if (valid) {
-        const double idiv = l[LV_IDIV][lane];
-        if (!FLUX_ONLY) src[p] = a.fortran ? sr + idiv * (fabove - flux) : sr + fm::fdiv(fabove - flux, idiv);
+        if (!FLUX_ONLY) src[p] = sed_species_source(a.fortran, l[LV_IDIV], sr, fabove, flux);
         if (fpr) fpr[p] = flux;
       }
       fabove = flux;

@@ -1,8 +1,10 @@
-// sedimentation_point.cuh — fall speeds and cloud parameters of the
-// statistical sedimentation (ICE4_SEDIMENTATION_STAT,
-// mode_ice4_sedimentation_stat.F90 and src/ice3/jax/stencils/sedimentation.py),
-// shared by the forward sweep (sedimentation.cu), its adjoint
-// (sedimentation_vjp.cu) and the host builds of the tests.
+// sedimentation_point.cuh — one species at one level of the statistical
+// sedimentation (ICE4_SEDIMENTATION_STAT, mode_ice4_sedimentation_stat.F90 and
+// src/ice3/jax/stencils/sedimentation.py) and of its adjoint: the code of the
+// kernels (sedimentation.cu, sedimentation_vjp.cu), which bring the columns,
+// the levels' shared quantities and the fluxes.  The sed_column_* functions
+// are sweeps of one column over the same levels for the host builds of the
+// tests.  Then the time-split form, whole columns.
 #pragma once
 
 #include "ice3gb_device.cuh"
@@ -122,17 +124,6 @@ ICE3_HD double fall_speed_d(const Cst &c, int s, double r, double lrho, double w
   }
 }
 
-// Fields of one sedimentation sweep; element (k, col) at k * nij + col.
-struct SedColumnIO {
-  const double *rhodref, *dzz, *pabs, *tht;
-  const double *src_in[5];   // sources read (rcs, rrs, ris, rss, rgs)
-  double *src_out[5];        // updated sources (may alias src_in), or NULL
-  double *fpr[5];            // fluxes F_k, or NULL
-  double *inpr[5];           // [nij] surface precipitation, or NULL
-  long nij;
-  int nk;
-};
-
 ICE3_HD double sed_rtmin(const Cst &c, int s)
 {
   return (s == 0) ? c.C_RTMIN : (s == 1) ? c.R_RTMIN : (s == 2) ? dmax(c.I_RTMIN, 1.0e-7) : (s == 3) ? c.S_RTMIN
@@ -149,58 +140,131 @@ ICE3_HD double sed_load(const double *p, long i)
 #endif
 }
 
-// Top-down sweep of one column (mode_ice4_sedimentation_stat.F90:143-229,
-// sedimentation.py:58-352): the five species side by side, the flux from the
-// level above carried in a register.  skip_c: PHYEX's LSEDIC = .FALSE.
-// (cloud not sedimented, its outputs left to the caller).
+// What a species needs of the constants: its threshold and the power law
+// F exp(a log r + b log rho) (rain, snow, graupel, hail), the sum fused as in
+// power_speed.
+struct SpeciesPar {
+  double rtmin, f, a, b;
+};
+ICE3_HD SpeciesPar species_par(const Cst &c, int s)
+{
+  const double ex = s == 1 ? c.EXSEDR : s == 3 ? c.EXSEDS : s == 4 ? c.EXSEDG : c.EXSEDH;
+  return {sed_rtmin(c, s), s == 1 ? c.FSEDR : s == 3 ? c.FSEDS : s == 4 ? c.FSEDG : c.FSEDH, ex - 1.0,
+          ex - c.CEXVT - 1.0};
+}
+
+// What the species share at a level; LV_IDIV is dt / (rho dz) / dt (Fortran
+// scaling) or rho dz dt (the divisor of the JAX form).  Lev: anything indexed by
+// these (the kernel's columns lie 32 apart and are read where they are used;
+// held in registers across the fall speeds they made the kernel spill).
+enum { LV_RHO = 0, LV_LRHO, LV_RHODZ_IDT, LV_TSO, LV_IDIV, LV_DZ_IDT, LV_N };
+#if defined(__CUDACC__)
+struct LaneLev {                                       // a lane's column in shared memory
+  double (*l)[32];
+  int lane;
+  __device__ __forceinline__ double &operator[](int q) const { return l[q][lane]; }
+};
+#endif
+template <class Lev>
+ICE3_HD void sed_shared(bool fortran, double dt, double inv_dt, double rho, double dz, Lev &&l)
+{
+  const double rhodz = rho * dz, tso = fm::fdiv(dt, rhodz);
+  l[LV_RHO] = rho;
+  l[LV_LRHO] = fm::flog(rho);
+  l[LV_RHODZ_IDT] = rhodz * inv_dt;
+  l[LV_TSO] = tso;
+  l[LV_IDIV] = fortran ? tso * inv_dt : rhodz * dt;
+  l[LV_DZ_IDT] = dz * inv_dt;
+}
+
+// The species does not move at the level: content rt at or below its threshold
+// (c1) and not negative, nothing falling in (c2): a zero flux, the source kept.
+ICE3_HD bool sed_idle(bool c1, bool c2, double rt, double fabove) { return !c1 && !c2 && !negd(rt) && zerod_(fabove); }
+
+// The flux leaving the level: content rt, incoming flux fabove as the content
+// qp = fabove dt / (rho dz), c1 / c2 whether each is above the threshold.  The
+// two fall speeds are formed as pairs; one that is not wanted carries 1/2
+// through.
+template <class Lev>
+ICE3_HD double sed_species_flux(const Cst &c, int s, const SpeciesPar &par, const CloudPar &cp, const Lev &l,
+                                double rt, double qp, bool c1, bool c2, double fabove, const double *pabs,
+                                const double *tht, long p)
+{
+  const double lrho = l[LV_LRHO];
+  const fm::Pair lr = fm::flog2(c1 ? rt : 0.5, c2 ? qp : 0.5);
+  fm::Pair w;
+  if (s == 0) {          // as fall_speed's cloud droplets
+    double wlbda = 0.0;
+    if (c1 || c2) wlbda = 6.6e-8 * fm::fdiv(101325.0, sed_load(pabs, p)) * (sed_load(tht, p) * (1.0 / 293.15));
+    const double lc = cp.log_lbc_conc - lrho, lx = -c.CEXVT * lrho;
+    const fm::Pair lw = {c.LBEXC * (lc - lr.a), c.LBEXC * (lc - lr.b)};
+    const fm::Pair e2 = fm::fexp2(lw.a, lw.b), e1 = fm::fexp2(lx - c.DC * lw.a, lx - c.DC * lw.b);
+    const double k = 1.26 * wlbda * cp.ray_inv;
+    w = {e1.a * (c.CC * (1.0 + k * e2.a)) * cp.fsedc, e1.b * (c.CC * (1.0 + k * e2.b)) * cp.fsedc};
+  } else if (s == 2) {   // as fall_speed's pristine ice
+    const fm::Pair ld = fm::flog2(dmax(0.05e6, -0.15319e6 - 0.021454e6 * (lrho + lr.a)),
+                                  dmax(0.05e6, -0.15319e6 - 0.021454e6 * (lrho + lr.b)));
+    const double lx = -c.CEXVT * lrho;
+    const fm::Pair e = fm::fexp2(lx + c.EXCSEDI * ld.a, lx + c.EXCSEDI * ld.b);
+    w = {c.FSEDI * e.a, c.FSEDI * e.b};
+  } else {
+    const double blr = par.b * lrho;
+    const fm::Pair e = fm::fexp2(fm::fma_(par.a, lr.a, blr), fm::fma_(par.a, lr.b, blr));
+    w = {par.f * e.a, par.f * e.b};
+  }
+  const double w1 = c1 ? w.a : 0.0, w2 = c2 ? w.b : 0.0;
+  double flux = dmin(l[LV_RHODZ_IDT] * rt, w1 * l[LV_RHO] * rt);
+  if (!zerod_(w2)) flux += pmax0(1.0 - l[LV_DZ_IDT] * fm::frcp(w2)) * fabove;
+  return flux;
+}
+
+// The source after the level's fluxes.
+ICE3_HD double sed_species_source(bool fortran, double idiv, double src, double fabove, double flux)
+{
+  return fortran ? src + idiv * (fabove - flux) : src + fm::fdiv(fabove - flux, idiv);
+}
+
+// Fields of one sedimentation sweep; element (k, col) at k * nij + col.
+struct SedColumnIO {
+  const double *rhodref, *dzz, *pabs, *tht;
+  const double *src_in[5];   // sources read (rcs, rrs, ris, rss, rgs)
+  double *src_out[5];        // updated sources (may alias src_in), or NULL
+  double *fpr[5];            // fluxes F_k, or NULL
+  double *inpr[5];           // [nij] surface precipitation, or NULL
+  long nij;
+  int nk;
+};
+
+// Top-down sweep of one column and species (mode_ice4_sedimentation_stat.F90:
+// 143-229, sedimentation.py:58-352) with the flux from the level above carried
+// along.  src_out, fpr and inpr may be NULL.
+ICE3_HD void sed_species_column(const Cst &c, int s, bool fortran, const CloudPar &cp, double dt, const SedColumnIO &io,
+                                const double *src_in, double *src_out, double *fpr, double *inpr, long col)
+{
+  const double inv_dt = 1.0 / dt;
+  const SpeciesPar par = species_par(c, s);
+  double fabove = 0.0;
+  for (int k = io.nk - 1; k >= 0; --k) {
+    const long p = (long)k * io.nij + col;
+    double l[LV_N];
+    sed_shared(fortran, dt, inv_dt, sed_load(io.rhodref, p), sed_load(io.dzz, p), l);
+    const double sr = src_in[p], rt = sr * dt, qp = fabove * l[LV_TSO];
+    const bool c1 = gtp(rt, par.rtmin), c2 = gtp(qp, par.rtmin), idle = sed_idle(c1, c2, rt, fabove);
+    const double flux = idle ? 0.0 : sed_species_flux(c, s, par, cp, l, rt, qp, c1, c2, fabove, io.pabs, io.tht, p);
+    if (src_out) src_out[p] = idle ? sr : sed_species_source(fortran, l[LV_IDIV], sr, fabove, flux);
+    if (fpr) fpr[p] = flux;
+    fabove = flux;
+  }
+  if (inpr) inpr[col] = fabove / c.RHOLW;
+}
+
+// The five species of a column; skip_c: PHYEX's LSEDIC = .FALSE. (cloud not
+// sedimented, its outputs left to the caller).
 ICE3_HD void sed_column_forward(const Cst &c, bool fortran, bool skip_c, const CloudPar &cp, double dt,
                                 const SedColumnIO &io, long col)
 {
-  const double inv_dt = 1.0 / dt;
-  double rtmin[5];
-#pragma unroll
-  for (int s = 0; s < 5; ++s) rtmin[s] = sed_rtmin(c, s);
-  double fabove[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
-  for (int k = io.nk - 1; k >= 0; --k) {
-    const long p = (long)k * io.nij + col;
-    const double rho = sed_load(io.rhodref, p), dz = sed_load(io.dzz, p);
-    const double rhodz = rho * dz;
-    const double tsorhodz = fm::fdiv(dt, rhodz);
-    double src[5], rt[5], qp[5];
-    bool c1[5], c2[5];
-    bool any = false;
-#pragma unroll
-    for (int s = 0; s < 5; ++s) {
-      if (s == 0 && skip_c) { c1[s] = c2[s] = false; src[s] = rt[s] = qp[s] = 0.0; continue; }
-      src[s] = io.src_in[s][p];
-      rt[s] = src[s] * dt;
-      qp[s] = fabove[s] * tsorhodz;
-      c1[s] = gtp(rt[s], rtmin[s]);
-      c2[s] = gtp(qp[s], rtmin[s]);
-      any = any || c1[s] || c2[s];
-    }
-    const double lrho = any ? fm::flog(rho) : 0.0;
-    const double wlbda =
-        (c1[0] || c2[0]) ? 6.6e-8 * fm::fdiv(101325.0, sed_load(io.pabs, p)) * (sed_load(io.tht, p) * (1.0 / 293.15))
-                         : 0.0;
-#pragma unroll
-    for (int s = 0; s < 5; ++s) {
-      if (s == 0 && skip_c) continue;
-      const double w1 = c1[s] ? fall_speed(c, s, rt[s], lrho, wlbda, cp) : 0.0;
-      const double w2 = c2[s] ? fall_speed(c, s, qp[s], lrho, wlbda, cp) : 0.0;
-      double flux = dmin(rhodz * rt[s] * inv_dt, w1 * rho * rt[s]);
-      if (!zerod_(w2)) flux += pmax0(1.0 - fm::fdiv(dz, dt * w2)) * fabove[s];
-      if (io.src_out[s]) {
-        if (fortran) io.src_out[s][p] = src[s] + tsorhodz * (fabove[s] - flux) * inv_dt;
-        else io.src_out[s][p] = src[s] + fm::fdiv(fabove[s] - flux, rhodz * dt);
-      }
-      if (io.fpr[s]) io.fpr[s][p] = flux;
-      fabove[s] = flux;
-    }
-  }
-#pragma unroll
-  for (int s = 0; s < 5; ++s)
-    if (!(s == 0 && skip_c) && io.inpr[s]) io.inpr[s][col] = fabove[s] / c.RHOLW;
+  for (int s = skip_c ? 1 : 0; s < 5; ++s)
+    sed_species_column(c, s, fortran, cp, dt, io, io.src_in[s], io.src_out[s], io.fpr[s], io.inpr[s], col);
 }
 
 // Hail in the statistical sweep (NRR = 7; species 7 of
@@ -209,26 +273,11 @@ ICE3_HD void sed_column_forward(const Cst &c, bool fortran, bool skip_c, const C
 ICE3_HD void sed_hail_column(const Cst &c, double dt, const double *rhodref, const double *dzz, double *rhs,
                              double *fpr, double *inpr, long nij, int nk, long col)
 {
-  const double inv_dt = 1.0 / dt;
-  const CloudPar cp{};
-  double fabove = 0.0;
-  for (int k = nk - 1; k >= 0; --k) {
-    const long p = (long)k * nij + col;
-    const double rho = sed_load(rhodref, p), dz = sed_load(dzz, p);
-    const double rhodz = rho * dz;
-    const double tsorhodz = fm::fdiv(dt, rhodz);
-    const double src = rhs[p], rt = src * dt, qp = fabove * tsorhodz;
-    const bool c1 = gtp(rt, c.H_RTMIN), c2 = gtp(qp, c.H_RTMIN);
-    const double lrho = (c1 || c2) ? fm::flog(rho) : 0.0;
-    const double w1 = c1 ? fall_speed(c, 5, rt, lrho, 0.0, cp) : 0.0;
-    const double w2 = c2 ? fall_speed(c, 5, qp, lrho, 0.0, cp) : 0.0;
-    double flux = dmin(rhodz * rt * inv_dt, w1 * rho * rt);
-    if (!zerod_(w2)) flux += pmax0(1.0 - fm::fdiv(dz, dt * w2)) * fabove;
-    rhs[p] = src + tsorhodz * (fabove - flux) * inv_dt;
-    if (fpr) fpr[p] = flux;
-    fabove = flux;
-  }
-  inpr[col] = fabove / c.RHOLW;
+  SedColumnIO io = {};
+  io.rhodref = rhodref; io.dzz = dzz;
+  io.nij = nij;
+  io.nk = nk;
+  sed_species_column(c, 5, true, CloudPar{}, dt, io, rhs, rhs, fpr, inpr, col);
 }
 
 // Cotangents of the sweep's outputs (NULL = zero) and the wanted gradients
@@ -243,10 +292,25 @@ struct SedGradients {
   double *rhodref, *dzz, *pabs, *tht;
 };
 
-// What the species share at a level of the reverse sweep, and the cotangents
-// of it that a species adds to.
+// What the species share at a level of the reverse sweep, indexed as in
+// sed_shared: RV_TSOR is RV_TSO / (rho dz), RV_IRHO 1 / rho.
+enum { RV_RHO = 0, RV_DZ, RV_RHODZ, RV_TSO, RV_LRHO, RV_TSOR, RV_IRHO, RV_N };
+template <class Lev>
+ICE3_HD void sed_vjp_shared(double dt, double rho, double dz, Lev &&l)
+{
+  const double rhodz = rho * dz, tso = fm::fdiv(dt, rhodz);
+  l[RV_RHO] = rho;
+  l[RV_DZ] = dz;
+  l[RV_RHODZ] = rhodz;
+  l[RV_TSO] = tso;
+  l[RV_LRHO] = fm::flog(rho);
+  l[RV_TSOR] = fm::fdiv(tso, rhodz);
+  l[RV_IRHO] = fm::frcp(rho);
+}
+// A species' view of them (tso = dt / (rho dz); wlbda: cloud only) and the
+// cotangents that it adds to.
 struct SedLevel {
-  double rho, dz, rhodz, tso, lrho, wlbda;   // tso = dt / (rho dz); wlbda: cloud only
+  double rho, dz, rhodz, tso, lrho, wlbda;
 };
 struct SedLevelCot {
   double rho, dz, rhodz, tso, lrho, wlbda;
@@ -335,6 +399,26 @@ ICE3_HD void sed_cloud_gradients(bool cloud, double wlbda, double pabs, double t
   }
 }
 
+// sed_vjp_species with the level's gradients: c_rho and c_dz receive the
+// species' parts of those of rho and dz (all its cotangents taken back to the
+// two), g_pabs and g_tht the cloud's (pabs and tht are read for it only).
+template <class Lev>
+ICE3_HD double sed_vjp_level(const Cst &c, int s, bool fortran, const CloudPar &cp, double dt, double inv_dt,
+                             const Lev &lv, double src, double rtmin, double fa, double fk, double gS, double bF, double pabs,
+                             double tht, double &b_src, double &c_rho, double &c_dz, double &g_pabs, double &g_tht)
+{
+  SedLevel l = {lv[RV_RHO], lv[RV_DZ], lv[RV_RHODZ], lv[RV_TSO], lv[RV_LRHO], 0.0};
+  if (s == 0) l.wlbda = 6.6e-8 * fm::fdiv(101325.0, pabs) * (tht * (1.0 / 293.15));
+  SedLevelCot b = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+  const double b_fa = sed_vjp_species(c, s, fortran, cp, dt, inv_dt, l, src, rtmin, fa, fk, gS, bF, b_src, b);
+  b.rhodz -= lv[RV_TSOR] * b.tso;
+  c_rho = b.rho + l.dz * b.rhodz + b.lrho * lv[RV_IRHO];
+  c_dz = b.dz + l.rho * b.rhodz;
+  if (s == 0)
+    sed_cloud_gradients(gtp(src * dt, rtmin) || gtp(fa * l.tso, rtmin), l.wlbda, pabs, tht, b.wlbda, g_pabs, g_tht);
+  return b_fa;
+}
+
 // Reverse sweep of one column (hand-written adjoint of sed_column_forward):
 // bottom-up, carrying the cotangent of the flux entering each level from
 // above.  `flux` holds the forward fluxes F_k of the column (io.fpr layout),
@@ -344,23 +428,14 @@ ICE3_HD void sed_column_vjp(const Cst &c, bool fortran, bool skip_c, const Cloud
                             const SedGradients &gx, long col)
 {
   const double inv_dt = 1.0 / dt;
-  double rtmin[5];
-  for (int s = 0; s < 5; ++s) rtmin[s] = sed_rtmin(c, s);
   // cotangent of F_k (flux leaving level k downward), starting at the surface
   double bF[5];
   for (int s = 0; s < 5; ++s) bF[s] = (g.inpr[s] && !(s == 0 && skip_c)) ? g.inpr[s][col] / c.RHOLW : 0.0;
   for (int k = 0; k < io.nk; ++k) {
     const long p = (long)k * io.nij + col;
-    SedLevel l;
-    l.rho = sed_load(io.rhodref, p);
-    l.dz = sed_load(io.dzz, p);
-    l.rhodz = l.rho * l.dz;
-    l.tso = fm::fdiv(dt, l.rhodz);
-    l.lrho = fm::flog(l.rho);
-    const double pabs = sed_load(io.pabs, p), tht = sed_load(io.tht, p);
-    l.wlbda = 6.6e-8 * fm::fdiv(101325.0, pabs) * (tht * (1.0 / 293.15));
-    SedLevelCot b = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
-    bool cloud = false;
+    double l[RV_N];
+    sed_vjp_shared(dt, sed_load(io.rhodref, p), sed_load(io.dzz, p), l);
+    double r = 0.0, d = 0.0, g_pabs = 0.0, g_tht = 0.0;
     for (int s = 0; s < 5; ++s) {
       const double gS = g.src[s] ? g.src[s][p] : 0.0;
       if (s == 0 && skip_c) {                       // sources passed through unchanged
@@ -369,18 +444,15 @@ ICE3_HD void sed_column_vjp(const Cst &c, bool fortran, bool skip_c, const Cloud
       }
       if (g.fpr[s]) bF[s] += g.fpr[s][p];
       const double fa = (k + 1 < io.nk) ? flux[s][p + io.nij] : 0.0;
-      if (s == 0) cloud = gtp(io.src_in[s][p] * dt, rtmin[s]) || gtp(fa * l.tso, rtmin[s]);
-      double b_src;
-      bF[s] = sed_vjp_species(c, s, fortran, cp, dt, inv_dt, l, io.src_in[s][p], rtmin[s], fa, flux[s][p], gS, bF[s],
-                              b_src, b);
+      double b_src, c_rho, c_dz;
+      bF[s] = sed_vjp_level(c, s, fortran, cp, dt, inv_dt, l, io.src_in[s][p], sed_rtmin(c, s), fa, flux[s][p], gS,
+                            bF[s], sed_load(io.pabs, p), sed_load(io.tht, p), b_src, c_rho, c_dz, g_pabs, g_tht);
       if (gx.src[s]) gx.src[s][p] = b_src;
+      r += c_rho;
+      d += c_dz;
     }
-    // level quantities shared by the species
-    b.rhodz += -fm::fdiv(l.tso, l.rhodz) * b.tso;
-    if (gx.rhodref) gx.rhodref[p] = b.rho + l.dz * b.rhodz + fm::fdiv(b.lrho, l.rho);
-    if (gx.dzz) gx.dzz[p] = b.dz + l.rho * b.rhodz;
-    double g_pabs, g_tht;
-    sed_cloud_gradients(cloud, l.wlbda, pabs, tht, b.wlbda, g_pabs, g_tht);
+    if (gx.rhodref) gx.rhodref[p] = r;
+    if (gx.dzz) gx.dzz[p] = d;
     if (gx.pabs) gx.pabs[p] = g_pabs;
     if (gx.tht) gx.tht[p] = g_tht;
   }

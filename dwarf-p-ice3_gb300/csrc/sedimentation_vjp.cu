@@ -4,7 +4,7 @@
 // The forward sweep (sedimentation.cu) first recomputes the fluxes F_k of the
 // five species into a scratch array (nothing is kept from the forward call);
 // the reverse sweep then walks the columns bottom-up with the cotangent of
-// the flux entering each level in a register (sed_vjp_species).  As in the
+// the flux entering each level in a register (sed_vjp_level).  As in the
 // forward kernel a block holds 32 columns and a warp per species; per SED_CH
 // levels the warps form what the species share, one level each, and at the end
 // add up the species' parts of the rho and dz gradients in the species' order
@@ -22,12 +22,11 @@ namespace {
 using namespace ice3sed;
 
 constexpr int SED_CH = 5;
-enum { LV_RHO = 0, LV_DZ, LV_RHODZ, LV_TSO, LV_LRHO, LV_TSOR, LV_IRHO, LV_N };   // TSOR: tso / (rho dz)
 
 __global__ void __launch_bounds__(32 * 5) sedimentation_vjp_kernel(const __grid_constant__ Cst c,
                                                                    const __grid_constant__ SedVjpArgs a)
 {
-  __shared__ double lev[SED_CH][LV_N][32];
+  __shared__ double lev[SED_CH][RV_N][32];
   __shared__ double part[SED_CH][5][2][32];            // the species' parts of the rho and dz gradients
   const int lane = threadIdx.x & 31, s = threadIdx.x >> 5;
   const long nij = a.nij, col = blockIdx.x * 32L + lane;
@@ -49,16 +48,7 @@ __global__ void __launch_bounds__(32 * 5) sedimentation_vjp_kernel(const __grid_
   for (int k0 = 0; k0 < a.nk; k0 += SED_CH) {
     if (k0 + s < a.nk) {
       const long p = (long)(k0 + s) * nij + col;
-      const double rho = valid ? ld1(a.rhodref, p) : 1.0, dz = valid ? ld1(a.dzz, p) : 1.0, rhodz = rho * dz;
-      const double tso = fm::fdiv(dt, rhodz);
-      double (*l)[32] = lev[s];
-      l[LV_RHO][lane] = rho;
-      l[LV_DZ][lane] = dz;
-      l[LV_RHODZ][lane] = rhodz;
-      l[LV_TSO][lane] = tso;
-      l[LV_LRHO][lane] = fm::flog(rho);
-      l[LV_TSOR][lane] = fm::fdiv(tso, rhodz);
-      l[LV_IRHO][lane] = fm::frcp(rho);
+      sed_vjp_shared(dt, valid ? ld1(a.rhodref, p) : 1.0, valid ? ld1(a.dzz, p) : 1.0, LaneLev{lev[s], lane});
     }
     __syncthreads();
     const int nlev = a.nk - k0 < SED_CH ? a.nk - k0 : SED_CH;
@@ -74,30 +64,14 @@ __global__ void __launch_bounds__(32 * 5) sedimentation_vjp_kernel(const __grid_
           if (a.gx.pabs) a.gx.pabs[p] = 0.0;
           if (a.gx.tht) a.gx.tht[p] = 0.0;
         } else {
-          const double (*lv)[32] = lev[j];
-          SedLevel l;
-          l.rho = lv[LV_RHO][lane]; l.dz = lv[LV_DZ][lane]; l.rhodz = lv[LV_RHODZ][lane];
-          l.tso = lv[LV_TSO][lane]; l.lrho = lv[LV_LRHO][lane];
-          l.wlbda = 0.0;
-          double pabs = 1.0, tht = 1.0;
-          if (s == 0) {
-            pabs = ld1(a.pabs, p);
-            tht = ld1(a.tht, p);
-            l.wlbda = 6.6e-8 * fm::fdiv(101325.0, pabs) * (tht * (1.0 / 293.15));
-          }
+          const double pabs = s == 0 ? ld1(a.pabs, p) : 1.0, tht = s == 0 ? ld1(a.tht, p) : 1.0;
           if (g_fpr) bF += ld1(g_fpr, p);
           const double fa = (k + 1 < a.nk) ? flux[p + nij] : 0.0;
-          SedLevelCot b = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
-          double b_src;
-          const double sr = ld1(src, p);
-          bF = sed_vjp_species(c, s, fortran, cp, dt, inv_dt, l, sr, rtmin, fa, flux[p], gS, bF, b_src, b);
+          double b_src, gp, gt;
+          bF = sed_vjp_level(c, s, fortran, cp, dt, inv_dt, LaneLev{lev[j], lane}, ld1(src, p), rtmin, fa, flux[p], gS, bF,
+                             pabs, tht, b_src, c_rho, c_dz, gp, gt);
           if (gx_src) gx_src[p] = b_src;
-          b.rhodz -= lv[LV_TSOR][lane] * b.tso;
-          c_rho = b.rho + l.dz * b.rhodz + b.lrho * lv[LV_IRHO][lane];
-          c_dz = b.dz + l.rho * b.rhodz;
           if (s == 0) {
-            double gp, gt;
-            sed_cloud_gradients(gtp(sr * dt, rtmin) || gtp(fa * l.tso, rtmin), l.wlbda, pabs, tht, b.wlbda, gp, gt);
             if (a.gx.pabs) a.gx.pabs[p] = gp;
             if (a.gx.tht) a.gx.tht[p] = gt;
           }
