@@ -385,27 +385,27 @@ ICE3_HD double sed_vjp_species(const Cst &c, int s, bool fortran, const CloudPar
   return b_fa;
 }
 
-// The gradients of the pressure and of theta at a level from the cotangent of
-// wlbda (proportional to theta / pressure): formed wherever a cloud speed was,
-// also where its cotangent is 0, so that a NaN input gives a NaN gradient;
-// 0 at a level without falling cloud.
-ICE3_HD void sed_cloud_gradients(bool cloud, double wlbda, double pabs, double tht, double b_wlbda, double &g_pabs,
-                                 double &g_tht)
-{
-  g_pabs = g_tht = 0.0;
-  if (cloud) {
-    g_pabs = -fm::fdiv(wlbda, pabs) * b_wlbda;
-    g_tht = fm::fdiv(wlbda, tht) * b_wlbda;
-  }
-}
+// Where a cloud speed is formed at a level, the factors that take the cotangent
+// of wlbda (proportional to theta / pressure) to the pressure and to theta.
+struct SedCloud {
+  bool falls;
+  double to_pabs, to_tht;
+};
+// The gradient from the sum of the species' cotangents of wlbda (that of a
+// species other than cloud is 0, or NaN where it has no finite value): formed
+// wherever cloud falls, also where the sum is 0, so that a NaN input gives a NaN
+// gradient; 0 at a level without falling cloud.
+ICE3_HD double sed_cloud_gradient(bool falls, double factor, double b_wlbda) { return falls ? factor * b_wlbda : 0.0; }
 
 // sed_vjp_species with the level's gradients: c_rho and c_dz receive the
 // species' parts of those of rho and dz (all its cotangents taken back to the
-// two), g_pabs and g_tht the cloud's (pabs and tht are read for it only).
+// two), b_wlbda its cotangent of wlbda, and cloud the factors (s = 0 only, for
+// which pabs and tht are read).
 template <class Lev>
 ICE3_HD double sed_vjp_level(const Cst &c, int s, bool fortran, const CloudPar &cp, double dt, double inv_dt,
-                             const Lev &lv, double src, double rtmin, double fa, double fk, double gS, double bF, double pabs,
-                             double tht, double &b_src, double &c_rho, double &c_dz, double &g_pabs, double &g_tht)
+                             const Lev &lv, double src, double rtmin, double fa, double fk, double gS, double bF,
+                             double pabs, double tht, double &b_src, double &c_rho, double &c_dz, double &b_wlbda,
+                             SedCloud &cloud)
 {
   SedLevel l = {lv[RV_RHO], lv[RV_DZ], lv[RV_RHODZ], lv[RV_TSO], lv[RV_LRHO], 0.0};
   if (s == 0) l.wlbda = 6.6e-8 * fm::fdiv(101325.0, pabs) * (tht * (1.0 / 293.15));
@@ -414,8 +414,12 @@ ICE3_HD double sed_vjp_level(const Cst &c, int s, bool fortran, const CloudPar &
   b.rhodz -= lv[RV_TSOR] * b.tso;
   c_rho = b.rho + l.dz * b.rhodz + b.lrho * lv[RV_IRHO];
   c_dz = b.dz + l.rho * b.rhodz;
-  if (s == 0)
-    sed_cloud_gradients(gtp(src * dt, rtmin) || gtp(fa * l.tso, rtmin), l.wlbda, pabs, tht, b.wlbda, g_pabs, g_tht);
+  b_wlbda = b.wlbda;
+  if (s == 0) {
+    cloud.falls = gtp(src * dt, rtmin) || gtp(fa * l.tso, rtmin);
+    cloud.to_pabs = cloud.falls ? -fm::fdiv(l.wlbda, pabs) : 0.0;
+    cloud.to_tht = cloud.falls ? fm::fdiv(l.wlbda, tht) : 0.0;
+  }
   return b_fa;
 }
 
@@ -435,7 +439,8 @@ ICE3_HD void sed_column_vjp(const Cst &c, bool fortran, bool skip_c, const Cloud
     const long p = (long)k * io.nij + col;
     double l[RV_N];
     sed_vjp_shared(dt, sed_load(io.rhodref, p), sed_load(io.dzz, p), l);
-    double r = 0.0, d = 0.0, g_pabs = 0.0, g_tht = 0.0;
+    double r = 0.0, d = 0.0, w = 0.0;
+    SedCloud cloud = {false, 0.0, 0.0};
     for (int s = 0; s < 5; ++s) {
       const double gS = g.src[s] ? g.src[s][p] : 0.0;
       if (s == 0 && skip_c) {                       // sources passed through unchanged
@@ -444,17 +449,18 @@ ICE3_HD void sed_column_vjp(const Cst &c, bool fortran, bool skip_c, const Cloud
       }
       if (g.fpr[s]) bF[s] += g.fpr[s][p];
       const double fa = (k + 1 < io.nk) ? flux[s][p + io.nij] : 0.0;
-      double b_src, c_rho, c_dz;
+      double b_src, c_rho, c_dz, b_wlbda;
       bF[s] = sed_vjp_level(c, s, fortran, cp, dt, inv_dt, l, io.src_in[s][p], sed_rtmin(c, s), fa, flux[s][p], gS,
-                            bF[s], sed_load(io.pabs, p), sed_load(io.tht, p), b_src, c_rho, c_dz, g_pabs, g_tht);
+                            bF[s], sed_load(io.pabs, p), sed_load(io.tht, p), b_src, c_rho, c_dz, b_wlbda, cloud);
       if (gx.src[s]) gx.src[s][p] = b_src;
       r += c_rho;
       d += c_dz;
+      w += b_wlbda;
     }
     if (gx.rhodref) gx.rhodref[p] = r;
     if (gx.dzz) gx.dzz[p] = d;
-    if (gx.pabs) gx.pabs[p] = g_pabs;
-    if (gx.tht) gx.tht[p] = g_tht;
+    if (gx.pabs) gx.pabs[p] = sed_cloud_gradient(cloud.falls, cloud.to_pabs, w);
+    if (gx.tht) gx.tht[p] = sed_cloud_gradient(cloud.falls, cloud.to_tht, w);
   }
 }
 

@@ -7,8 +7,8 @@
 // the flux entering each level in a register (sed_vjp_level).  As in the
 // forward kernel a block holds 32 columns and a warp per species; per SED_CH
 // levels the warps form what the species share, one level each, and at the end
-// add up the species' parts of the rho and dz gradients in the species' order
-// (deterministic), one level each.
+// add up the species' parts of the gradients in the species' order (deterministic),
+// one level each.
 //
 // Bound: the FP64 pipe (about 45 operations per species and level) and the
 // integer exp / log / division.  A thread per column with its five species
@@ -27,7 +27,9 @@ __global__ void __launch_bounds__(32 * 5) sedimentation_vjp_kernel(const __grid_
                                                                    const __grid_constant__ SedVjpArgs a)
 {
   __shared__ double lev[SED_CH][RV_N][32];
-  __shared__ double part[SED_CH][5][2][32];            // the species' parts of the rho and dz gradients
+  __shared__ double part[SED_CH][5][3][32];            // the species' parts: gradients of rho, dz, cotangent of wlbda
+  __shared__ double to[SED_CH][2][32];                 // SedCloud's factors
+  __shared__ unsigned falls[SED_CH];                   // and its lanes
   const int lane = threadIdx.x & 31, s = threadIdx.x >> 5;
   const long nij = a.nij, col = blockIdx.x * 32L + lane;
   const bool valid = col < nij, fortran = a.fortran;
@@ -56,39 +58,45 @@ __global__ void __launch_bounds__(32 * 5) sedimentation_vjp_kernel(const __grid_
     for (int j = 0; j < nlev; ++j) {
       const int k = k0 + j;
       const long p = (long)k * nij + col;
-      double c_rho = 0.0, c_dz = 0.0;
+      double c_rho = 0.0, c_dz = 0.0, b_wlbda = 0.0;
+      SedCloud cloud = {false, 0.0, 0.0};
       if (valid) {
         const double gS = g_src ? ld1(g_src, p) : 0.0;
         if (!moves) {                                  // source passed through unchanged
           if (gx_src) gx_src[p] = gS;
-          if (a.gx.pabs) a.gx.pabs[p] = 0.0;
-          if (a.gx.tht) a.gx.tht[p] = 0.0;
         } else {
           const double pabs = s == 0 ? ld1(a.pabs, p) : 1.0, tht = s == 0 ? ld1(a.tht, p) : 1.0;
           if (g_fpr) bF += ld1(g_fpr, p);
           const double fa = (k + 1 < a.nk) ? flux[p + nij] : 0.0;
-          double b_src, gp, gt;
+          double b_src;
           bF = sed_vjp_level(c, s, fortran, cp, dt, inv_dt, LaneLev{lev[j], lane}, ld1(src, p), rtmin, fa, flux[p], gS, bF,
-                             pabs, tht, b_src, c_rho, c_dz, gp, gt);
+                             pabs, tht, b_src, c_rho, c_dz, b_wlbda, cloud);
           if (gx_src) gx_src[p] = b_src;
-          if (s == 0) {
-            if (a.gx.pabs) a.gx.pabs[p] = gp;
-            if (a.gx.tht) a.gx.tht[p] = gt;
-          }
         }
       }
       part[j][s][0][lane] = c_rho;
       part[j][s][1][lane] = c_dz;
+      part[j][s][2][lane] = b_wlbda;
+      if (s == 0) {
+        to[j][0][lane] = cloud.to_pabs;
+        to[j][1][lane] = cloud.to_tht;
+        const unsigned m = __ballot_sync(0xffffffffu, cloud.falls);
+        if (lane == 0) falls[j] = m;
+      }
     }
     __syncthreads();
     if (s < nlev && valid) {
       const long p = (long)(k0 + s) * nij + col;
-      double r = part[s][0][0][lane], d = part[s][0][1][lane];
+      double r = part[s][0][0][lane], d = part[s][0][1][lane], w = part[s][0][2][lane];
 #pragma unroll
       for (int q = 1; q < 5; ++q) {
         r += part[s][q][0][lane];
         d += part[s][q][1][lane];
+        w += part[s][q][2][lane];
       }
+      const bool cloud = (falls[s] >> lane) & 1u;
+      if (a.gx.pabs) a.gx.pabs[p] = sed_cloud_gradient(cloud, to[s][0][lane], w);
+      if (a.gx.tht) a.gx.tht[p] = sed_cloud_gradient(cloud, to[s][1][lane], w);
       if (a.gx.rhodref) a.gx.rhodref[p] = r;
       if (a.gx.dzz) a.gx.dzz[p] = d;
     }
