@@ -85,7 +85,9 @@ __global__ void __launch_bounds__(32 * 6) sedimentation_kernel(const __grid_cons
       const LaneLev l = {lev[buf][j], lane};
       const double rt = sr * dt, qp = fabove * l[LV_TSO];
       const bool c1 = valid && gtp(rt, par.rtmin), c2 = valid && gtp(qp, par.rtmin);
-      if (__all_sync(0xffffffffu, sed_idle(c1, c2, rt, fabove))) {   // no lane moves the species here
+      // no lane moves the species here (the adjoint's fluxes: at a level whose
+      // rho dz is a positive normal number, elsewhere they may be NaN)
+      if (__all_sync(0xffffffffu, sed_idle(c1, c2, rt, fabove) && (!FLUX_ONLY || fm::frsqrt_ok(l[LV_RHODZ_IDT])))) {
         if (valid && fpr) fpr[p] = 0.0;
         fabove = 0.0;
         continue;
