@@ -319,10 +319,11 @@ ICE3_HD void ia_point(const Cst &c, const IaDerived &d, double dt, double inv_dt
   if (!d.subg) {
     cldfr = fgt((rcs + ris) * dt, 1e-12) ? 1.0 : 0.0;
     if (srcs) *srcs = cldfr;
-  } else if (warp_any(nz(x.cf_mf) || nz(x.rc_mf) || nz(x.ri_mf) || !fge(rvs, 0.0) || !finite_(inv_cphex))) {
+  } else if (warp_any(nz(x.cf_mf) || nz(x.rc_mf) || nz(x.ri_mf) || !fge(rvs, 0.0) || !finite_(inv_cphex) ||
+                      !finite_(lv))) {
     // the mass-flux clouds; a warp without any adds zeros (a negative vapour
     // source with no mass flux gives 0 * inf = NaN in the limiter, as in the
-    // reference, so it goes through)
+    // reference, and so does an infinite latent heat, so they go through)
     double w1m = x.rc_mf * inv_dt, w2m = x.ri_mf * inv_dt;
     const double tot = w1m + w2m;
     const double scale = fgt(tot, rvs) ? fm::fdiv(rvs, tot) : 1.0;
