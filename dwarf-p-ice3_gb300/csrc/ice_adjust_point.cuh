@@ -715,15 +715,17 @@ ICE3_HD void ia_point_vjp(const Cst &c, const IaDerived &d, double dt, double in
     const double b_qsl0 = (1.0 - frac) * b_qsl, b_qsi = frac * b_qsl;
     b_frac += (qsi - qsl0) * b_qsl;
     // qsi = rdrv piv / (pabs - piv), qsl0 = rdrv pv / (pabs - pv)
+    // (nothing flows through a pressure that is 0 or was not formed, unless its
+    // cotangent is not finite: a NaN)
     const double di = x.pabs - piv, dw = x.pabs - pv;
     double b_piv = 0.0, b_pv = 0.0;
-    if (nz(piv)) {
+    if (nz(piv) || !finite_(b_qsi)) {
       double ki, kip;
       fm::fdiv_rn2(d.rdrv * x.pabs, -d.rdrv * piv, di * di, ki, kip);
       b_piv = ki * b_qsi;
       b.pabs += kip * b_qsi;
     }
-    if (nz(pv)) {
+    if (nz(pv) || !finite_(b_qsl0)) {
       double kw, kwp;
       fm::fdiv_rn2(d.rdrv * x.pabs, d.rdrv * pv, dw * dw, kw, kwp);
       b_pv = kw * b_qsl0;
