@@ -541,9 +541,10 @@ ICE3_HD void ia_point_vjp(const Cst &c, const IaDerived &d, double dt, double in
     double b_w1m = 0.0, b_w2m = 0.0, b_cf = 0.0;
     const int mfpdf = d.mfpdf;
     // (a warp without mass-flux clouds has zero contents on the flat part of
-    // the PDF: nothing flows back where the thresholds are finite)
+    // the PDF: nothing flows back where the thresholds are finite, for a positive
+    // normal density and a finite temperature)
     if ((mfpdf == 0 || mfpdf == 1) &&
-        warp_any(nz(x.cf_mf) || nz(w1m) || nz(w2m) || !finite_(x.rho) || !finite_(t))) {
+        warp_any(nz(x.cf_mf) || nz(w1m) || nz(w2m) || !fm::frsqrt_ok(x.rho) || !finite_(t))) {
       const double criaut = fm::fdiv(c.CRIAUTC, x.rho);
       const double p10 = fm::fexp10(c.ACRIAUTI * (t - c.TT) + c.BCRIAUTI);
       bool ci_const;
