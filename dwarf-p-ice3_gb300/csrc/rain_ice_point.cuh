@@ -1585,9 +1585,10 @@ ICE3_HD unsigned int rain_ice_point(const Cst &c, const Derived &d, const double
     const double wr = (vart[IRR] - rr0) * inv_dt, wi = (vart[IRI] - ri0) * inv_dt;
     const double ws = (vart[IRS] - rs0) * inv_dt, wg = (vart[IRG] - rg0) * inv_dt;
     const double wh = H ? (vart[NVT - 1] - ldp(f.rht, p)) * inv_dt : 0.0;
-    // (zrvheni = MIN(rvs, 0) here: 0 but for a negative vapour source)
+    // (zrvheni = MIN(rvs, 0) here: 0 but for a negative vapour source; 0 times
+    // an infinite lsx is NaN)
     double dth = (wc + wr) * lvx + (H ? wi + ws + wg + wh : wi + ws + wg) * lsx, dv = wv, di = wi;
-    if (warp_any(nz(zrvheni))) {
+    if (warp_any(nz(zrvheni) || !finite_(lsx))) {
       dth += zrvheni * lsx;
       dv -= zrvheni;
       di += zrvheni;
