@@ -724,8 +724,11 @@ __global__ void to_bf16_t_kernel(const float *__restrict__ x, __nv_bfloat16 *__r
 
 }  // namespace
 
-// The stage ring takes 192 KB, so one CTA is resident per SM and no
-// tcgen05.alloc has to wait for columns.
+// The stage ring takes 96 KB of an SM's 227 KB, so at most two CTAs are resident
+// per SM, with at most G_NT of the 512 TMEM columns each: no tcgen05.alloc has to
+// wait for another CTA of this kernel.
+constexpr int SM_SMEM = 227 * 1024, TMEM_COLS = 512;
+static_assert(SM_SMEM / (G_NST * G_STAGE * 2) * G_NT <= TMEM_COLS, "TMEM columns of the CTAs of an SM");
 static_assert(G_NST * G_STAGE * 2 >= G_THREADS * G_LINE * 4, "the epilogue's buffers fit in the ring");
 size_t tc_gemm_smem_bytes() { return (size_t)G_NST * G_STAGE * sizeof(__nv_bfloat16); }
 

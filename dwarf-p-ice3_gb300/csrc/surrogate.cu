@@ -232,7 +232,8 @@ cudaError_t mlp_infer_dev(Mlp *m, long n, const float *x, float *y, cudaStream_t
 }
 
 // Batch ranges of a weight gradient: 256 rows each, so that a batch of 16,384
-// gives 64 x 2 tiles of a 256-wide layer for the 152 SMs.
+// gives 64 x 2 x 2 tiles of 128 x 128 of a 256-wide layer for the two CTAs of
+// each of the 152 SMs.
 int split_for(int n) { int sp = n / 256; return sp < 1 ? 1 : (sp > 64 ? 64 : sp); }
 
 cudaError_t ensure_part(Mlp *m, long words)
