@@ -119,7 +119,6 @@ __device__ __forceinline__ double fma_(double a, double b, double c) { return __
 __device__ __forceinline__ double add_(double a, double b) { return __dadd_rn(a, b); }
 __device__ __forceinline__ double mul_(double a, double b) { return __dmul_rn(a, b); }
 __device__ __forceinline__ float fmaf_(float a, float b, float c) { return __fmaf_rn(a, b, c); }
-__device__ __forceinline__ float addf_(float a, float b) { return __fadd_rn(a, b); }
 __device__ __forceinline__ float mulf_(float a, float b) { return __fmul_rn(a, b); }
 __device__ __forceinline__ int64_t bits_(double x) { return __double_as_longlong(x); }
 __device__ __forceinline__ double from_bits_(int64_t b) { return __longlong_as_double(b); }
@@ -153,7 +152,6 @@ inline double fma_(double a, double b, double c) { return std::fma(a, b, c); }
 inline double add_(double a, double b) { volatile double s = a + b; return s; }
 inline double mul_(double a, double b) { volatile double s = a * b; return s; }
 inline float fmaf_(float a, float b, float c) { return std::fmaf(a, b, c); }
-inline float addf_(float a, float b) { volatile float s = a + b; return s; }
 inline float mulf_(float a, float b) { volatile float s = a * b; return s; }
 inline int64_t bits_(double x) { int64_t b; memcpy(&b, &x, 8); return b; }
 inline double from_bits_(int64_t b) { double x; memcpy(&x, &b, 8); return x; }
@@ -202,13 +200,6 @@ FM_HD double i2d(int32_t k)
   const int n = 31 - clz32_(a);                                  // index of the leading bit
   const int64_t mant = ((int64_t)a << (52 - n)) & 0x000fffffffffffffLL;
   return from_bits_(s | ((int64_t)(1023 + n) << 52) | mant);
-}
-
-// Nearest integer of a float with |t| < 2^22 (shifter trick, FP32 add).
-FM_HD int32_t rint_f32(float t)
-{
-  const float sh = 12582912.0f;                                  // 1.5 * 2^23
-  return fbits_(addf_(t, sh)) - fbits_(sh);
 }
 
 // hi : lo of a 64 x 64-bit product's upper half, without the carry of the
@@ -612,10 +603,5 @@ FM_NI double fatan(double x)
   const uint64_t m = (top >> 11) + ((uint32_t)(top >> 10) & 1u);
   return from_bits_((int64_t)(m + ((uint64_t)((comp ? 1023u : 1021u) - lz) << 52) + ((uint64_t)(h & 0x80000000u) << 32)));
 }
-
-// x^a = e^(a log x) for x > 0 (relative error ~|a log x| ulp).
-FM_HD double fpow(double x, double a) { return fexp(mul_(a, flog(x))); }
-// x^a from a precomputed log x.
-FM_HD double fpowl(double logx, double a) { return fexp(mul_(a, logx)); }
 
 }  // namespace fm

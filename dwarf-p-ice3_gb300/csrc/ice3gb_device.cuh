@@ -144,7 +144,6 @@ ICE3_HD bool quot_above(double num, double den, double bound) { return est_above
 // fraction of the FP64 instructions; callers raising one base to several
 // powers pass a shared log.
 ICE3_HD double powl_(double logx, double a) { return fm::fexp(a * logx); }
-ICE3_HD double fpow(double x, double a) { return fm::fexp(a * fm::flog(x)); }
 
 // TIWMX saturation tables of OCND2 (micro/modd_tiwmx.F90, filled by
 // micro/mode_ini_tiwmx.F90 from micro/mode_tiwmx_fun.F90) at T = j/100 K,
