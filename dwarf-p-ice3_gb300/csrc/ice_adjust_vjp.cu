@@ -15,9 +15,9 @@ using namespace ice3ia;
 
 __device__ __forceinline__ double ldz(const double *p, long i) { return p ? __ldg(p + i) : 0.0; }
 
-// Bound: the FP64 pipe (about 300 operations per point; IEEE divisions and the
+// Bound: the FP64 pipe (289 instructions per warp of points, 83 % busy; IEEE divisions and the
 // square root are integer, what a point's ice fraction or missing mass-flux
-// cloud gives no weight is not formed; 483 before): 5.72 -> 3.41 ms for
+// cloud gives no weight is not formed; 483 before): 5.72 -> 3.28 ms for
 // 256x256x90.  Two blocks per SM (128 registers, 148 bytes spilled) against
 // one (200): 13.89 / 14.13 ms for the whole adjoint.
 __global__ void __launch_bounds__(256, 2) ice_adjust_vjp_kernel(const __grid_constant__ Cst c,

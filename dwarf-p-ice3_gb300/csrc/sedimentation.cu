@@ -15,13 +15,14 @@
 // each of the next SED_CH and leave it in shared memory (two buffers, one
 // barrier per SED_CH levels).
 //
-// Bound: per warp and level the FP64 pipe (about 15 operations per species)
-// and the issue of the integer exp / log / reciprocal; a column's chain of nk
+// Bound: per warp and level the FP64 pipe (18 instructions per species, 23 in
+// the JAX form; 61 % busy at 256x256x90), the barrier between warps of unequal
+// work, and the issue of the integer exp / log / reciprocal; a column's chain of nk
 // levels where the columns are few.  One thread per column with its five
 // species one after the other (their fall speeds dealt out over the warp with
 // shuffles) took 2.88 ms for 65,535 x 87 and 1.64 ms for a single block of 32
 // columns x 90; five warps per 32 columns took 2.01 and 0.40 ms, and with the
-// two fall speeds of a level formed as a pair 1.88 and 0.38 ms.
+// two fall speeds of a level formed as a pair 1.89 and 0.30 ms.
 #include "ice3gb_device.cuh"
 #include "ice3gb_kernels.h"
 #include "sedimentation_point.cuh"

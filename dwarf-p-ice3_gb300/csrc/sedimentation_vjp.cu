@@ -10,10 +10,10 @@
 // add up the species' parts of the gradients in the species' order (deterministic),
 // one level each.
 //
-// Bound: the FP64 pipe (about 45 operations per species and level) and the
-// integer exp / log / division.  A thread per column with its five species
+// Bound: the FP64 pipe (61 instructions per warp, species and level; 71 % busy)
+// and the integer exp / log / division.  A thread per column with its five species
 // one after the other, forward and reverse in one kernel, took 8.03 ms for
-// 65,536 x 90; the two kernels take 1.83 + 4.25 ms.
+// 65,536 x 90; the two kernels take 1.74 + 4.06 ms.
 #include "ice3gb_device.cuh"
 #include "ice3gb_kernels.h"
 #include "sedimentation_point.cuh"
