@@ -379,7 +379,10 @@ int     ice3gb_mlp_set_params(void *mlp, const float *host);
  * aligned x runs one fused persistent kernel (weights streamed from L2,
  * activations kept on chip); other shapes, and ice3gb_mlp_forward_layered
  * always, run one tensor-core GEMM launch per layer (the training forward).
- * Both give the same values bit for bit. */
+ * Both give the same values bit for bit.  The first fused call after the
+ * parameters changed packs them on its stream: the caller orders calls on other
+ * streams behind it, and captures a forward after such a call (a graph captured
+ * before the change keeps the weights packed then). */
 int     ice3gb_mlp_forward(void *mlp, int n, const float *x, float *y, void *stream);
 int     ice3gb_mlp_forward_layered(void *mlp, int n, const float *x, float *y, void *stream);
 /* Loss (binary cross-entropy of the activity logits + squared error of the
